@@ -212,6 +212,8 @@ GraphEngine::~GraphEngine() {
     cudaFree(q.qbg_ovf);
     cudaFree(q.blob_dist);
   }
+  cudaFree(linear_scratch_.dev);
+  if (linear_scratch_.pinned) cudaFreeHost(linear_scratch_.pinned);
   tc_release(tc_);
   if (stream_) cudaStreamDestroy(stream_);
 }
@@ -1190,38 +1192,79 @@ void GraphEngine::linear_search(const void* queries, QueryType qt, size_t nq, si
   if (!fn) throw std::runtime_error("unsupported distance for linear search");
   cudaStream_t s = stream_;
   const uint32_t rc = dev_.row_chunks;
-  const size_t nrows = host_.nrows;
-  size_t qb = std::max<size_t>(1, std::min<size_t>({nq, (size_t)(1u << 28) / nrows, (size_t)65535}));
-  uint4* d_rows = nullptr;
-  float* d_dist = nullptr;
-  ObjDist* d_out = nullptr;
-  uint32_t* d_counts = nullptr;
-  NGT_CUDA(cudaMallocAsync(&d_rows, rows.size(), s));
-  NGT_CUDA(cudaMallocAsync(&d_dist, qb * nrows * 4, s));
-  NGT_CUDA(cudaMallocAsync(&d_out, nq * kmax * sizeof(ObjDist), s));
-  NGT_CUDA(cudaMallocAsync(&d_counts, nq * 4, s));
-  NGT_CUDA(cudaMemcpyAsync(d_rows, rows.data(), rows.size(), cudaMemcpyHostToDevice, s));
+  const size_t nrows = host_.nrows, rb = host_.row_bytes();
+  // queries per block: at most 16 MB of distances (or one query's)
+  const size_t qb = std::max<size_t>(1, std::min<size_t>({nq, ((size_t)1 << 22) / nrows, (size_t)65535}));
+  const uint32_t kpow = next_pow2((uint32_t)size);
+  auto al = [](size_t x) { return (x + 255) & ~(size_t)255; };
+  // device block: rows | distances | histograms, states | keys | results, counts; the
+  // pinned block holds the rows going in and the results and counts coming out
+  const size_t o_dist = al(qb * rb), o_hist = o_dist + al(qb * nrows * 4);
+  const size_t o_sel = o_hist + al(qb * kSelBins * 4), o_keys = o_sel + al(qb * sizeof(LinearSelect));
+  const size_t o_out = o_keys + al(qb * (size_t)kpow * 8), o_cnt = o_out + al(qb * kmax * sizeof(ObjDist));
+  const size_t total = o_cnt + al(qb * 4), back = total - o_out;
+  LinearScratch& w = linear_scratch_;
+  if (w.dev_bytes < total) {
+    NGT_CUDA(cudaFree(w.dev));
+    w.dev = nullptr;
+    w.dev_bytes = 0;
+    NGT_CUDA(cudaMalloc(&w.dev, total));
+    w.dev_bytes = total;
+  }
+  if (w.pinned_bytes < o_dist + back) {
+    NGT_CUDA(cudaFreeHost(w.pinned));
+    w.pinned = nullptr;
+    w.pinned_bytes = 0;
+    NGT_CUDA(cudaMallocHost(&w.pinned, o_dist + back));
+    w.pinned_bytes = o_dist + back;
+  }
+  uint8_t* d = static_cast<uint8_t*>(w.dev);
+  uint8_t* h = static_cast<uint8_t*>(w.pinned);
+  const uint4* d_rows = reinterpret_cast<const uint4*>(d);
+  float* d_dist = reinterpret_cast<float*>(d + o_dist);
+  uint32_t* d_hist = reinterpret_cast<uint32_t*>(d + o_hist);
+  LinearSelect* d_sel = reinterpret_cast<LinearSelect*>(d + o_sel);
+  unsigned long long* d_keys = reinterpret_cast<unsigned long long*>(d + o_keys);
+  ObjDist* d_out = reinterpret_cast<ObjDist*>(d + o_out);
+  uint32_t* d_counts = reinterpret_cast<uint32_t*>(d + o_cnt);
   const uint32_t group = std::min<uint32_t>(32, next_pow2(rc));
-  const size_t sel_smem = (256 + 16) * 4 + 2 * kmax * 8;
-  NGT_CUDA(cudaFuncSetAttribute((const void*)linear_select_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)sel_smem));
+  int sms = 0;
+  NGT_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device_));
+  NGT_CUDA(cudaFuncSetAttribute((const void*)linear_collect_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)(kpow * 8)));
   for (size_t q0 = 0; q0 < nq; q0 += qb) {
-    size_t nb = std::min(qb, nq - q0);
+    const size_t nb = std::min(qb, nq - q0);
+    std::memcpy(h, rows.data() + q0 * rb, nb * rb);
+    NGT_CUDA(cudaMemcpyAsync(d, h, nb * rb, cudaMemcpyHostToDevice, s));
+    NGT_CUDA(cudaMemsetAsync(d_hist, 0, o_keys - o_hist, s));
     dim3 grid((unsigned)((nrows + kLinRowsPerBlock - 1) / kLinRowsPerBlock), (unsigned)nb);
-    fn<<<grid, kLinThreads, rc * 16, s>>>(dev_, d_rows, (uint32_t)q0, (uint32_t)nb, d_present_, d_dist, group);
+    fn<<<grid, kLinThreads, rc * 16, s>>>(dev_, d_rows, 0, (uint32_t)nb, d_present_, d_dist, group);
     NGT_CUDA(cudaGetLastError());
-    linear_select_kernel<<<(unsigned)nb, 512, sel_smem, s>>>(d_dist, (uint32_t)nrows, (uint32_t)q0, (uint32_t)nb,
-                                                               (uint32_t)size, FLT_MAX, d_out, d_counts);
+    // about two blocks per SM over the block's queries, 4096 rows or more each
+    const size_t per_query = std::max<size_t>(1, (size_t)sms * 2 / nb);
+    dim3 sgrid((unsigned)std::min((nrows + kSelRowsPerBlock - 1) / kSelRowsPerBlock, per_query), (unsigned)nb);
+    auto pass = [&](uint32_t shift, uint32_t bits, bool first) {
+      linear_radix_kernel<<<sgrid, kSelThreads, 0, s>>>(d_dist, (uint32_t)nrows, (uint32_t)size, shift, bits,
+                                                        first ? 1u : 0u, d_hist, d_sel);
+      NGT_CUDA(cudaGetLastError());
+      launches_++;
+    };
+    pass(53, 11, true);
+    pass(42, 11, false);
+    pass(32, 10, false);
+    // ties at the k-th distance: the lowest ids (digits above the largest id are zero)
+    if (nrows > (1u << 21)) pass(21, 11, false);
+    if (nrows > (1u << 10)) pass(10, 11, false);
+    pass(0, 10, false);
+    linear_collect_kernel<<<sgrid, kSelThreads, kpow * 8, s>>>(d_dist, (uint32_t)nrows, 0, (uint32_t)size, kpow,
+                                                               d_sel, d_keys, d_out, d_counts);
     NGT_CUDA(cudaGetLastError());
     launches_ += 2;
+    NGT_CUDA(cudaMemcpyAsync(h + o_dist, d_out, back, cudaMemcpyDeviceToHost, s));
+    NGT_CUDA(cudaStreamSynchronize(s));
+    std::memcpy(out.results.data() + q0 * kmax, h + o_dist, nb * kmax * sizeof(ObjDist));
+    std::memcpy(out.counts.data() + q0, h + o_dist + (o_cnt - o_out), nb * 4);
   }
-  NGT_CUDA(cudaMemcpyAsync(out.results.data(), d_out, nq * kmax * sizeof(ObjDist), cudaMemcpyDeviceToHost, s));
-  NGT_CUDA(cudaMemcpyAsync(out.counts.data(), d_counts, nq * 4, cudaMemcpyDeviceToHost, s));
-  NGT_CUDA(cudaFreeAsync(d_rows, s));
-  NGT_CUDA(cudaFreeAsync(d_dist, s));
-  NGT_CUDA(cudaFreeAsync(d_out, s));
-  NGT_CUDA(cudaFreeAsync(d_counts, s));
-  NGT_CUDA(cudaStreamSynchronize(s));
 }
 
 }  // namespace ngtg

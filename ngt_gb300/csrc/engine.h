@@ -439,6 +439,15 @@ class GraphEngine {
   float sq8_offset_ = 0.f, sq8_scale_ = 1.f;
   FastTuning tuning_;
   DevGraph dev_;
+  // buffers of the exhaustive search, grown on demand and kept (mu_ held): at most about
+  // 115 MB, or one query's distances where those are more
+  struct LinearScratch {
+    void* dev = nullptr;
+    size_t dev_bytes = 0;
+    void* pinned = nullptr;
+    size_t pinned_bytes = 0;
+  };
+  LinearScratch linear_scratch_;
   void ensure_tc_rows();
   void ensure_tc_rows8();
   TcState* tc_ = nullptr;
