@@ -184,6 +184,24 @@ struct Acc {
     }
   }
 
+  // This lane's sums plus those of another lane: one level of reduce() between two lanes
+  // that one thread holds.
+  __device__ __forceinline__ void fold(const Acc& o) {
+    if constexpr (M == Metric::Lorentz) {
+      float lo = f1 + o.f1;
+      two_sum_acc(f0, lo, o.f0);
+      f1 = lo;
+      return;
+    }
+    if constexpr (kUseF0) f0 += o.f0;
+    if constexpr (kUseF12) {
+      f1 += o.f1;
+      f2 += o.f2;
+    }
+    if constexpr (kUseI0) i0 += o.i0;
+    if constexpr (kUseI1) i1 += o.i1;
+  }
+
   __device__ __forceinline__ float finish() const {
     if constexpr (OT == ObjType::Qsint8 && M == Metric::L2) {
       // the squared sum itself: PrimitiveComparator::compareL2(qsint8) of the x86
@@ -256,6 +274,53 @@ __device__ __forceinline__ float group_distance(const uint4* __restrict__ q, con
   }
   acc.reduce(width);
   return acc.finish();
+}
+
+// Distances of U rows by a quarter of the lanes: with `width` lanes a row in
+// group_distance, width / 4 threads (at least one) each hold four of those lanes' sums
+// and add them in the order of reduce(), so every distance has group_distance's bits.
+// Bound by instruction issue where the rows are in flight already: a 512-byte float row
+// then takes about 18 warp instructions instead of 50 (two shuffle-and-adds fewer per
+// row and lane, one square root per row and not per lane).  t: the thread's index inside
+// its packed_width(width) threads; all lanes of the warp take part.
+__device__ __forceinline__ int packed_width(int width) { return width >= 4 ? width >> 2 : 1; }
+
+template <ObjType OT, Metric M, int U>
+__device__ __forceinline__ void packed_distances(const uint4* __restrict__ q, const uint4* __restrict__ objects,
+                                                 const uint32_t (&id)[U], int nchunks, int t, int width,
+                                                 float (&d)[U]) {
+  const int pw = packed_width(width);
+  Acc<OT, M> acc[U][4];
+  for (int c0 = t; c0 < nchunks; c0 += width) {
+    uint4 xv[U][4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const int c = c0 + j * pw;
+      const bool on = c < nchunks && j < width;
+#pragma unroll
+      for (int u = 0; u < U; u++)
+        xv[u][j] = on ? __ldg(objects + (size_t)id[u] * nchunks + c) : make_uint4(0u, 0u, 0u, 0u);
+    }
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const int c = c0 + j * pw;
+      if (c < nchunks && j < width) {
+        const uint4 qc = q[c];
+#pragma unroll
+        for (int u = 0; u < U; u++) acc[u][j].add(qc, xv[u][j], c);
+      }
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < U; u++) {
+    if (width >= 4) {
+      acc[u][0].fold(acc[u][2]);
+      acc[u][1].fold(acc[u][3]);
+    }
+    if (width >= 2) acc[u][0].fold(acc[u][1]);
+    acc[u][0].reduce(pw);
+    d[u] = acc[u][0].finish();
+  }
 }
 
 // Monotone map of a float to unsigned bits (negative distances occur: the

@@ -53,13 +53,13 @@ uint32_t next_pow2(uint32_t v) {
   return p;
 }
 
-ExactKernelFn exact_kernel(ObjType t, Metric m) {
+ExactKernelFn exact_kernel(ObjType t, Metric m, uint32_t threads = kExactThreads) {
   if (t != ObjType::Qsint8) m = kernel_metric(m);   // qsint8 inner product: its own comparator
   switch (t) {
-    case ObjType::Float: return exact_kernel_float(m);
-    case ObjType::Float16: return exact_kernel_half(m);
-    case ObjType::Uint8: return exact_kernel_u8(m);
-    case ObjType::Qsint8: return exact_kernel_qs8(m);
+    case ObjType::Float: return exact_kernel_float(m, threads);
+    case ObjType::Float16: return exact_kernel_half(m, threads);
+    case ObjType::Uint8: return exact_kernel_u8(m, threads);
+    case ObjType::Qsint8: return exact_kernel_qs8(m, threads);
     default: return nullptr;
   }
 }
@@ -678,12 +678,14 @@ void GraphEngine::search_device(const uint4* d_rows, size_t nq, const SearchArgs
   build_params(args, nargs, nq, kmax, params, seeds, max_size);
   QueryParams* d_params = nullptr;
   uint32_t* d_seeds = nullptr;
-  NGT_CUDA(cudaMallocAsync(&d_params, nq * sizeof(QueryParams), stream));
+  // the launch's own work counter lies behind its parameters
+  NGT_CUDA(cudaMallocAsync(&d_params, nq * sizeof(QueryParams) + 4, stream));
   NGT_CUDA(cudaMallocAsync(&d_seeds, seeds.size() * 4, stream));
   NGT_CUDA(cudaMemcpyAsync(d_params, params.data(), nq * sizeof(QueryParams), cudaMemcpyHostToDevice, stream));
   NGT_CUDA(cudaMemcpyAsync(d_seeds, seeds.data(), seeds.size() * 4, cudaMemcpyHostToDevice, stream));
   if (kernel == Kernel::Exact)
-    launch_exact(d_rows, nq, d_params, d_seeds, max_size, d_out, d_counts, d_stats, stream);
+    launch_exact(d_rows, nq, d_params, d_seeds, max_size, d_out, d_counts, d_stats, stream, nullptr, nullptr, 0,
+                 reinterpret_cast<uint32_t*>(d_params + nq));
   else if (kernel == Kernel::Wide)
     launch_wide(d_rows, nq, d_params, d_seeds, max_size, d_out, d_counts, d_stats, stream, fast_scratch_[0]);
   else
@@ -732,25 +734,44 @@ uint32_t GraphEngine::visited_hash_capacity() const { return host_.nrows >= (1u 
 // more CTAs per SM: 1M x 128: plain kernel +17 %, QG +18 %, results unchanged).
 uint32_t GraphEngine::candidate_list_capacity() const { return host_.nrows >= (1u << 18) ? 512u : 1024u; }
 
-size_t GraphEngine::exact_launch_config(uint32_t max_size, ExactConfig& cfg) const {
+size_t GraphEngine::exact_launch_config(uint32_t max_size, ExactConfig& cfg, uint32_t threads) const {
   cfg = ExactConfig{};
   cfg.kcap = max_size + 1;
-  cfg.ccap = std::max<uint32_t>(candidate_list_capacity(), std::min<uint32_t>(1024, next_pow2(cfg.kcap)));
-  cfg.hcap = visited_hash_capacity();
+  // a short shared list: what it cannot hold waits in the overflow tier, and a step merges
+  // less (1M x 128, 10,000 queries: 1024 keys 42.5 ms, 512 35.0 ms, 256 34.4 ms)
+  cfg.ccap = std::min<uint32_t>(1024, std::max<uint32_t>(256, next_pow2(cfg.kcap)));
+  // the visited set: a bitmap in shared memory of at most 32 KB (200,000 objects, 25 KB:
+  // 1,500 queries in 1.03 ms against 1.10 ms with a hash that moves to global memory;
+  // 50,000 objects, 6 KB: 10,000 queries in 1.14 against 1.22 ms), else a small hash, from
+  // which every query of a large index moves to its global bitmap soon anyway
+  cfg.hcap = 2048;
   cfg.mode = (uint32_t)mode_;
   cfg.group = std::min<uint32_t>(32, next_pow2((uint32_t)dev_.row_chunks));
   cfg.bitmap_words = (host_.nrows + 31) / 32;
   cfg.ocap = kOverflowCapacity;
   int max_smem = 0;
   NGT_CUDA(cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, device_));
-  size_t smem = exact_smem_bytes(dev_.row_chunks, cfg);
-  while (smem > (size_t)max_smem && cfg.hcap > 2048) {
+  if (threads == 512) {
+    // the query has an SM to itself: a visited bitmap in shared memory where it fits (up
+    // to about 1.6M objects), else a larger hash
+    cfg.hcap = cfg.bitmap_words;
+    cfg.smem_bitmap = 1;
+    const size_t smem = exact_smem_bytes(dev_.row_chunks, cfg, threads);
+    if (smem <= (size_t)max_smem) return smem;
+    cfg.smem_bitmap = 0;
+    cfg.hcap = 16384;
+  } else if (cfg.bitmap_words <= 8192) {
+    cfg.smem_bitmap = 1;
+    cfg.hcap = cfg.bitmap_words;
+  }
+  size_t smem = exact_smem_bytes(dev_.row_chunks, cfg, threads);
+  while (smem > (size_t)max_smem && !cfg.smem_bitmap && cfg.hcap > 2048) {
     cfg.hcap >>= 1;
-    smem = exact_smem_bytes(dev_.row_chunks, cfg);
+    smem = exact_smem_bytes(dev_.row_chunks, cfg, threads);
   }
   while (smem > (size_t)max_smem && cfg.ccap > 256) {
     cfg.ccap >>= 1;
-    smem = exact_smem_bytes(dev_.row_chunks, cfg);
+    smem = exact_smem_bytes(dev_.row_chunks, cfg, threads);
   }
   if (smem > (size_t)max_smem) throw std::runtime_error("result size too large for the on-chip search state");
   return smem;
@@ -759,14 +780,16 @@ size_t GraphEngine::exact_launch_config(uint32_t max_size, ExactConfig& cfg) con
 void GraphEngine::launch_exact(const uint4* d_rows, size_t nq, const QueryParams* d_params, const uint32_t* d_seeds,
                                uint32_t max_size, ObjDist* d_out, uint32_t* d_counts, QueryStats* d_stats,
                                cudaStream_t stream, uint32_t* bitmaps, unsigned long long* overflow,
-                               size_t grid_cap) {
+                               size_t grid_cap, uint32_t* work) {
   ExactConfig cfg;
-  const size_t smem = exact_launch_config(max_size, cfg);
-  ExactKernelFn fn = exact_kernel(host_.prop.otype, host_.prop.metric);
-  NGT_CUDA(cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   int per_sm = 0, sms = 0;
-  NGT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)fn, kExactThreads, smem));
   NGT_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device_));
+  // a launch of no more CTAs than SMs leaves each query an SM: 512 threads per query
+  const uint32_t threads = (bitmaps ? std::min(nq, grid_cap) : nq) <= (size_t)sms ? 512u : (uint32_t)kExactThreads;
+  const size_t smem = exact_launch_config(max_size, cfg, threads);
+  ExactKernelFn fn = exact_kernel(host_.prop.otype, host_.prop.metric, threads);
+  NGT_CUDA(cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  NGT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)fn, (int)threads, smem));
   size_t grid = std::min<size_t>(nq, (size_t)std::max(1, per_sm) * sms);
   if (bitmaps) {
     grid = std::min(grid, grid_cap);
@@ -775,8 +798,12 @@ void GraphEngine::launch_exact(const uint4* d_rows, size_t nq, const QueryParams
     bitmaps = d_bitmaps_;
     overflow = d_overflow_;
   }
-  fn<<<(unsigned)grid, kExactThreads, smem, stream>>>(dev_, d_rows, (uint32_t)nq, d_params, d_seeds, d_out, d_counts,
-                                                       d_stats, bitmaps, overflow, cfg);
+  if (work && grid < nq) {
+    cfg.work = work;
+    NGT_CUDA(cudaMemsetAsync(work, 0, 4, stream));
+  }
+  fn<<<(unsigned)grid, threads, smem, stream>>>(dev_, d_rows, (uint32_t)nq, d_params, d_seeds, d_out, d_counts,
+                                                d_stats, bitmaps, overflow, cfg);
   NGT_CUDA(cudaGetLastError());
   launches_++;
 }
@@ -1298,7 +1325,7 @@ void GraphEngine::search_device_noalloc(void* scratch, size_t scratch_bytes, con
   uint32_t max_size = 0;
   build_params(args, nargs, nq, kmax, params, seeds, max_size);
   ExactConfig cfg;
-  const size_t smem = exact_launch_config(max_size, cfg);
+  const size_t smem = exact_launch_config(max_size, cfg, kExactThreads);
   // scratch layout: params | seeds | bitmaps[grid] | overflow[grid], each 256-byte aligned
   auto up = [](size_t v) { return (v + 255) & ~(size_t)255; };
   const size_t params_bytes = up(nq * sizeof(QueryParams));
@@ -1653,17 +1680,19 @@ void GraphEngine::qbg_probe_blobs(const uint4* d_rows, size_t nq, const QBGArgs*
     QueryParams* d_params = nullptr;
     uint32_t* d_seeds = nullptr;
     QueryStats* d_st = nullptr;
-    NGT_CUDA(cudaMallocAsync(&d_params, nq * sizeof(QueryParams), stream));
+    NGT_CUDA(cudaMallocAsync(&d_params, nq * sizeof(QueryParams) + 4, stream));
     NGT_CUDA(cudaMallocAsync(&d_seeds, seeds.size() * 4, stream));
     NGT_CUDA(cudaMallocAsync(&d_st, nq * sizeof(QueryStats), stream));
     NGT_CUDA(cudaMemcpyAsync(d_params, params.data(), nq * sizeof(QueryParams), cudaMemcpyHostToDevice, stream));
     NGT_CUDA(cudaMemcpyAsync(d_seeds, seeds.data(), seeds.size() * 4, cudaMemcpyHostToDevice, stream));
+    uint32_t* work = reinterpret_cast<uint32_t*>(d_params + nq);
     if (slot == 0) {
-      launch_exact(d_rows, nq, d_params, d_seeds, max_size, d_blobs, d_bcounts, d_st, stream);
+      launch_exact(d_rows, nq, d_params, d_seeds, max_size, d_blobs, d_bcounts, d_st, stream, nullptr, nullptr, 0,
+                   work);
     } else {
       QbgScratch& q = qbg_scratch_.at(slot);
       launch_exact(d_rows, nq, d_params, d_seeds, max_size, d_blobs, d_bcounts, d_st, stream, q.bitmaps,
-                   q.exact_ovf, q.grid);
+                   q.exact_ovf, q.grid, work);
     }
     // (the copies above read pageable host memory: staged before they return)
     NGT_CUDA(cudaFreeAsync(d_params, stream));

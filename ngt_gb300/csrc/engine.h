@@ -267,9 +267,10 @@ class GraphEngine {
   void search_device_noalloc(void* scratch, size_t scratch_bytes, const uint4* d_rows, size_t nq,
                              const SearchArgs* args, size_t nargs, ObjDist* d_out, uint32_t* d_counts,
                              QueryStats* d_stats, size_t kmax, cudaStream_t stream);
-  // The exact kernel's configuration for result sizes up to max_size: fills cfg and
-  // returns its dynamic shared memory (shared by every exact launch path).
-  size_t exact_launch_config(uint32_t max_size, ExactConfig& cfg) const;
+  // The exact kernel's configuration for result sizes up to max_size and `threads` per
+  // query: fills cfg and returns its dynamic shared memory (shared by every exact launch
+  // path).
+  size_t exact_launch_config(uint32_t max_size, ExactConfig& cfg, uint32_t threads) const;
   void set_tuning(const FastTuning& t) { tuning_ = t; }
   const FastTuning& tuning() const { return tuning_; }
   bool fast_supported(Kernel k) const;
@@ -326,10 +327,13 @@ class GraphEngine {
   // search rows the wide kernel uses for this index and tuning
   SearchRows wide_search_rows();
  private:
-  // bitmaps / overflow: a caller's scratch for `grid_cap` CTAs (nullptr: the engine's own)
+  // bitmaps / overflow: a caller's scratch for `grid_cap` CTAs (nullptr: the engine's own);
+  // work: a word of this launch's own, from which its CTAs take the queries (nullptr: fixed
+  // strides)
   void launch_exact(const uint4* d_rows, size_t nq, const QueryParams* d_params, const uint32_t* d_seeds,
                     uint32_t max_size, ObjDist* d_out, uint32_t* d_counts, QueryStats* d_stats, cudaStream_t stream,
-                    uint32_t* bitmaps = nullptr, unsigned long long* overflow = nullptr, size_t grid_cap = 0);
+                    uint32_t* bitmaps = nullptr, unsigned long long* overflow = nullptr, size_t grid_cap = 0,
+                    uint32_t* work = nullptr);
   void launch_fast(const uint4* d_rows, size_t nq, const QueryParams* d_params, const uint32_t* d_seeds,
                    uint32_t max_size, ObjDist* d_out, uint32_t* d_counts, QueryStats* d_stats, cudaStream_t stream,
                    Kernel kernel, FastScratch& scratch);

@@ -40,41 +40,50 @@ constexpr int kExactThreads = 128;
 constexpr int kExactWarps = kExactThreads / 32;
 constexpr int kExactChunk = kExactThreads;   // neighbours processed per round
 
+// Neighbours processed per round by a CTA of T threads, at most one per thread.
+template <int T> constexpr int exact_chunk() { return T < 256 ? T : 256; }
+// Rows each group of threads keeps in flight while computing distances.
+// (One where a row has three sums: two rows' twenty-four would spill.)
+template <class A, int T> constexpr int exact_rows() { return T == 128 && A::kUseF12 ? 1 : 2; }
+
 struct ExactShared {
   float radius;
   uint32_t nres;
-  uint32_t head, tail, cur;
-  uint32_t nvisited;
-  uint32_t spilled;
-  uint32_t done;
-  uint32_t target;
-  uint32_t nnew;
-  uint32_t nbatch;
+  uint32_t keep;                  // neighbours of the round within the exploration radius
   uint32_t live_old;
-  uint32_t status;
-  uint32_t dc;
-  uint32_t expansions;
-  uint32_t edges;
   uint32_t seed_leaf;
-  uint32_t ovf_n;                 // entries in the global overflow tier
-  uint32_t ovf_tmp;
-  unsigned long long ovf_min;     // smallest key in the overflow tier (~0 when empty)
+  uint32_t seed_status;
+  uint32_t nmoved;                // refill: keys moved to shared memory
+  uint32_t ovf_n;                 // refill: keys left in the overflow tier
+  uint32_t sel_bin, sel_acc;
+  uint32_t query;
+  unsigned long long key_min, key_max;
   unsigned long long evict_min;
-  unsigned long long sel_prefix;
-  uint32_t sel_need;
-  uint32_t warp_cnt[kExactWarps];
+  __align__(16) uint32_t warp_cnt[8];
   uint32_t hist[256];
 };
 
 struct ExactConfig {
   uint32_t kcap;     // result capacity (>= max size in the batch)
   uint32_t ccap;     // candidate-list capacity
-  uint32_t hcap;     // visited hash capacity (power of two)
+  uint32_t hcap;     // visited hash capacity (power of two), or words of the shared-memory bitmap
   uint32_t mode;     // GraphMode
   uint32_t group;    // lanes per distance (power of two <= 32)
   uint32_t bitmap_words;  // words per CTA in the spill bitmap
   uint32_t ocap;          // overflow-tier capacity per CTA (keys)
+  uint32_t smem_bitmap;   // 1: the visited set is a bitmap of every id in shared memory (hcap words)
+  uint32_t* work;         // zeroed counter from which the CTAs take the queries; null: CTA i
+                          // takes queries i, i + grid, ...
 };
+
+// The next query of this CTA (nq or more: none); `at` is the query just searched (or
+// UINT32_MAX).  Executed by the whole CTA; sh: a shared word.
+__device__ __forceinline__ uint32_t exact_next_query(uint32_t at, uint32_t* work, uint32_t* sh) {
+  if (!work) return at == 0xffffffffu ? blockIdx.x : at + gridDim.x;
+  if (threadIdx.x == 0) *sh = atomicAdd(work, 1u);
+  __syncthreads();
+  return *sh;
+}
 
 __device__ __forceinline__ uint32_t hash_slot(uint32_t id, uint32_t mask) {
   return (id * 0x9E3779B1u) & mask;
@@ -190,46 +199,227 @@ __device__ __forceinline__ uint32_t upper_bound_dist(const unsigned long long* a
   return lo;
 }
 
-template <ObjType OT, Metric M>
-__global__ void __launch_bounds__(kExactThreads)
+// Ranks of the m <= T unique keys in[0..m), written sorted to out, by the whole CTA:
+// as many threads per key as the CTA has to spare (at most 8) split the comparisons.
+template <int T>
+__device__ __forceinline__ void rank_sort_split(const unsigned long long* in, unsigned long long* out, uint32_t m) {
+  uint32_t split = 1;
+  while (split < 8 && m * split * 2 <= (uint32_t)T) split *= 2;
+  const uint32_t i = threadIdx.x / split, sub = threadIdx.x & (split - 1);
+  const unsigned long long k = i < m ? in[i] : 0ull;
+  uint32_t r = 0;
+  if (i < m)
+    for (uint32_t j = sub; j < m; j += split) r += in[j] < k ? 1u : 0u;
+  for (uint32_t off = 1; off < split; off <<= 1) r += __shfl_xor_sync(0xffffffffu, r, off);
+  if (i < m && sub == 0) out[r] = k;
+}
+
+// Moves the smallest live keys of the overflow tier (ovf[0..n), scratch tmp) into the
+// empty shared list cl, sorted: entries above the exploration radius are dropped, and
+// when more than ccap live, a threshold is taken at the edge of a radix bin, so that at
+// least half of the list is filled and every key left behind is larger.  (Which keys
+// wait in which tier does not change the order of the pops.)  Returns the keys moved;
+// n and ovf_min are updated.  Executed by the whole CTA of T threads.
+template <int T>
+__device__ __noinline__ uint32_t exact_refill(unsigned long long* cl, uint32_t ccap, unsigned long long* ovf,
+                                              unsigned long long* tmp, uint32_t& n, unsigned long long& ovf_min,
+                                              float expR, ExactShared& s) {
+  const uint32_t tid = threadIdx.x, lane = tid & 31;
+  const uint32_t below = (1u << lane) - 1u;
+  if (tid == 0) {
+    s.nmoved = 0;
+    s.key_min = ~0ull;
+    s.key_max = 0ull;
+  }
+  __syncthreads();
+  unsigned long long mn = ~0ull, mx = 0ull;
+  for (uint32_t b = 0; b < n; b += T) {
+    const uint32_t i = b + tid;
+    const unsigned long long k = i < n ? ovf[i] : ~0ull;
+    const bool live = i < n && key_dist(k) <= expR;
+    const uint32_t mask = __ballot_sync(0xffffffffu, live);
+    uint32_t at = 0;
+    if (lane == 0 && mask) at = atomicAdd(&s.nmoved, (uint32_t)__popc(mask));
+    at = __shfl_sync(0xffffffffu, at, 0);
+    if (live) {
+      tmp[at + __popc(mask & below)] = k;
+      mn = k < mn ? k : mn;
+      mx = k > mx ? k : mx;
+    }
+  }
+  for (int off = 16; off > 0; off >>= 1) {
+    const unsigned long long a = __shfl_xor_sync(0xffffffffu, mn, off), c = __shfl_xor_sync(0xffffffffu, mx, off);
+    mn = a < mn ? a : mn;
+    mx = c > mx ? c : mx;
+  }
+  if (lane == 0 && mn != ~0ull) {
+    atomicMin(&s.key_min, mn);
+    atomicMax(&s.key_max, mx);
+  }
+  __syncthreads();
+  const uint32_t r = s.nmoved;
+  if (r <= ccap) {
+    for (uint32_t i = tid; i < r; i += T) cl[i] = tmp[i];
+    __syncthreads();
+    bitonic_sort(cl, r, ccap);
+    n = 0;
+    ovf_min = ~0ull;
+    return r;
+  }
+  // radix bins of 8 bits from the highest byte in which the keys differ
+  const unsigned long long diff = s.key_min ^ s.key_max;
+  int shift = (63 - __clzll((long long)diff)) / 8 * 8;
+  unsigned long long prefix = s.key_min >> shift >> 8 << 8 << shift;      // the common bits above the digit
+  uint32_t acc = 0;                    // keys below the prefix
+  unsigned long long thr;
+  while (true) {
+    for (uint32_t i = tid; i < 256; i += T) s.hist[i] = 0;
+    __syncthreads();
+    for (uint32_t i = tid; i < r; i += T) {
+      const unsigned long long x = tmp[i];
+      if ((x >> shift >> 8) == (prefix >> shift >> 8)) atomicAdd(&s.hist[(uint32_t)(x >> shift) & 255u], 1u);
+    }
+    __syncthreads();
+    if (tid < 32) {
+      // the bins that fit: the largest b with acc + (keys in bins below b) <= ccap
+      uint32_t c[8], sum = 0;
+#pragma unroll
+      for (int j = 0; j < 8; j++) {
+        c[j] = s.hist[lane * 8 + j];
+        sum += c[j];
+      }
+      uint32_t incl = sum;
+#pragma unroll
+      for (int off = 1; off < 32; off <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, incl, off);
+        if (lane >= (uint32_t)off) incl += y;
+      }
+      uint32_t run = acc + incl - sum, fit = 0, got = run;
+      if (run <= ccap)
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+          run += c[j];
+          if (run <= ccap) {
+            fit = j + 1;
+            got = run;
+          }
+        }
+      // bins fit in order: the last lane whose first bin starts within the capacity
+      const uint32_t okm = __ballot_sync(0xffffffffu, acc + incl - sum <= ccap);
+      if ((int)lane == 31 - __clz((int)okm)) {
+        s.sel_bin = lane * 8 + fit;
+        s.sel_acc = got;
+      }
+    }
+    __syncthreads();
+    const uint32_t bin = s.sel_bin;
+    acc = s.sel_acc;
+    __syncthreads();
+    thr = prefix + ((unsigned long long)bin << shift) - 1ull;
+    if (acc >= ccap / 2 || shift == 0 || bin > 255) break;
+    prefix += (unsigned long long)bin << shift;          // the bin that does not fit, split further
+    shift -= 8;
+  }
+  if (tid == 0) {
+    s.nmoved = 0;
+    s.ovf_n = 0;
+    s.key_min = ~0ull;
+  }
+  __syncthreads();
+  mn = ~0ull;
+  for (uint32_t b = 0; b < r; b += T) {
+    const uint32_t i = b + tid;
+    const unsigned long long k = i < r ? tmp[i] : ~0ull;
+    const bool take = i < r && k <= thr, leave = i < r && k > thr;
+    const uint32_t tm = __ballot_sync(0xffffffffu, take), lm = __ballot_sync(0xffffffffu, leave);
+    uint32_t at = 0, al = 0;
+    if (lane == 0) {
+      if (tm) at = atomicAdd(&s.nmoved, (uint32_t)__popc(tm));
+      if (lm) al = atomicAdd(&s.ovf_n, (uint32_t)__popc(lm));
+    }
+    at = __shfl_sync(0xffffffffu, at, 0);
+    al = __shfl_sync(0xffffffffu, al, 0);
+    if (take) cl[at + __popc(tm & below)] = k;
+    if (leave) {
+      ovf[al + __popc(lm & below)] = k;
+      mn = k < mn ? k : mn;
+    }
+  }
+  for (int off = 16; off > 0; off >>= 1) {
+    const unsigned long long a = __shfl_xor_sync(0xffffffffu, mn, off);
+    mn = a < mn ? a : mn;
+  }
+  if (lane == 0 && mn != ~0ull) atomicMin(&s.key_min, mn);
+  __syncthreads();
+  n = s.ovf_n;
+  ovf_min = s.key_min;
+  const uint32_t moved = s.nmoved;
+  bitonic_sort(cl, moved, ccap);
+  __syncthreads();
+  return moved;
+}
+
+// Bound by latency: each expansion is a chain of dependent accesses (the node's offsets,
+// its edges, their visited bits, the new rows) and the chunk's bookkeeping between CTA
+// barriers.  What keeps the chain short:
+//   * after the survivors of a chunk are sorted, the next node is known (the smaller of
+//     the list's head and the best survivor): its offsets and edges are loaded while the
+//     list is merged;
+//   * the loop's counters (list head and size, tier size, statistics) are computed alike
+//     by every thread, so a chunk takes five barriers, and a sixth when a neighbour
+//     enters the results (twelve before);
+//   * distances by packed groups of threads (packed_distances), two rows each in flight;
+//   * T: launches that leave SMs idle give each query 512 threads (128 float rows in
+//     flight instead of 32) and, where it fits, a visited bitmap in shared memory.
+// Measured on 1M x 128 float objects (fixed seeds, L2): single queries, k = 20, epsilon 0.1
+// (about 2,000 expansions): 25.0 ms before, 8.4 ms with 512 threads; 2,000 queries, k = 10,
+// epsilon 0.08: 17.3 -> 11.6 ms; 100 of them: 3.5 ms with 512 threads, 5.0 ms with 128;
+// 300 of them: 6.1 and 5.2 ms, so 512 threads serve launches of at most one CTA per SM.  Seven 128-thread CTAs per SM (72 registers): six 44.1 ms for 10,000
+// queries against 40.9 ms, nine (56 registers, more spills) 46.7 ms; then the work
+// counter, 40.9 -> 35.0 ms, and a shared list of 256 keys instead of 512, 34.4 ms.
+template <ObjType OT, Metric M, int T>
+__global__ void __launch_bounds__(T, T == 128 ? 7 : 1)
 graph_search_exact_kernel(DevGraph g, const uint4* __restrict__ queries, uint32_t nq,
                           const QueryParams* __restrict__ params, const uint32_t* __restrict__ seed_list,
                           ObjDist* __restrict__ out, uint32_t* __restrict__ out_count,
                           QueryStats* __restrict__ stats, uint32_t* __restrict__ bitmaps,
                           unsigned long long* __restrict__ overflow, ExactConfig cfg) {
+  constexpr uint32_t CH = (uint32_t)exact_chunk<T>();
+  constexpr uint32_t CW = CH / 32;                        // warps that hold a chunk's neighbours
+  constexpr int U = exact_rows<Acc<OT, M>, T>();
   extern __shared__ __align__(16) unsigned char smem[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint32_t rc = g.row_chunks;
   // ---- shared-memory carve-up -------------------------------------------
   uint4* qv = reinterpret_cast<uint4*>(smem);
   unsigned long long* res = reinterpret_cast<unsigned long long*>(qv + rc);
-  unsigned long long* cand0 = res + cfg.kcap;
+  unsigned long long* cand0 = res + (cfg.kcap + 1) / 2 * 2;
   unsigned long long* cand1 = cand0 + cfg.ccap;
   unsigned long long* bkeys = cand1 + cfg.ccap;          // chunk survivors (unsorted)
-  unsigned long long* bsorted = bkeys + kExactChunk;     // chunk survivors (sorted)
-  uint32_t* table = reinterpret_cast<uint32_t*>(bsorted + kExactChunk);
-  uint32_t* nid = table + cfg.hcap;
-  float* nd = reinterpret_cast<float*>(nid + kExactChunk);
-  ExactShared& s = *reinterpret_cast<ExactShared*>(nd + kExactChunk);
+  unsigned long long* bsorted = bkeys + CH;              // chunk survivors (sorted)
+  uint32_t* table = reinterpret_cast<uint32_t*>(bsorted + CH);
+  uint32_t* seg = table + (cfg.hcap + 3) / 4 * 4;        // new ids, 32 slots per warp of the chunk
+  uint32_t* nid = seg + CH;                              // new ids in edge order
+  float* nd = reinterpret_cast<float*>(nid + CH);
+  ExactShared& s = *reinterpret_cast<ExactShared*>(nd + CH);
   uint32_t* bitmap = bitmaps + (size_t)blockIdx.x * cfg.bitmap_words;
   unsigned long long* ovf = overflow + (size_t)blockIdx.x * 2 * cfg.ocap;     // overflow tier
   unsigned long long* ovf_tmp = ovf + cfg.ocap;                                 // refill scratch
   const uint32_t hmask = cfg.hcap - 1;
   const int G = (int)cfg.group;
   const int gl = lane & (G - 1);                   // lane inside the distance group
-  const int ngroups = kExactThreads / G;
+  const uint32_t ngroups = T / G;
+  const int pw = packed_width(G);                  // threads per row in the loop
+  const uint32_t npacked = T / pw;
 
-  for (uint32_t q = blockIdx.x; q < nq; q += gridDim.x) {
+  for (uint32_t q = exact_next_query(0xffffffffu, cfg.work, &s.query); q < nq;
+       q = exact_next_query(q, cfg.work, &s.query)) {
     const QueryParams P = params[q];
     // ---- per-query initialisation ----------------------------------------
-    for (uint32_t i = tid; i < rc; i += blockDim.x) qv[i] = queries[(size_t)q * rc + i];
-    for (uint32_t i = tid; i < cfg.hcap; i += blockDim.x) table[i] = 0u;
-    if (tid == 0) {
-      s.radius = P.radius;
-      s.nres = 0; s.head = 0; s.tail = 0; s.cur = 0; s.nvisited = 0; s.spilled = 0;
-      s.done = 0; s.status = 0; s.dc = 0; s.expansions = 0; s.nnew = 0;
-      s.ovf_n = 0; s.ovf_min = ~0ull; s.edges = 0;
-    }
+    for (uint32_t i = tid; i < rc; i += T) qv[i] = queries[(size_t)q * rc + i];
+    for (uint32_t i = tid; i < (cfg.hcap + 3) / 4; i += T)
+      reinterpret_cast<uint4*>(table)[i] = make_uint4(0u, 0u, 0u, 0u);
+    if (tid == 0) s.seed_status = 0;
     __syncthreads();
     if (P.size == 0) {          // GraphIndex::search returns nothing for size 0
       if (tid == 0) { out_count[q] = 0; stats[q] = QueryStats{0, 0, 0, 0, 0}; }
@@ -255,7 +445,7 @@ graph_search_exact_kernel(DevGraph g, const uint4* __restrict__ queries, uint32_
         }
         if (lane == 0) {
           if (node & 0x80000000u) s.seed_leaf = node & 0x7fffffffu;
-          else { s.seed_leaf = 0xffffffffu; s.status |= kStatusTreeError; }
+          else { s.seed_leaf = 0xffffffffu; s.seed_status = kStatusTreeError; }
         }
       }
       __syncthreads();
@@ -270,10 +460,11 @@ graph_search_exact_kernel(DevGraph g, const uint4* __restrict__ queries, uint32_
       nseeds = P.seed_cnt;
     }
     nseeds = min(nseeds, (uint32_t)kExactChunk);
+    uint32_t status = s.seed_status;
     if (nseeds == 0) {
       if (tid == 0) {
         out_count[q] = 0;
-        stats[q] = QueryStats{0, 0, 0, 0, s.status | kStatusEmptySeeds};
+        stats[q] = QueryStats{0, 0, 0, 0, status | kStatusEmptySeeds};
       }
       __syncthreads();
       continue;
@@ -295,7 +486,7 @@ graph_search_exact_kernel(DevGraph g, const uint4* __restrict__ queries, uint32_
     // marked visited and become candidates.
     if (tid == 0) {
       uint32_t n = 0;
-      float radius = s.radius;
+      float radius = P.radius;
       for (uint32_t i = 0; i < nseeds; i++) {
         float d = key_dist(bsorted[i]);
         if (n < P.size && d <= radius) res[n++] = bsorted[i];
@@ -304,234 +495,191 @@ graph_search_exact_kernel(DevGraph g, const uint4* __restrict__ queries, uint32_
       if (n >= P.size) radius = key_dist(res[n - 1]);
       s.nres = n;
       s.radius = radius;
-      s.dc = nseeds;
-      s.tail = nseeds;
     }
-    for (uint32_t i = tid; i < nseeds; i += blockDim.x) {
+    for (uint32_t i = tid; i < nseeds; i += T) {
       cand0[i] = bsorted[i];
-      visit_insert(table, hmask, bitmap, false, key_id(bsorted[i]));
+      const uint32_t id = key_id(bsorted[i]);
+      if (cfg.smem_bitmap) {
+        if (id < g.nrows) atomicOr(&table[id >> 5], 1u << (id & 31u));
+      } else {
+        visit_insert(table, hmask, bitmap, false, id);
+      }
     }
-    if (tid == 0) s.nvisited = nseeds;
     __syncthreads();
 
     // ---- best-first loop -----------------------------------------------------
+    // Alike in every thread: the shared list is cl[head..tail) (cl: cand1 when cur), the
+    // overflow tier holds ovf_n keys, the smallest ovf_min.
+    uint32_t head = 0, tail = nseeds, cur = 0, ovf_n = 0;
+    unsigned long long ovf_min = ~0ull;
+    uint32_t nvisited = nseeds, dc = nseeds, expansions = 0, edges = 0;
+    bool spilled = false, have = false;
+    float radius = s.radius;
+    uint32_t e0 = 0, nsz = 0, eid = 0;            // the node to expand: edges, this thread's neighbour
     uint32_t guard = 0;
     while (true) {
-      if (s.head >= s.tail && s.ovf_n > 0) {
-        // ---- refill the shared list from the overflow tier ----
-        const float expR0 = P.coef * s.radius;
-        const uint32_t r0 = s.ovf_n;
-        if (tid == 0) s.ovf_tmp = 0;
-        __syncthreads();
-        for (uint32_t i = tid; i < r0; i += blockDim.x) {      // drop entries above the radius
-          unsigned long long k = ovf[i];
-          if (key_dist(k) <= expR0) ovf_tmp[atomicAdd(&s.ovf_tmp, 1u)] = k;
+      if (!have) {
+        if (head >= tail && ovf_n > 0) {
+          head = 0;
+          tail = exact_refill<T>(cur ? cand1 : cand0, cfg.ccap, ovf, ovf_tmp, ovf_n, ovf_min, P.coef * radius, s);
         }
-        __syncthreads();
-        const uint32_t r = s.ovf_tmp;
-        unsigned long long* cl = s.cur ? cand1 : cand0;
-        if (r <= cfg.ccap) {
-          for (uint32_t i = tid; i < r; i += blockDim.x) cl[i] = ovf_tmp[i];
-          __syncthreads();
-          bitonic_sort(cl, r, cfg.ccap);
-          if (tid == 0) { s.head = 0; s.tail = r; s.ovf_n = 0; s.ovf_min = ~0ull; }
-        } else {
-          // exact radix select of the ccap-th smallest 64-bit key
-          unsigned long long prefix = 0, mask = 0;
-          uint32_t need = cfg.ccap;
-          for (int shift = 56; shift >= 0; shift -= 8) {
-            for (uint32_t i = tid; i < 256; i += blockDim.x) s.hist[i] = 0;
-            __syncthreads();
-            for (uint32_t i = tid; i < r; i += blockDim.x) {
-              unsigned long long k = ovf_tmp[i];
-              if ((k & mask) == prefix) atomicAdd(&s.hist[(uint32_t)(k >> shift) & 255u], 1u);
-            }
-            __syncthreads();
-            if (tid == 0) {
-              uint32_t acc = 0, b;
-              for (b = 0; b < 255; b++) {
-                if (acc + s.hist[b] >= need) break;
-                acc += s.hist[b];
-              }
-              s.sel_prefix = prefix | ((unsigned long long)b << shift);
-              s.sel_need = need - acc;
-            }
-            __syncthreads();
-            prefix = s.sel_prefix;
-            need = s.sel_need;
-            mask |= 255ull << shift;
-            __syncthreads();
-          }
-          // keys <= prefix (exactly ccap) go to shared memory, the rest stay in the tier
-          if (tid == 0) { s.ovf_n = 0; s.nnew = 0; s.ovf_min = ~0ull; }
-          __syncthreads();
-          for (uint32_t i = tid; i < r; i += blockDim.x) {
-            unsigned long long k = ovf_tmp[i];
-            if (k <= prefix) {
-              cl[atomicAdd(&s.nnew, 1u)] = k;
-            } else {
-              ovf[atomicAdd(&s.ovf_n, 1u)] = k;
-              atomicMin(&s.ovf_min, k);
-            }
-          }
-          __syncthreads();
-          bitonic_sort(cl, cfg.ccap, cfg.ccap);
-          if (tid == 0) { s.head = 0; s.tail = cfg.ccap; }
-        }
-        __syncthreads();
+        if (head >= tail) break;
+        const unsigned long long t = (cur ? cand1 : cand0)[head];
+        if (key_dist(t) > P.coef * radius) break;
+        head++;
+        e0 = g.offsets[key_id(t)];
+        nsz = min(g.offsets[key_id(t) + 1] - e0, P.edge_size);
+        if ((uint32_t)tid < min(nsz, CH)) eid = g.edges[e0 + tid];
       }
-      if (tid == 0) {
-        unsigned long long* cl = s.cur ? cand1 : cand0;
-        float expR = P.coef * s.radius;
-        if (s.head >= s.tail) {
-          s.done = 1;
-        } else {
-          unsigned long long t = cl[s.head++];
-          if (key_dist(t) > expR) s.done = 1;
-          else { s.target = key_id(t); s.expansions++; }
-        }
-      }
-      __syncthreads();
-      if (s.done) break;
-      if (++guard > g.nrows + 8) {     // cannot happen: each id is expanded at most once
-        if (tid == 0) s.status |= kStatusIterationLimit;
+      have = false;
+      if (guard++ > g.nrows + 8) {     // cannot happen: each id is expanded at most once
+        status |= kStatusIterationLimit;
         break;
       }
-      const uint32_t target = s.target;
-      const uint32_t e0 = g.offsets[target];
-      const uint32_t deg = g.offsets[target + 1] - e0;
-      const uint32_t nsz = min(deg, P.edge_size);
-      if (tid == 0) s.edges += nsz;
-      for (uint32_t c0 = 0; c0 < nsz; c0 += kExactChunk) {
-        const uint32_t clen = min((uint32_t)kExactChunk, nsz - c0);
+      expansions++;
+      edges += nsz;
+      bool finished = false;
+      const uint32_t n_edges = nsz;                // nsz and e0 move on to the next node in the last chunk
+      for (uint32_t c0 = 0; c0 < n_edges; c0 += CH) {
+        const uint32_t clen = min(CH, n_edges - c0);
         // spill the visited set to the bitmap before it gets more than half full
-        if (!s.spilled && s.nvisited + clen > (cfg.hcap >> 1)) {
-          for (uint32_t i = tid; i < cfg.hcap; i += blockDim.x) {
+        if (!cfg.smem_bitmap && !spilled && nvisited + clen > (cfg.hcap >> 1)) {
+          for (uint32_t i = tid; i < cfg.hcap; i += T) {
             uint32_t id = table[i];
             if (id) atomicOr(&bitmap[id >> 5], 1u << (id & 31u));
           }
           __threadfence_block();
           __syncthreads();
-          if (tid == 0) { s.spilled = 1; s.status |= kStatusVisitedSpill; }
+          spilled = true;
+          status |= kStatusVisitedSpill;
+        }
+        // visited filter in edge order; each warp packs its new ids
+        if ((uint32_t)warp < CW) {
+          bool isnew = false;
+          if ((uint32_t)tid < clen) {
+            if (cfg.smem_bitmap) {
+              const uint32_t bit = 1u << (eid & 31u);
+              isnew = (atomicOr(&table[eid >> 5], bit) & bit) == 0u;
+            } else {
+              isnew = visit_insert(table, hmask, bitmap, spilled, eid);
+            }
+          }
+          const unsigned ballot = __ballot_sync(0xffffffffu, isnew);
+          if (isnew) seg[warp * 32 + __popc(ballot & ((1u << lane) - 1u))] = eid;
+          if (lane == 0) s.warp_cnt[warp] = __popc(ballot);
+        }
+        if (tid == 0) s.keep = 0;
+        __syncthreads();
+        uint32_t pre[CW + 1];                     // new ids before each warp's
+        pre[0] = 0;
+#pragma unroll
+        for (uint32_t w = 0; w < CW; w++) pre[w + 1] = pre[w] + s.warp_cnt[w];
+        const uint32_t nnew = pre[CW];
+        // distances, U rows per group of threads in flight
+        bool pass = false;
+        for (uint32_t b = (uint32_t)(warp * (32 / pw)); b < nnew; b += npacked * U) {
+          uint32_t id[U];
+          float d[U];
+#pragma unroll
+          for (int u = 0; u < U; u++) {
+            const uint32_t i = b + u * npacked + (uint32_t)(lane / pw);
+            uint32_t at = i;
+#pragma unroll
+            for (uint32_t w = 1; w < CW; w++) at = i >= pre[w] ? w * 32 + i - pre[w] : at;
+            id[u] = i < nnew ? seg[at] : 0u;
+          }
+          packed_distances<OT, M, U>(qv, g.objects, id, (int)rc, lane & (pw - 1), G, d);
+#pragma unroll
+          for (int u = 0; u < U; u++) {
+            const uint32_t i = b + u * npacked + (uint32_t)(lane / pw);
+            if (i < nnew && (lane & (pw - 1)) == 0) {
+              nd[i] = d[u];
+              nid[i] = id[u];
+              pass = pass || (d[u] <= radius && d[u] <= P.coef * radius);
+            }
+          }
+        }
+        // sequential replay of the result-set updates (warp 0), when there is one
+        if (__syncthreads_or(pass ? 1 : 0)) {
+          if (warp == 0) {
+            uint32_t n = s.nres;
+            float rad = radius;
+            for (uint32_t b = 0; b < nnew; b += 32) {
+              uint32_t i = b + lane;
+              // a neighbour joins when within the exploration radius and the radius
+              // of that moment (both only shrink; with epsilon < 0 the first is
+              // the tighter one)
+              float d = i < nnew ? nd[i] : FLT_MAX;
+              float lim = fminf(rad, P.coef * rad);
+              unsigned m = __ballot_sync(0xffffffffu, i < nnew && d <= lim);
+              while (m) {
+                int src = __ffs(m) - 1;
+                float dj = __shfl_sync(0xffffffffu, d, src);
+                uint32_t idj = nid[b + src];
+                if (dj <= rad && dj <= P.coef * rad)
+                  result_insert(res, n, rad, P.size, cfg.mode, pack_key(dj, idj), lane);
+                m &= (src == 31) ? 0u : ~((2u << src) - 1u);
+                lim = fminf(rad, P.coef * rad);
+                m &= __ballot_sync(0xffffffffu, i < nnew && d <= lim);
+              }
+            }
+            if (lane == 0) {
+              s.radius = rad;
+              s.nres = n;
+            }
+          }
           __syncthreads();
+          radius = s.radius;
         }
-        const bool spilled = s.spilled != 0;
-        // visited filter in edge order + order-preserving compaction
-        bool isnew = false;
-        uint32_t id = 0;
-        if ((uint32_t)tid < clen) {
-          id = g.edges[e0 + c0 + tid];
-          isnew = visit_insert(table, hmask, bitmap, spilled, id);
-        }
-        unsigned ballot = __ballot_sync(0xffffffffu, isnew);
-        if (lane == 0) s.warp_cnt[warp] = __popc(ballot);
-        __syncthreads();
-        uint32_t base = 0;
-        for (int w = 0; w < warp; w++) base += s.warp_cnt[w];
-        if (isnew) nid[base + __popc(ballot & ((1u << lane) - 1u))] = id;
-        __syncthreads();
-        uint32_t nnew = 0;
-        for (int w = 0; w < kExactWarps; w++) nnew += s.warp_cnt[w];
-        // distances
-        if (rc <= (uint32_t)G) {
-          // one 16-byte chunk per lane per row: U rows per group in flight
-          constexpr int U = 4;
-          const uint4 q1 = (uint32_t)gl < rc ? qv[gl] : make_uint4(0, 0, 0, 0);
-          const uint32_t step = (uint32_t)ngroups;
-          for (uint32_t b = (uint32_t)(warp * (32 / G)); b < nnew; b += step * U) {
-            uint4 xv[U];
-            uint32_t iu[U];
-#pragma unroll
-            for (int u = 0; u < U; u++) {
-              iu[u] = b + u * step + (uint32_t)(lane / G);
-              uint32_t v = iu[u] < nnew ? nid[iu[u]] : 0u;
-              xv[u] = (uint32_t)gl < rc ? __ldg(g.objects + (size_t)v * rc + gl) : make_uint4(0, 0, 0, 0);
-            }
-#pragma unroll
-            for (int u = 0; u < U; u++) {
-              Acc<OT, M> acc;
-              if ((uint32_t)gl < rc) acc.add(q1, xv[u], gl);
-              acc.reduce(G);
-              float d = acc.finish();
-              if (iu[u] < nnew && gl == 0) nd[iu[u]] = d;
-            }
-          }
-        } else {
-          for (uint32_t b = (uint32_t)(warp * (32 / G)); b < nnew; b += ngroups) {
-            uint32_t i = b + (uint32_t)(lane / G);
-            bool valid = i < nnew;
-            uint32_t v = valid ? nid[i] : 0u;
-            float d = group_distance<OT, M>(qv, g.objects + (size_t)v * rc, (int)rc, gl, G);
-            if (valid && gl == 0) nd[i] = d;
-          }
-        }
-        __syncthreads();
-        // sequential replay of the result-set updates (warp 0)
-        if (warp == 0) {
-          float radius = s.radius;
-          uint32_t n = s.nres;
-          for (uint32_t b = 0; b < nnew; b += 32) {
-            uint32_t i = b + lane;
-            // a neighbour joins when within the exploration radius and the radius
-            // of that moment (both only shrink; with epsilon < 0 the first is
-            // the tighter one)
-            float d = i < nnew ? nd[i] : FLT_MAX;
-            float lim = fminf(radius, P.coef * radius);
-            unsigned m = __ballot_sync(0xffffffffu, i < nnew && d <= lim);
-            while (m) {
-              int src = __ffs(m) - 1;
-              float dj = __shfl_sync(0xffffffffu, d, src);
-              uint32_t idj = nid[b + src];
-              if (dj <= radius && dj <= P.coef * radius)
-                result_insert(res, n, radius, P.size, cfg.mode, pack_key(dj, idj), lane);
-              m &= (src == 31) ? 0u : ~((2u << src) - 1u);
-              lim = fminf(radius, P.coef * radius);
-              m &= __ballot_sync(0xffffffffu, i < nnew && d <= lim);
-            }
-          }
-          if (lane == 0) {
-            s.radius = radius;
-            s.nres = n;
-            s.dc += nnew;
-            s.nvisited += nnew;
-          }
-        }
-        __syncthreads();
+        dc += nnew;
+        nvisited += nnew;
         // chunk survivors within the exploration radius become candidates
-        const float expR = P.coef * s.radius;
+        const float expR = P.coef * radius;
+        if (tid == 0) s.evict_min = ~0ull;
         {
-          bool keep = (uint32_t)tid < nnew && nd[tid] <= expR;
-          unsigned kb = __ballot_sync(0xffffffffu, keep);
-          if (lane == 0) s.warp_cnt[warp] = __popc(kb);
-          __syncthreads();
-          uint32_t kbase = 0;
-          for (int w = 0; w < warp; w++) kbase += s.warp_cnt[w];
-          if (keep) bkeys[kbase + __popc(kb & ((1u << lane) - 1u))] = pack_key(nd[tid], nid[tid]);
-          __syncthreads();
+          const bool keep = (uint32_t)tid < nnew && nd[tid] <= expR;
+          const unsigned kb = __ballot_sync(0xffffffffu, keep);
+          uint32_t at = 0;
+          if (lane == 0 && kb) at = atomicAdd(&s.keep, (uint32_t)__popc(kb));
+          at = __shfl_sync(0xffffffffu, at, 0);
+          if (keep) bkeys[at + __popc(kb & ((1u << lane) - 1u))] = pack_key(nd[tid], nid[tid]);
         }
-        uint32_t m = 0;
-        for (int w = 0; w < kExactWarps; w++) m += s.warp_cnt[w];
-        rank_sort(bkeys, bsorted, m);
-        unsigned long long* cl = s.cur ? cand1 : cand0;
-        unsigned long long* cn = s.cur ? cand0 : cand1;
-        if (tid == 0) {
-          // entries above the exploration radius can never be expanded again
-          s.live_old = upper_bound_dist(cl + s.head, s.tail - s.head, expR);
-        }
+        __syncthreads();
+        const uint32_t m = s.keep;
+        unsigned long long* cl = cur ? cand1 : cand0;
+        unsigned long long* cn = cur ? cand0 : cand1;
+        const unsigned long long* old = cl + head;
+        rank_sort_split<T>(bkeys, bsorted, m);
+        // entries above the exploration radius can never be expanded again
+        if (tid == T - 1) s.live_old = upper_bound_dist(old, tail - head, expR);
         __syncthreads();
         const uint32_t nold = s.live_old;
-        const unsigned long long* old = cl + s.head;
         // survivors not below the overflow tier's minimum join the tier directly
-        const uint32_t mk = s.ovf_n ? lower_bound_keys(bsorted, m, s.ovf_min) : m;
-        const uint32_t obase = s.ovf_n;
+        const uint32_t mk = ovf_n && m && bsorted[m - 1] >= ovf_min ? lower_bound_keys(bsorted, m, ovf_min) : m;
+        // the next node: its offsets load while the list is merged
+        const bool last = c0 + CH >= n_edges;
+        uint32_t o0 = 0, o1 = 0;
+        if (last) {
+          unsigned long long t = nold ? old[0] : ~0ull;
+          if (mk && bsorted[0] < t) t = bsorted[0];
+          if (nold + mk > 0) {
+            have = !(key_dist(t) > expR);
+            finished = !have;
+          }
+          if (have) {
+            o0 = __ldg(g.offsets + key_id(t));
+            o1 = __ldg(g.offsets + key_id(t) + 1);
+          }
+        } else if (tid < (int)CH && c0 + CH + tid < n_edges) {
+          eid = g.edges[e0 + c0 + CH + tid];
+        }
+        const uint32_t obase = ovf_n;
         const uint32_t nevict = (nold + mk > cfg.ccap) ? nold + mk - cfg.ccap : 0u;
-        if (tid == 0) s.evict_min = ~0ull;
-        __syncthreads();
-        for (uint32_t i = tid; i < m - mk; i += blockDim.x) {
+        for (uint32_t i = tid; i < m - mk; i += T) {
           uint32_t o = obase + i;
           if (o < cfg.ocap) ovf[o] = bsorted[mk + i];
         }
-        for (uint32_t i = tid; i < nold; i += blockDim.x) {
+        for (uint32_t i = tid; i < nold; i += T) {
           unsigned long long k = old[i];
           uint32_t pos = i + lower_bound_keys(bsorted, mk, k);
           if (pos < cfg.ccap) cn[pos] = k;
@@ -541,7 +689,7 @@ graph_search_exact_kernel(DevGraph g, const uint4* __restrict__ queries, uint32_
             if (pos == cfg.ccap) s.evict_min = k;
           }
         }
-        for (uint32_t i = tid; i < mk; i += blockDim.x) {
+        for (uint32_t i = tid; i < mk; i += T) {
           unsigned long long k = bsorted[i];
           uint32_t pos = i + lower_bound_keys(old, nold, k);
           if (pos < cfg.ccap) cn[pos] = k;
@@ -551,51 +699,52 @@ graph_search_exact_kernel(DevGraph g, const uint4* __restrict__ queries, uint32_
             if (pos == cfg.ccap) s.evict_min = k;
           }
         }
-        __syncthreads();
-        if (tid == 0) {
-          uint32_t added = (m - mk) + nevict;
-          if (added) {
-            unsigned long long mn = s.evict_min;
-            if (mk < m && bsorted[mk] < mn) mn = bsorted[mk];
-            if (mn < s.ovf_min) s.ovf_min = mn;
-            uint32_t n2 = s.ovf_n + added;
-            if (n2 > cfg.ocap) { n2 = cfg.ocap; s.status |= kStatusCandidateOverflow; }
-            s.ovf_n = n2;
-          }
-          s.head = 0;
-          s.tail = nold + mk - nevict;
-          s.cur ^= 1u;
+        if (have) {
+          e0 = o0;
+          nsz = min(o1 - o0, P.edge_size);
+          if ((uint32_t)tid < min(nsz, CH)) eid = g.edges[e0 + tid];
         }
         __syncthreads();
+        const uint32_t added = (m - mk) + nevict;
+        if (added) {
+          unsigned long long mn = s.evict_min;
+          if (mk < m && bsorted[mk] < mn) mn = bsorted[mk];
+          if (mn < ovf_min) ovf_min = mn;
+          ovf_n += added;
+          if (ovf_n > cfg.ocap) { ovf_n = cfg.ocap; status |= kStatusCandidateOverflow; }
+        }
+        head = have ? 1u : 0u;
+        tail = nold + mk - nevict;
+        cur ^= 1u;
       }
-      // every thread is done with this expansion's target before thread 0 pops the next one
-      __syncthreads();
+      if (finished) break;
     }
     // ---- results ---------------------------------------------------------------
     __syncthreads();
     {
       uint32_t n = s.nres;
       if (n > P.size_out) n = P.size_out;       // RESULT_DEFINED_RANGE: cut back to sizeBackup
-      for (uint32_t i = tid; i < n; i += blockDim.x) {
+      for (uint32_t i = tid; i < n; i += T) {
         unsigned long long k = res[i];
         out[P.out_off + i] = ObjDist{key_id(k), key_dist(k)};
       }
       if (tid == 0) {
         out_count[q] = n;
-        stats[q] = QueryStats{s.dc, s.expansions, s.nvisited, s.edges, s.status};
+        stats[q] = QueryStats{dc, expansions, nvisited, edges, status};
       }
     }
-    if (s.spilled) {                         // leave the bitmap clean for the next query
-      for (uint32_t i = tid; i < cfg.bitmap_words; i += blockDim.x) bitmap[i] = 0u;
+    if (spilled) {                           // leave the bitmap clean for the next query
+      for (uint32_t i = tid; i < cfg.bitmap_words; i += T) bitmap[i] = 0u;
       __threadfence();
     }
     __syncthreads();
   }
 }
 
-inline size_t exact_smem_bytes(uint32_t row_chunks, const ExactConfig& c) {
-  return (size_t)row_chunks * 16 + (size_t)c.kcap * 8 + (size_t)c.ccap * 16 + (size_t)kExactChunk * 16 +
-         (size_t)c.hcap * 4 + (size_t)kExactChunk * 8 + sizeof(ExactShared) + 16;
+inline size_t exact_smem_bytes(uint32_t row_chunks, const ExactConfig& c, uint32_t threads = kExactThreads) {
+  const size_t chunk = threads < 256 ? threads : 256;
+  return (size_t)row_chunks * 16 + ((size_t)c.kcap + 1) / 2 * 16 + (size_t)c.ccap * 16 + chunk * 16 +
+         ((size_t)c.hcap + 3) / 4 * 16 + chunk * 12 + sizeof(ExactShared) + 16;
 }
 
 }  // namespace ngtg

@@ -77,11 +77,12 @@ FastKernelFn fast_kernel(ObjType ot, Metric m, bool bf16_rows, uint32_t rows_in_
                          uint32_t ctas_per_sm = 0);
 void launch_float_rows_to_bf16(const void* in, void* out, size_t nfloats, cudaStream_t s);
 
-// Return nullptr when the (type, metric) pair is not supported.
-ExactKernelFn exact_kernel_float(Metric m);
-ExactKernelFn exact_kernel_half(Metric m);
-ExactKernelFn exact_kernel_u8(Metric m);
-ExactKernelFn exact_kernel_qs8(Metric m);
+// Return nullptr when the (type, metric) pair is not supported.  threads: 128 or 512
+// per query.
+ExactKernelFn exact_kernel_float(Metric m, uint32_t threads);
+ExactKernelFn exact_kernel_half(Metric m, uint32_t threads);
+ExactKernelFn exact_kernel_u8(Metric m, uint32_t threads);
+ExactKernelFn exact_kernel_qs8(Metric m, uint32_t threads);
 LinearKernelFn linear_kernel_float(Metric m);
 LinearKernelFn linear_kernel_half(Metric m);
 LinearKernelFn linear_kernel_u8(Metric m);

@@ -1,0 +1,94 @@
+"""The exact-order graph kernel where its forms meet: 512 threads per query up to one CTA
+per SM (152 on this chip), 128 above; the visited set as a bitmap or a hash in shared
+memory; rows of every lane-group width.  Results and counters against the oracle on random
+graphs; coordinates are whole numbers, so the distances are exact."""
+import os
+
+import numpy as np
+import pytest
+
+import oracle
+
+pytestmark = pytest.mark.gpu
+
+
+def _index(path, n, dim, degree, seed, bytes_=False):
+    from ngt_gb300.graph_build import write_index
+    rng = np.random.default_rng(seed)
+    x = rng.integers(0, 60, (n, dim)).astype(np.float32)
+    # neighbours near in id and far ones; ascending by distance as an index has them
+    near = (np.arange(n)[:, None] + rng.integers(1, 20, (n, degree // 2))) % n
+    to = np.concatenate([near, rng.integers(0, n, (n, degree - degree // 2))], 1)
+    d = np.sqrt(sum((x[:, None, c] - x[to, c]) ** 2 for c in range(dim)))
+    order = np.argsort(d, axis=1, kind="stable")
+    to, d = np.take_along_axis(to, order, 1), np.take_along_axis(d, order, 1)
+    offsets = np.concatenate([[0, 0], np.cumsum(np.full(n, degree))]).astype(np.int64)
+    write_index(path, x, offsets, (to + 1).reshape(-1).astype(np.uint32), d.reshape(-1).astype(np.float32))
+    if bytes_:
+        prf = open(os.path.join(path, "prf")).read().replace("ObjectType\tFloat-4", "ObjectType\tInteger-1")
+        open(os.path.join(path, "prf"), "w").write(prf)
+        rec = np.empty((n, 1 + dim), np.uint8)
+        rec[:, 0] = ord("+")
+        rec[:, 1:] = x
+        with open(os.path.join(path, "obj"), "wb") as f:
+            f.write(np.uint64(n + 1).tobytes() + b"-" + rec.tobytes())
+    return rng.integers(0, 60, (310, dim)).astype(np.float32)
+
+
+def _same(path, q, nqs, k, eps, mode="read_only"):
+    from ngt_gb300 import Index
+    o = oracle.Oracle(oracle.IndexFiles(path))
+    oi, od, on, dc = o.search(q, k=k, epsilon=eps, mode=mode, threads=8)
+    with Index(path, read_only=mode == "read_only") as ix:
+        for nq in nqs:
+            ids, ds, n, st = ix.batch_search(q[:nq], k=k, epsilon=eps, with_stats=True)
+            assert np.array_equal(n, on[:nq])
+            assert np.array_equal(st["distance_computations"], dc[:nq])
+            assert (st["status"] & 1 == 0).all()
+            for j in range(nq):
+                assert np.array_equal(ids[j, :n[j]], oi[j, :n[j]]), (nq, j)
+                assert np.array_equal(ds[j, :n[j]], od[j, :n[j]]), (nq, j)
+
+
+# the 128-thread kernel's visited bitmap in shared memory holds 262,144 ids (with id 0)
+@pytest.mark.parametrize("n", [300, 262_143, 262_144])
+def test_batch_sizes_and_visited_sets(tmp_path, n):
+    path = str(tmp_path / "ix")
+    q = _index(path, n, 4, 12, n)
+    _same(path, q, (1, 152, 153, 310), 10, 0.4)
+
+
+@pytest.mark.parametrize("dim,bytes_", [(10, True), (20, True), (40, True), (70, True), (3, False), (20, False),
+                                        (70, False), (129, False), (600, False)])
+def test_row_widths(tmp_path, dim, bytes_):
+    path = str(tmp_path / "ix")
+    q = _index(path, 2000, dim, 40, dim, bytes_)
+    for mode in ("read_only", "updatable"):
+        _same(path, q, (7, 310), 30, 0.1, mode)
+
+
+def test_long_edge_lists_and_refills(tmp_path):
+    """300 edges a node: several rounds per expansion, in either kernel; epsilon wide enough
+    that the overflow tier refills the shared list many times."""
+    path = str(tmp_path / "ix")
+    q = _index(path, 20_000, 8, 300, 5)
+    from ngt_gb300 import Index
+    o = oracle.Oracle(oracle.IndexFiles(path))
+    oi, od, on, dc = o.search(q[:160], k=50, epsilon=0.6, edge_size=0, threads=8)
+    with Index(path, read_only=True) as ix:
+        for nq in (5, 160):
+            ids, ds, n, st = ix.batch_search(q[:nq], k=50, epsilon=0.6, edge_size=0, with_stats=True)
+            assert np.array_equal(ids, oi[:nq, :50]) and np.array_equal(ds, od[:nq, :50])
+            assert np.array_equal(st["distance_computations"], dc[:nq])
+
+
+def test_large_index_without_a_shared_bitmap(tmp_path):
+    """1.9M objects: the 512-thread kernel falls back to its hash and the global bitmap."""
+    from ngt_gb300 import Index
+    path = str(tmp_path / "ix")
+    q = _index(path, 1_900_000, 2, 8, 9)
+    with Index(path, read_only=True) as ix:
+        a = ix.batch_search(q, k=10, epsilon=0.3, with_stats=True)
+        b = ix.batch_search(q[:20], k=10, epsilon=0.3, with_stats=True)
+    assert np.array_equal(a[0][:20], b[0]) and np.array_equal(a[1][:20], b[1])
+    assert np.array_equal(a[3]["distance_computations"][:20], b[3]["distance_computations"])
