@@ -60,6 +60,16 @@ __device__ __forceinline__ void unpack<ObjType::Uint8>(const uint4& v, float* f)
   for (int i = 0; i < 16; i++) f[i] = (float)((w[i >> 2] >> ((i & 3) * 8)) & 0xffu);
 }
 
+// a - b of two floats each, rounded as the scalar subtraction rounds.
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) {
+  float2 d;
+  asm("{\n .reg .b64 ra, rb, rd;\n mov.b64 ra, {%2, %3};\n mov.b64 rb, {%4, %5};\n"
+      " sub.rn.f32x2 rd, ra, rb;\n mov.b64 {%0, %1}, rd;\n}"
+      : "=f"(d.x), "=f"(d.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return d;
+}
+
 // Metric accumulator.  add() consumes one 16-byte chunk of the query and of
 // the row; chunk_index is the chunk's position in the row (Lorentz needs to
 // know which element is the first one).
@@ -108,6 +118,16 @@ struct Acc {
       float a[P], b[P];
       unpack<OT>(q, a);
       unpack<OT>(x, b);
+      if constexpr (OT == ObjType::Float && (M == Metric::L2 || M == Metric::InnerProduct)) {
+        // the differences two at a time (add.rn.f32x2), then the sum in element order
+#pragma unroll
+        for (int i = 0; i < P; i += 2) {
+          const float2 d = sub2(make_float2(a[i], a[i + 1]), make_float2(b[i], b[i + 1]));
+          f0 = __fmaf_rn(d.x, d.x, f0);
+          f0 = __fmaf_rn(d.y, d.y, f0);
+        }
+        return;
+      }
 #pragma unroll
       for (int i = 0; i < P; i++) {
         if constexpr (M == Metric::L2 || M == Metric::InnerProduct) {
@@ -202,6 +222,13 @@ struct Acc {
     if constexpr (kUseI1) i1 += o.i1;
   }
 
+  // Whether finish() is above `limit` beyond doubt, from far_limit(limit): for the float L2
+  // without its square root (the limit squared, with room for the rounding of either);
+  // never for the others.  False for NaN.
+  static constexpr bool kFar = kUseF0 && (M == Metric::L2 || M == Metric::InnerProduct);
+  static __device__ __forceinline__ float far_limit(float limit) { return kFar ? limit * limit * 1.00001f : limit; }
+  __device__ __forceinline__ bool is_far(float far) const { return kFar && f0 > far; }
+
   __device__ __forceinline__ float finish() const {
     if constexpr (OT == ObjType::Qsint8 && M == Metric::L2) {
       // the squared sum itself: PrimitiveComparator::compareL2(qsint8) of the x86
@@ -280,15 +307,15 @@ __device__ __forceinline__ float group_distance(const uint4* __restrict__ q, con
 // group_distance, width / 4 threads (at least one) each hold four of those lanes' sums
 // and add them in the order of reduce(), so every distance has group_distance's bits.
 // Bound by instruction issue where the rows are in flight already: a 512-byte float row
-// then takes about 18 warp instructions instead of 50 (two shuffle-and-adds fewer per
+// then takes about a third of the warp instructions (two shuffle-and-adds fewer per
 // row and lane, one square root per row and not per lane).  t: the thread's index inside
 // its packed_width(width) threads; all lanes of the warp take part.
 __device__ __forceinline__ int packed_width(int width) { return width >= 4 ? width >> 2 : 1; }
 
 template <ObjType OT, Metric M, int U>
-__device__ __forceinline__ void packed_distances(const uint4* __restrict__ q, const uint4* __restrict__ objects,
-                                                 const uint32_t (&id)[U], int nchunks, int t, int width,
-                                                 float (&d)[U]) {
+__device__ __forceinline__ void packed_sums(const uint4* __restrict__ q, const uint4* __restrict__ objects,
+                                            const uint32_t (&id)[U], int nchunks, int t, int width,
+                                            Acc<OT, M> (&sum)[U]) {
   const int pw = packed_width(width);
   Acc<OT, M> acc[U][4];
   for (int c0 = t; c0 < nchunks; c0 += width) {
@@ -319,7 +346,7 @@ __device__ __forceinline__ void packed_distances(const uint4* __restrict__ q, co
     }
     if (width >= 2) acc[u][0].fold(acc[u][1]);
     acc[u][0].reduce(pw);
-    d[u] = acc[u][0].finish();
+    sum[u] = acc[u][0];
   }
 }
 

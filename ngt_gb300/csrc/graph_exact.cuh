@@ -31,6 +31,7 @@
 // global memory when the table is half full.
 #pragma once
 #include <cfloat>
+#include <type_traits>
 #include "distance.cuh"
 #include "device_index.h"
 
@@ -49,7 +50,7 @@ template <class A, int T> constexpr int exact_rows() { return T == 128 && A::kUs
 struct ExactShared {
   float radius;
   uint32_t nres;
-  uint32_t keep;                  // neighbours of the round within the exploration radius
+  uint32_t keep[2];               // neighbours of the round within the exploration radius (rounds in turn)
   uint32_t live_old;
   uint32_t seed_leaf;
   uint32_t seed_status;
@@ -59,6 +60,7 @@ struct ExactShared {
   uint32_t query;
   unsigned long long key_min, key_max;
   unsigned long long evict_min;
+  unsigned long long edge[2];     // merge_results: the keys at places size - 1 and size
   __align__(16) uint32_t warp_cnt[8];
   uint32_t hist[256];
 };
@@ -199,6 +201,13 @@ __device__ __forceinline__ uint32_t upper_bound_dist(const unsigned long long* a
   return lo;
 }
 
+// Asks for the first KB of a row (rc 16-byte chunks) to be brought into L2.
+__device__ __forceinline__ void prefetch_row(const uint4* row, uint32_t rc) {
+#pragma unroll
+  for (uint32_t c = 0; c < 64; c += 8)
+    if (c < rc) asm volatile("prefetch.global.L2 [%0];" ::"l"(row + c));
+}
+
 // Ranks of the m <= T unique keys in[0..m), written sorted to out, by the whole CTA:
 // as many threads per key as the CTA has to spare (at most 8) split the comparisons.
 template <int T>
@@ -212,6 +221,102 @@ __device__ __forceinline__ void rank_sort_split(const unsigned long long* in, un
     for (uint32_t j = sub; j < m; j += split) r += in[j] < k ? 1u : 0u;
   for (uint32_t off = 1; off < split; off <<= 1) r += __shfl_xor_sync(0xffffffffu, r, off);
   if (i < m && sub == 0) out[r] = k;
+}
+
+// A round's updates of the result set res (n = s.nres keys, ascending) as one merge: the
+// neighbours within `radius` (a prefix of the sorted survivors sv[0..m)) join in edge
+// order nd / nid, exploration coefficient >= 1.  Executed by the whole CTA; false (nothing
+// changed) when the order of the updates could matter: the replay decides.
+//
+// What the sequence of updates leaves, without going through it: once the set is full and
+// `radius` is its largest distance, every update drops the maximum and takes a neighbour
+// no farther, so the distances kept are always the `size` smallest seen, and so are the
+// keys unless the distances at places size - 1 and size of the union are equal (then it
+// is the order that decides, read-only search; the updatable one keeps the smaller key).
+// The read-only search fills the set first, with the first size - n neighbours, and the
+// next one then replaces the maximum of that moment whatever it is, because the radius
+// still is the initial one: that maximum alone is missing from the union.
+// One by one, an update costs warp 0 about 400 cycles, and a search that approaches its
+// query takes most neighbours of its first expansions: half the time of short searches.
+template <int T>
+__device__ __noinline__ bool merge_results(unsigned long long* res, uint32_t size, uint32_t mode, float radius,
+                                           const unsigned long long* sv, uint32_t m, const float* nd,
+                                           const uint32_t* nid, uint32_t nnew, ExactShared& s) {
+  const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const uint32_t n = s.nres;
+  // below zero (the scalar-quantized inner product) the exploration radius is the tighter one
+  if (key_dist(sv[0]) < 0.f || (n && key_dist(res[0]) < 0.f)) return false;
+  const uint32_t p = upper_bound_dist(sv, m, radius);
+  const bool ro = mode == (uint32_t)GraphMode::ReadOnly;
+  const uint32_t fill = n < size ? size - n : 0u;
+  const bool stale = ro && n >= size && key_dist(res[n - 1]) != radius;
+  const bool removal = ro && ((fill && p > fill) || stale);
+  unsigned long long rem = ~0ull;
+  if (tid == 0) {
+    s.edge[0] = s.edge[1] = ~0ull;
+    s.key_max = n ? res[n - 1] : 0ull;
+  }
+  if (removal) {
+    const bool in = tid < nnew && nd[tid] <= radius;
+    const uint32_t mask = __ballot_sync(0xffffffffu, in);
+    if (lane == 0 && warp < 8) s.warp_cnt[warp] = __popc(mask);     // nnew <= 256: eight warps at most
+    __syncthreads();
+    if (in && fill) {
+      uint32_t o = __popc(mask & ((1u << lane) - 1u));
+      for (uint32_t w = 0; w < warp; w++) o += s.warp_cnt[w];
+      if (o < fill) atomicMax(&s.key_max, pack_key(nd[tid], nid[tid]));
+    }
+    __syncthreads();
+    rem = s.key_max;
+  } else {
+    __syncthreads();
+  }
+  const uint32_t total = n + p - (removal ? 1u : 0u);
+  // places of this thread's survivor, and the keys at the cut
+  unsigned long long mine = ~0ull;
+  uint32_t at = 0xffffffffu;
+  if (tid < p) {
+    mine = sv[tid];
+    if (!(removal && mine == rem)) {
+      at = tid + lower_bound_keys(res, n, mine) - (removal && mine > rem ? 1u : 0u);
+      if (at == size - 1) s.edge[0] = mine;
+      if (at == size) s.edge[1] = mine;
+    }
+  }
+  for (uint32_t i = tid; i < n; i += T) {
+    const unsigned long long r = res[i];
+    if (removal && r == rem) continue;
+    const uint32_t to = i + lower_bound_keys(sv, p, r) - (removal && r > rem ? 1u : 0u);
+    if (to == size - 1) s.edge[0] = r;
+    if (to == size) s.edge[1] = r;
+  }
+  __syncthreads();
+  if (ro && total > size && key_dist(s.edge[0]) == key_dist(s.edge[1])) {
+    __syncthreads();                         // s.edge is read before a later call resets it
+    return false;
+  }
+  // the old keys move up, from the top; then the survivors take their places
+  for (uint32_t top = n; top > 0;) {
+    const uint32_t b = top > (uint32_t)T ? top - T : 0u, i = b + tid;
+    unsigned long long r = ~0ull;
+    uint32_t to = 0xffffffffu;
+    if (i < top) {
+      r = res[i];
+      if (!(removal && r == rem)) to = i + lower_bound_keys(sv, p, r) - (removal && r > rem ? 1u : 0u);
+    }
+    __syncthreads();
+    if (to < size) res[to] = r;
+    __syncthreads();
+    top = b;
+  }
+  if (at < size) res[at] = mine;
+  if (tid == 0) {
+    s.nres = min(total, size);
+    const bool moved = ro ? n >= size || p > fill : total >= size;
+    s.radius = moved ? key_dist(s.edge[0]) : radius;
+  }
+  __syncthreads();
+  return true;
 }
 
 // Moves the smallest live keys of the overflow tier (ovf[0..n), scratch tmp) into the
@@ -359,26 +464,31 @@ __device__ __noinline__ uint32_t exact_refill(unsigned long long* cl, uint32_t c
   return moved;
 }
 
-// Bound by latency: each expansion is a chain of dependent accesses (the node's offsets,
-// its edges, their visited bits, the new rows) and the chunk's bookkeeping between CTA
-// barriers.  What keeps the chain short:
-//   * after the survivors of a chunk are sorted, the next node is known (the smaller of
-//     the list's head and the best survivor): its offsets and edges are loaded while the
-//     list is merged;
-//   * the loop's counters (list head and size, tier size, statistics) are computed alike
-//     by every thread, so a chunk takes five barriers, and a sixth when a neighbour
-//     enters the results (twelve before);
-//   * distances by packed groups of threads (packed_distances), two rows each in flight;
+// Bound by latency and instruction issue: each expansion is a chain of dependent accesses
+// (the node's offsets, its edges, their visited bits, the new rows) and the chunk's
+// bookkeeping between CTA barriers.  What keeps the chain short:
+//   * the list's head, which is the next node unless a survivor is nearer (four times in
+//     five), has its offsets and edges loaded beside the current node's rows; another next
+//     node's offsets load while the list is merged;
+//   * a chunk without survivors (two in three: nearly all neighbours are past the
+//     exploration radius) leaves the list as it is and takes two barriers; with survivors
+//     four (twelve before);
+//   * distances by packed groups of threads (packed_sums), two rows each in flight, and no
+//     square root for rows past the exploration radius;
+//   * result updates merged at once (merge_results);
 //   * T: launches that leave SMs idle give each query 512 threads (128 float rows in
 //     flight instead of 32) and, where it fits, a visited bitmap in shared memory.
 // Measured on 1M x 128 float objects (fixed seeds, L2): single queries, k = 20, epsilon 0.1
-// (about 2,000 expansions): 25.0 ms before, 8.4 ms with 512 threads; 2,000 queries, k = 10,
-// epsilon 0.08: 17.3 -> 11.6 ms; 100 of them: 3.5 ms with 512 threads, 5.0 ms with 128;
-// 300 of them: 6.1 and 5.2 ms, so 512 threads serve launches of at most one CTA per SM.  Seven 128-thread CTAs per SM (72 registers): six 44.1 ms for 10,000
-// queries against 40.9 ms, nine (56 registers, more spills) 46.7 ms; then the work
-// counter, 40.9 -> 35.0 ms, and a shared list of 256 keys instead of 512, 34.4 ms.
+// (about 2,000 expansions): 25.1 ms before, 6.4 ms with 512 threads; 2,000 queries, k = 10,
+// epsilon 0.08: 17.3 -> 10.7 ms; 100 of them: 2.8 ms with 512 threads, 5.0 ms with 128;
+// 300 of them: 6.1 and 5.2 ms, so 512 threads serve launches of at most one CTA per SM.
+// Six 128-thread CTAs per SM (80 registers): seven (72, spills) are as fast for L2 and
+// 5-8 % slower for cosine and short searches; four 56.5 ms, nine 46.7 ms for 10,000
+// queries against 44.1 ms; then the work counter and the shorter shared list, 33.9 ms.
+// Not kept: fetching a survivor's neighbours' rows into L2 when it joins the list (512
+// threads; 10 % slower), the result set in a warp's registers (slower than shared memory).
 template <ObjType OT, Metric M, int T>
-__global__ void __launch_bounds__(T, T == 128 ? 7 : 1)
+__global__ void __launch_bounds__(T, T == 128 ? 6 : 1)
 graph_search_exact_kernel(DevGraph g, const uint4* __restrict__ queries, uint32_t nq,
                           const QueryParams* __restrict__ params, const uint32_t* __restrict__ seed_list,
                           ObjDist* __restrict__ out, uint32_t* __restrict__ out_count,
@@ -419,7 +529,10 @@ graph_search_exact_kernel(DevGraph g, const uint4* __restrict__ queries, uint32_
     for (uint32_t i = tid; i < rc; i += T) qv[i] = queries[(size_t)q * rc + i];
     for (uint32_t i = tid; i < (cfg.hcap + 3) / 4; i += T)
       reinterpret_cast<uint4*>(table)[i] = make_uint4(0u, 0u, 0u, 0u);
-    if (tid == 0) s.seed_status = 0;
+    if (tid == 0) {
+      s.seed_status = 0;
+      s.keep[0] = s.keep[1] = 0;
+    }
     __syncthreads();
     if (P.size == 0) {          // GraphIndex::search returns nothing for size 0
       if (tid == 0) { out_count[q] = 0; stats[q] = QueryStats{0, 0, 0, 0, 0}; }
@@ -516,7 +629,7 @@ graph_search_exact_kernel(DevGraph g, const uint4* __restrict__ queries, uint32_
     bool spilled = false, have = false;
     float radius = s.radius;
     uint32_t e0 = 0, nsz = 0, eid = 0;            // the node to expand: edges, this thread's neighbour
-    uint32_t guard = 0;
+    uint32_t guard = 0, turn = 0;
     while (true) {
       if (!have) {
         if (head >= tail && ovf_n > 0) {
@@ -532,6 +645,14 @@ graph_search_exact_kernel(DevGraph g, const uint4* __restrict__ queries, uint32_
         if ((uint32_t)tid < min(nsz, CH)) eid = g.edges[e0 + tid];
       }
       have = false;
+      // the list's head is the next node unless this one has a nearer survivor: its edges
+      // load beside this node's rows
+      const unsigned long long guess = head < tail ? (cur ? cand1 : cand0)[head] : ~0ull;
+      uint32_t g0 = 0, g1 = 0, gid = 0;
+      if (head < tail) {
+        g0 = __ldg(g.offsets + key_id(guess));
+        g1 = __ldg(g.offsets + key_id(guess) + 1);
+      }
       if (guard++ > g.nrows + 8) {     // cannot happen: each id is expanded at most once
         status |= kStatusIterationLimit;
         break;
@@ -566,99 +687,142 @@ graph_search_exact_kernel(DevGraph g, const uint4* __restrict__ queries, uint32_
           }
           const unsigned ballot = __ballot_sync(0xffffffffu, isnew);
           if (isnew) seg[warp * 32 + __popc(ballot & ((1u << lane) - 1u))] = eid;
+          // the rows of later rounds are under way to L2 beside the first round's (10,000
+          // queries: 35.9 -> 33.5 ms; no gain with 512 threads, whose rounds take them all)
+          if (T == 128 && isnew) prefetch_row(g.objects + (size_t)eid * rc, rc);
           if (lane == 0) s.warp_cnt[warp] = __popc(ballot);
         }
-        if (tid == 0) s.keep = 0;
         __syncthreads();
         uint32_t pre[CW + 1];                     // new ids before each warp's
         pre[0] = 0;
 #pragma unroll
         for (uint32_t w = 0; w < CW; w++) pre[w + 1] = pre[w] + s.warp_cnt[w];
         const uint32_t nnew = pre[CW];
-        // distances, U rows per group of threads in flight
+        const bool last = c0 + CH >= n_edges;
+        if (last) {
+          if (head < tail && (uint32_t)tid < min(min(g1 - g0, P.edge_size), CH)) gid = __ldg(g.edges + g0 + tid);
+        } else if (tid < (int)CH && c0 + CH + tid < n_edges) {
+          eid = __ldg(g.edges + e0 + c0 + CH + tid);
+        }
+        const float expR0 = P.coef * radius;
+        // distances, U rows per group of threads in flight while that many are left
         bool pass = false;
-        for (uint32_t b = (uint32_t)(warp * (32 / pw)); b < nnew; b += npacked * U) {
-          uint32_t id[U];
-          float d[U];
+        const float far = Acc<OT, M>::far_limit(expR0);
+        auto rows = [&](auto rows_at_once, uint32_t b) {
+          constexpr int R = decltype(rows_at_once)::value;
+          uint32_t id[R];
+          Acc<OT, M> sum[R];
 #pragma unroll
-          for (int u = 0; u < U; u++) {
+          for (int u = 0; u < R; u++) {
             const uint32_t i = b + u * npacked + (uint32_t)(lane / pw);
             uint32_t at = i;
 #pragma unroll
             for (uint32_t w = 1; w < CW; w++) at = i >= pre[w] ? w * 32 + i - pre[w] : at;
             id[u] = i < nnew ? seg[at] : 0u;
           }
-          packed_distances<OT, M, U>(qv, g.objects, id, (int)rc, lane & (pw - 1), G, d);
+          packed_sums<OT, M, R>(qv, g.objects, id, (int)rc, lane & (pw - 1), G, sum);
 #pragma unroll
-          for (int u = 0; u < U; u++) {
+          for (int u = 0; u < R; u++) {
             const uint32_t i = b + u * npacked + (uint32_t)(lane / pw);
             if (i < nnew && (lane & (pw - 1)) == 0) {
-              nd[i] = d[u];
+              float d = FLT_MAX;                   // past the exploration radius: no more is asked of it
+              if (!sum[u].is_far(far)) {
+                d = sum[u].finish();
+                pass = pass || (d <= radius && d <= expR0);
+                if (d <= expR0) bkeys[atomicAdd(&s.keep[turn], 1u)] = pack_key(d, id[u]);
+              }
+              nd[i] = d;
               nid[i] = id[u];
-              pass = pass || (d[u] <= radius && d[u] <= P.coef * radius);
             }
+          }
+        };
+        for (uint32_t b = (uint32_t)(warp * (32 / pw)); b < nnew;) {
+          if (U > 1 && b + npacked < nnew) {
+            rows(std::integral_constant<int, U>(), b);
+            b += U * npacked;
+          } else {
+            rows(std::integral_constant<int, 1>(), b);
+            b += npacked;
           }
         }
-        // sequential replay of the result-set updates (warp 0), when there is one
-        if (__syncthreads_or(pass ? 1 : 0)) {
-          if (warp == 0) {
-            uint32_t n = s.nres;
-            float rad = radius;
-            for (uint32_t b = 0; b < nnew; b += 32) {
-              uint32_t i = b + lane;
-              // a neighbour joins when within the exploration radius and the radius
-              // of that moment (both only shrink; with epsilon < 0 the first is
-              // the tighter one)
-              float d = i < nnew ? nd[i] : FLT_MAX;
-              float lim = fminf(rad, P.coef * rad);
-              unsigned m = __ballot_sync(0xffffffffu, i < nnew && d <= lim);
-              while (m) {
-                int src = __ffs(m) - 1;
-                float dj = __shfl_sync(0xffffffffu, d, src);
-                uint32_t idj = nid[b + src];
-                if (dj <= rad && dj <= P.coef * rad)
-                  result_insert(res, n, rad, P.size, cfg.mode, pack_key(dj, idj), lane);
-                m &= (src == 31) ? 0u : ~((2u << src) - 1u);
-                lim = fminf(rad, P.coef * rad);
-                m &= __ballot_sync(0xffffffffu, i < nnew && d <= lim);
+        // the result-set updates, when there are some: merged at once, or (with epsilon < 0, or
+        // a tie at the last result) replayed one by one by warp 0
+        const bool replay = __syncthreads_or(pass ? 1 : 0) != 0;
+        uint32_t m = s.keep[turn];                // survivors: within the exploration radius
+        turn ^= 1u;
+        if (tid == 0) s.keep[turn] = 0;           // the next round's (last read two rounds ago)
+        if (replay) {
+          rank_sort_split<T>(bkeys, bsorted, m);
+          __syncthreads();
+          if (!(P.coef >= 1.0f) || !merge_results<T>(res, P.size, cfg.mode, radius, bsorted, m, nd, nid, nnew, s)) {
+            if (warp == 0) {
+              uint32_t n = s.nres;
+              float rad = radius;
+              for (uint32_t b = 0; b < nnew; b += 32) {
+                uint32_t i = b + lane;
+                // a neighbour joins when within the exploration radius and the radius
+                // of that moment (both only shrink; with epsilon < 0 the first is
+                // the tighter one)
+                float d = i < nnew ? nd[i] : FLT_MAX;
+                float lim = fminf(rad, P.coef * rad);
+                unsigned m = __ballot_sync(0xffffffffu, i < nnew && d <= lim);
+                while (m) {
+                  int src = __ffs(m) - 1;
+                  float dj = __shfl_sync(0xffffffffu, d, src);
+                  uint32_t idj = nid[b + src];
+                  if (dj <= rad && dj <= P.coef * rad)
+                    result_insert(res, n, rad, P.size, cfg.mode, pack_key(dj, idj), lane);
+                  m &= (src == 31) ? 0u : ~((2u << src) - 1u);
+                  lim = fminf(rad, P.coef * rad);
+                  m &= __ballot_sync(0xffffffffu, i < nnew && d <= lim);
+                }
+              }
+              if (lane == 0) {
+                s.radius = rad;
+                s.nres = n;
               }
             }
-            if (lane == 0) {
-              s.radius = rad;
-              s.nres = n;
-            }
+            __syncthreads();
           }
-          __syncthreads();
           radius = s.radius;
         }
         dc += nnew;
         nvisited += nnew;
-        // chunk survivors within the exploration radius become candidates
         const float expR = P.coef * radius;
-        if (tid == 0) s.evict_min = ~0ull;
-        {
-          const bool keep = (uint32_t)tid < nnew && nd[tid] <= expR;
-          const unsigned kb = __ballot_sync(0xffffffffu, keep);
-          uint32_t at = 0;
-          if (lane == 0 && kb) at = atomicAdd(&s.keep, (uint32_t)__popc(kb));
-          at = __shfl_sync(0xffffffffu, at, 0);
-          if (keep) bkeys[at + __popc(kb & ((1u << lane) - 1u))] = pack_key(nd[tid], nid[tid]);
-        }
-        __syncthreads();
-        const uint32_t m = s.keep;
         unsigned long long* cl = cur ? cand1 : cand0;
+        if (m == 0) {
+          // no candidate came: the list stays, and its head is the guess unless an earlier
+          // round of this node brought a nearer one (which is popped at the top then)
+          if (last && head < tail && cl[head] == guess) {
+            have = !(key_dist(guess) > expR);
+            finished = !have;
+            if (have) {
+              head++;
+              e0 = g0;
+              nsz = min(g1 - g0, P.edge_size);
+              eid = gid;
+            }
+          }
+          continue;
+        }
+        // chunk survivors become candidates
+        if (tid == 0) s.evict_min = ~0ull;
         unsigned long long* cn = cur ? cand0 : cand1;
         const unsigned long long* old = cl + head;
-        rank_sort_split<T>(bkeys, bsorted, m);
-        // entries above the exploration radius can never be expanded again
-        if (tid == T - 1) s.live_old = upper_bound_dist(old, tail - head, expR);
+        if (!replay) rank_sort_split<T>(bkeys, bsorted, m);
+        // entries above a smaller exploration radius can never be expanded again
+        if (replay && tid == T - 1) s.live_old = upper_bound_dist(old, tail - head, expR);
         __syncthreads();
-        const uint32_t nold = s.live_old;
+        uint32_t nold = tail - head;
+        if (replay) {
+          nold = s.live_old;
+          m = upper_bound_dist(bsorted, m, expR);
+        }
         // survivors not below the overflow tier's minimum join the tier directly
         const uint32_t mk = ovf_n && m && bsorted[m - 1] >= ovf_min ? lower_bound_keys(bsorted, m, ovf_min) : m;
-        // the next node: its offsets load while the list is merged
-        const bool last = c0 + CH >= n_edges;
-        uint32_t o0 = 0, o1 = 0;
+        // the next node: unless it is the guess, its offsets load while the list is merged
+        uint32_t o0 = g0, o1 = g1;
+        bool known = true;
         if (last) {
           unsigned long long t = nold ? old[0] : ~0ull;
           if (mk && bsorted[0] < t) t = bsorted[0];
@@ -666,12 +830,11 @@ graph_search_exact_kernel(DevGraph g, const uint4* __restrict__ queries, uint32_
             have = !(key_dist(t) > expR);
             finished = !have;
           }
-          if (have) {
+          if (have && t != guess) {
+            known = false;
             o0 = __ldg(g.offsets + key_id(t));
             o1 = __ldg(g.offsets + key_id(t) + 1);
           }
-        } else if (tid < (int)CH && c0 + CH + tid < n_edges) {
-          eid = g.edges[e0 + c0 + CH + tid];
         }
         const uint32_t obase = ovf_n;
         const uint32_t nevict = (nold + mk > cfg.ccap) ? nold + mk - cfg.ccap : 0u;
@@ -702,7 +865,8 @@ graph_search_exact_kernel(DevGraph g, const uint4* __restrict__ queries, uint32_
         if (have) {
           e0 = o0;
           nsz = min(o1 - o0, P.edge_size);
-          if ((uint32_t)tid < min(nsz, CH)) eid = g.edges[e0 + tid];
+          if (known) eid = gid;
+          else if ((uint32_t)tid < min(nsz, CH)) eid = __ldg(g.edges + e0 + tid);
         }
         __syncthreads();
         const uint32_t added = (m - mk) + nevict;

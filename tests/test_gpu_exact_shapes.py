@@ -92,3 +92,29 @@ def test_large_index_without_a_shared_bitmap(tmp_path):
         b = ix.batch_search(q[:20], k=10, epsilon=0.3, with_stats=True)
     assert np.array_equal(a[0][:20], b[0]) and np.array_equal(a[1][:20], b[1])
     assert np.array_equal(a[3]["distance_computations"][:20], b[3]["distance_computations"])
+
+
+# The result set's merge: sets that fill slowly (k beyond a node's neighbours), ties at the
+# last result everywhere (coordinates 0..2), a search radius that is reached at once.
+@pytest.mark.parametrize("mode", ["read_only", "updatable"])
+@pytest.mark.parametrize("k", [1, 2, 15, 130, 400])
+def test_result_sets_with_ties(tmp_path, k, mode):
+    path = str(tmp_path / "ix")
+    _index(path, 3000, 6, 24, 77)
+    x = np.random.default_rng(1).integers(0, 3, (3000, 6)).astype(np.float32)
+    rec = np.empty((3000, 25), np.uint8)
+    rec[:, 0] = ord("+")
+    rec[:, 1:] = x.view(np.uint8).reshape(3000, -1)
+    with open(os.path.join(path, "obj"), "wb") as f:      # other coordinates over the same graph
+        f.write(np.uint64(3001).tobytes() + b"-" + rec.tobytes())
+    q = np.random.default_rng(2).integers(0, 3, (160, 6)).astype(np.float32)
+    for eps in (0.0, 0.5):
+        _same(path, q, (9, 160), k, eps, mode)
+    from ngt_gb300 import Index
+    o = oracle.Oracle(oracle.IndexFiles(path))
+    oi, od, on, dc = o.search(q, k=k, epsilon=0.2, radius=1.5, mode=mode, threads=8)
+    with Index(path, read_only=mode == "read_only") as ix:
+        ids, ds, n = ix.batch_search(q, k=k, epsilon=0.2, radius=1.5)
+    assert np.array_equal(n, on)
+    for j in range(len(q)):
+        assert np.array_equal(ids[j, :n[j]], oi[j, :n[j]]) and np.array_equal(ds[j, :n[j]], od[j, :n[j]])
