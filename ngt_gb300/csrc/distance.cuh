@@ -119,15 +119,14 @@ struct Acc {
       unpack<OT>(q, a);
       unpack<OT>(x, b);
       if constexpr (OT == ObjType::Float && (M == Metric::L2 || M == Metric::InnerProduct)) {
-        // the differences two at a time (add.rn.f32x2), then the sum in element order
+        // the differences two at a time, then the sum in element order
 #pragma unroll
         for (int i = 0; i < P; i += 2) {
           const float2 d = sub2(make_float2(a[i], a[i + 1]), make_float2(b[i], b[i + 1]));
           f0 = __fmaf_rn(d.x, d.x, f0);
           f0 = __fmaf_rn(d.y, d.y, f0);
         }
-        return;
-      }
+      } else
 #pragma unroll
       for (int i = 0; i < P; i++) {
         if constexpr (M == Metric::L2 || M == Metric::InnerProduct) {

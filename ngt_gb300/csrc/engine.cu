@@ -724,16 +724,6 @@ void GraphEngine::search_device_slot(const uint4* d_rows, size_t nq, const Searc
   // the pageable host parameter copies above are complete once they return
 }
 
-// Shared-memory visited hash of the exact-order kernels (QG included): a query moves
-// its visited set to the global bitmap once the hash is half full, which every
-// query of a large index does after a few thousand visits, so large indexes get a
-// small hash (more CTAs per SM) and small ones a large hash (no bitmap at all).
-uint32_t GraphEngine::visited_hash_capacity() const { return host_.nrows >= (1u << 18) ? 2048u : 8192u; }
-// Shared-memory tier of the exact-order kernels' candidate queue: 512 keys on large
-// indexes (the overflow tier behind it keeps the queue exact; a smaller tier means
-// more CTAs per SM: 1M x 128: plain kernel +17 %, QG +18 %, results unchanged).
-uint32_t GraphEngine::candidate_list_capacity() const { return host_.nrows >= (1u << 18) ? 512u : 1024u; }
-
 size_t GraphEngine::exact_launch_config(uint32_t max_size, ExactConfig& cfg, uint32_t threads) const {
   cfg = ExactConfig{};
   cfg.kcap = max_size + 1;
@@ -1436,8 +1426,8 @@ void GraphEngine::qg_search_device(const uint4* d_rows, size_t nq, const QGArgs*
   if (seeds.empty()) seeds.push_back(0);
   ExactConfig cfg{};
   cfg.kcap = max_size + 1;
-  cfg.ccap = std::max<uint32_t>(candidate_list_capacity(), std::min<uint32_t>(1024, next_pow2(cfg.kcap)));
-  cfg.hcap = visited_hash_capacity();
+  cfg.ccap = std::min<uint32_t>(1024, std::max<uint32_t>(256, next_pow2(cfg.kcap)));
+  cfg.hcap = 2048;
   cfg.mode = (uint32_t)GraphMode::Updatable;
   cfg.group = std::min<uint32_t>(32, next_pow2((uint32_t)dev_.row_chunks));
   cfg.bitmap_words = (host_.nrows + 31) / 32;
@@ -1445,11 +1435,8 @@ void GraphEngine::qg_search_device(const uint4* d_rows, size_t nq, const QGArgs*
   if (cfg.kcap > cfg.ccap) throw std::runtime_error("size x result expansion too large for the quantized graph search");
   int max_smem = 0;
   NGT_CUDA(cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, device_));
-  size_t smem = qg_kernel_smem_bytes(dev_.row_chunks, qg_.dim, qg_.m, cfg);
-  while (smem > (size_t)max_smem && cfg.hcap > 2048) {
-    cfg.hcap >>= 1;
-    smem = qg_kernel_smem_bytes(dev_.row_chunks, qg_.dim, qg_.m, cfg);
-  }
+  cfg.table_bytes = (uint32_t)qg_table_bytes(qg_.m, cfg);
+  const size_t smem = qg_kernel_smem_bytes(dev_.row_chunks, qg_.dim, qg_.m, cfg);
   if (smem > (size_t)max_smem) throw std::runtime_error("quantized graph search state does not fit in shared memory");
   QGKernelFn fn = qg_kernel(qg_.m);
   NGT_CUDA(cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -1466,10 +1453,15 @@ void GraphEngine::qg_search_device(const uint4* d_rows, size_t nq, const QGArgs*
   }
   QGParams* d_params = nullptr;
   uint32_t* d_seeds = nullptr;
-  NGT_CUDA(cudaMallocAsync(&d_params, nq * sizeof(QGParams), stream));
+  // the launch's own work counter lies behind its parameters
+  NGT_CUDA(cudaMallocAsync(&d_params, nq * sizeof(QGParams) + 4, stream));
   NGT_CUDA(cudaMallocAsync(&d_seeds, seeds.size() * 4, stream));
   NGT_CUDA(cudaMemcpyAsync(d_params, params.data(), nq * sizeof(QGParams), cudaMemcpyHostToDevice, stream));
   NGT_CUDA(cudaMemcpyAsync(d_seeds, seeds.data(), seeds.size() * 4, cudaMemcpyHostToDevice, stream));
+  if (grid < nq) {
+    cfg.work = reinterpret_cast<uint32_t*>(d_params + nq);
+    NGT_CUDA(cudaMemsetAsync(cfg.work, 0, 4, stream));
+  }
   fn<<<(unsigned)grid, kExactThreads, smem, stream>>>(dev_, dqg_, d_rows, (uint32_t)nq, d_params, d_seeds, d_out,
                                                        d_counts, d_stats, bitmaps, overflow, cfg);
   NGT_CUDA(cudaGetLastError());

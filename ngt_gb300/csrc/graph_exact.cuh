@@ -50,7 +50,7 @@ template <class A, int T> constexpr int exact_rows() { return T == 128 && A::kUs
 struct ExactShared {
   float radius;
   uint32_t nres;
-  uint32_t keep[2];               // neighbours of the round within the exploration radius (rounds in turn)
+  uint32_t keep[3];               // neighbours of the round within the exploration radius (rounds in turn)
   uint32_t live_old;
   uint32_t seed_leaf;
   uint32_t seed_status;
@@ -73,6 +73,7 @@ struct ExactConfig {
   uint32_t group;    // lanes per distance (power of two <= 32)
   uint32_t bitmap_words;  // words per CTA in the spill bitmap
   uint32_t ocap;          // overflow-tier capacity per CTA (keys)
+  uint32_t table_bytes;   // quantized graph: qg_table_bytes
   uint32_t smem_bitmap;   // 1: the visited set is a bitmap of every id in shared memory (hcap words)
   uint32_t* work;         // zeroed counter from which the CTAs take the queries; null: CTA i
                           // takes queries i, i + grid, ...

@@ -36,30 +36,10 @@
 namespace ngtg {
 
 struct QGShared {
-  float radius;
-  uint32_t nres;
-  uint32_t head, tail, cur;
-  uint32_t nvisited;
-  uint32_t spilled;
-  uint32_t done;
-  uint32_t target;
-  uint32_t nnew;
-  uint32_t live_old;
-  uint32_t status;
-  uint32_t dc;
-  uint32_t expansions;
-  uint32_t edges;
-  uint32_t seed_leaf;
-  uint32_t ovf_n;
-  uint32_t ovf_tmp;
-  unsigned long long ovf_min;
-  unsigned long long evict_min;
-  unsigned long long sel_prefix;
-  uint32_t sel_need;
+  ExactShared x;                  // the exact kernel's shared state (merge_results, exact_refill)
+  uint32_t nkept;
   float lut_min, lut_scale, lut_offset;
   float wmin[kExactWarps], wmax[kExactWarps];
-  uint32_t warp_cnt[kExactWarps];
-  uint32_t hist[256];
 };
 
 // Four table lookups per byte_perm triple: nibble i of w (neighbour i) selects
@@ -86,6 +66,14 @@ __device__ __forceinline__ void qg_block_words(const uint8_t* __restrict__ blk, 
     const uint32_t s = (uint32_t)lane + 32u * (uint32_t)j;
     w[j] = s < ma ? *reinterpret_cast<const uint2*>(blk + 8u * s) : make_uint2(0u, 0u);
   }
+}
+
+// The neighbour (0..15) of a block whose distance qg_block_distance_words returns in
+// `lane`, or -1.
+__device__ __forceinline__ int qg_lane_object(uint32_t m, int lane) {
+  if (m > 256) return (lane & 1) ? -1 : ((lane >> 1) & 15);
+  const int g = ((lane >> 3) & 1) | (((lane >> 4) & 1) << 1), par = (lane >> 2) & 1, sub = lane & 3;
+  return sub == 0 ? 4 * g + par : sub == 1 ? 4 * g + 2 + par : -1;
 }
 
 // Quantized distances of the 16 neighbours of one code block, by one warp, from the
@@ -187,19 +175,34 @@ __device__ __forceinline__ float qg_block_distance(const uint8_t* __restrict__ b
   return qg_block_distance_words<SPL>(w, L, m, scale, offset, lane, obj);
 }
 
+// Shared memory of the float table, later reused by the lists and the visited hash.
+inline size_t qg_table_bytes(uint32_t m, const ExactConfig& c) {
+  const size_t lists = (size_t)c.ccap * 16 + (size_t)kExactChunk * 16 + (size_t)c.hcap * 4;
+  const size_t table = (size_t)m * 16 * 4;
+  return ((lists > table ? lists : table) + 15) / 16 * 16;
+}
 inline size_t qg_smem_bytes(uint32_t row_chunks, uint32_t dim, uint32_t m, const ExactConfig& c) {
   size_t b = (size_t)row_chunks * 16;
   b += ((size_t)dim * 4 + 15) / 16 * 16;                 // rotated query
-  b += (size_t)m * 16 * 4;                               // float table
   b += ((size_t)m * 16 + 15) / 16 * 16;                  // uint8 table
-  b += (size_t)c.kcap * 8 + (size_t)c.ccap * 16 + (size_t)kExactChunk * 16;
-  b += (size_t)c.hcap * 4 + (size_t)kExactChunk * 12;
+  b += ((size_t)c.kcap + 1) / 2 * 16;                    // results
+  b += qg_table_bytes(m, c);
+  b += (size_t)kExactChunk * 8;                          // a round's distances and ids
   b += sizeof(QGShared) + 16;
   return b;
 }
 
+// Bound by latency and instruction issue like the exact graph kernel, whose round it
+// shares: the guessed next node's ids and code lines load beside the current node's
+// codes, each lane that holds a distance checks and records its neighbour at once (one
+// barrier per round without survivors, twelve before), result updates are merged
+// (merge_results), the shared list holds 256 keys and the float table lies under the
+// lists, so that six CTAs fit an SM instead of three on indexes below 262,144 objects.
+// A visited set holds only neighbours within the exploration radius (hundreds), so a small
+// hash serves every index.  200k x 128, 128 subspaces, 2,000 queries from host buffers
+// (k = 20, epsilon 0.03, expansion 3): 2.87 -> 1.46 ms.
 template <int SPL>
-__global__ void __launch_bounds__(kExactThreads)
+__global__ void __launch_bounds__(kExactThreads, SPL <= 4 ? 6 : 2)
 qg_search_kernel(DevGraph g, DevQG qg, const uint4* __restrict__ queries, uint32_t nq,
                  const QGParams* __restrict__ params, const uint32_t* __restrict__ seed_list,
                  ObjDist* __restrict__ out, uint32_t* __restrict__ out_count, QueryStats* __restrict__ stats,
@@ -211,18 +214,18 @@ qg_search_kernel(DevGraph g, DevQG qg, const uint4* __restrict__ queries, uint32
   // ---- shared-memory carve-up -------------------------------------------
   uint4* qv = reinterpret_cast<uint4*>(smem);
   float* rq = reinterpret_cast<float*>(qv + rc);
-  float* flut = rq + (D + 3) / 4 * 4;
-  uint8_t* lut = reinterpret_cast<uint8_t*>(flut + (size_t)M * 16);
+  uint8_t* lut = reinterpret_cast<uint8_t*>(rq + (D + 3) / 4 * 4);
   unsigned long long* res = reinterpret_cast<unsigned long long*>(lut + ((size_t)M * 16 + 15) / 16 * 16);
-  unsigned long long* cand0 = res + cfg.kcap;
+  unsigned long long* cand0 = res + (cfg.kcap + 1) / 2 * 2;
   unsigned long long* cand1 = cand0 + cfg.ccap;
   unsigned long long* bkeys = cand1 + cfg.ccap;
   unsigned long long* bsorted = bkeys + kExactChunk;
   uint32_t* table = reinterpret_cast<uint32_t*>(bsorted + kExactChunk);
-  uint32_t* nid = table + cfg.hcap;
+  float* flut = reinterpret_cast<float*>(cand0);     // while the tables are built
+  uint32_t* nid = reinterpret_cast<uint32_t*>(reinterpret_cast<unsigned char*>(cand0) + cfg.table_bytes);
   float* nd = reinterpret_cast<float*>(nid + kExactChunk);
-  float* qd = nd + kExactChunk;
-  QGShared& s = *reinterpret_cast<QGShared*>(qd + kExactChunk);
+  QGShared& qs = *reinterpret_cast<QGShared*>(nd + kExactChunk);
+  ExactShared& s = qs.x;
   uint32_t* bitmap = bitmaps + (size_t)blockIdx.x * cfg.bitmap_words;
   unsigned long long* ovf = overflow + (size_t)blockIdx.x * 2 * cfg.ocap;
   unsigned long long* ovf_tmp = ovf + cfg.ocap;
@@ -233,15 +236,13 @@ qg_search_kernel(DevGraph g, DevQG qg, const uint4* __restrict__ queries, uint32
   const float* qf = reinterpret_cast<const float*>(qv);
   const uint32_t qlen = rc * 4;                      // floats in the padded query row
 
-  for (uint32_t q = blockIdx.x; q < nq; q += gridDim.x) {
+  for (uint32_t q = exact_next_query(0xffffffffu, cfg.work, &s.query); q < nq;
+       q = exact_next_query(q, cfg.work, &s.query)) {
     const QGParams P = params[q];
     for (uint32_t i = tid; i < rc; i += blockDim.x) qv[i] = queries[(size_t)q * rc + i];
-    for (uint32_t i = tid; i < cfg.hcap; i += blockDim.x) table[i] = 0u;
     if (tid == 0) {
-      s.radius = P.radius;
-      s.nres = 0; s.head = 0; s.tail = 0; s.cur = 0; s.nvisited = 0; s.spilled = 0;
-      s.done = 0; s.status = 0; s.dc = 0; s.expansions = 0; s.nnew = 0;
-      s.ovf_n = 0; s.ovf_min = ~0ull; s.edges = 0;
+      s.seed_status = 0;
+      s.keep[0] = s.keep[1] = s.keep[2] = 0;
     }
     __syncthreads();
     if (P.size == 0 || P.k == 0) {
@@ -287,20 +288,21 @@ qg_search_kernel(DevGraph g, DevQG qg, const uint4* __restrict__ queries, uint32
         lmin = fminf(lmin, __shfl_xor_sync(0xffffffffu, lmin, off));
         lmax = fmaxf(lmax, __shfl_xor_sync(0xffffffffu, lmax, off));
       }
-      if (lane == 0) { s.wmin[warp] = lmin; s.wmax[warp] = lmax; }
+      if (lane == 0) { qs.wmin[warp] = lmin; qs.wmax[warp] = lmax; }
       __syncthreads();
       if (tid == 0) {
-        float mn = s.wmin[0], mx = s.wmax[0];
-        for (int w = 1; w < kExactWarps; w++) { mn = fminf(mn, s.wmin[w]); mx = fmaxf(mx, s.wmax[w]); }
-        s.lut_min = mn;
-        s.lut_scale = __double2float_rn(__ddiv_rn((double)__fsub_rn(mx, mn), 255.0));
-        s.lut_offset = __fmul_rn(mn, (float)M);
+        float mn = qs.wmin[0], mx = qs.wmax[0];
+        for (int w = 1; w < kExactWarps; w++) { mn = fminf(mn, qs.wmin[w]); mx = fmaxf(mx, qs.wmax[w]); }
+        qs.lut_min = mn;
+        qs.lut_scale = __double2float_rn(__ddiv_rn((double)__fsub_rn(mx, mn), 255.0));
+        qs.lut_offset = __fmul_rn(mn, (float)M);
       }
       __syncthreads();
-      const float mn = s.lut_min, scale = s.lut_scale;
+      const float mn = qs.lut_min, scale = qs.lut_scale;
       for (uint32_t e = tid; e < M * 16; e += blockDim.x)
         lut[e] = (uint8_t)(int)rintf(__fdiv_rn(__fsub_rn(flut[e], mn), scale));
       __syncthreads();
+      for (uint32_t i = tid; i < cfg.hcap; i += blockDim.x) table[i] = 0u;   // the float table is done with
     }
     uint32_t L[SPL][4];
 #pragma unroll
@@ -309,7 +311,7 @@ qg_search_kernel(DevGraph g, DevQG qg, const uint4* __restrict__ queries, uint32
       const uint4 t = sv < M ? reinterpret_cast<const uint4*>(lut)[sv] : make_uint4(0, 0, 0, 0);
       L[j][0] = t.x; L[j][1] = t.y; L[j][2] = t.z; L[j][3] = t.w;
     }
-    const float lscale = s.lut_scale, loffset = s.lut_offset;
+    const float lscale = qs.lut_scale, loffset = qs.lut_offset;
     // ---- seeds --------------------------------------------------------------
     const uint32_t* seeds = nullptr;
     uint32_t nseeds = 0;
@@ -329,7 +331,7 @@ qg_search_kernel(DevGraph g, DevQG qg, const uint4* __restrict__ queries, uint32
         }
         if (lane == 0) {
           if (node & 0x80000000u) s.seed_leaf = node & 0x7fffffffu;
-          else { s.seed_leaf = 0xffffffffu; s.status |= kStatusTreeError; }
+          else { s.seed_leaf = 0xffffffffu; s.seed_status = kStatusTreeError; }
         }
       }
       __syncthreads();
@@ -344,10 +346,11 @@ qg_search_kernel(DevGraph g, DevQG qg, const uint4* __restrict__ queries, uint32
       nseeds = P.seed_cnt;
     }
     nseeds = min(nseeds, (uint32_t)kExactChunk);
+    uint32_t status = s.seed_status;
     if (nseeds == 0) {
       if (tid == 0) {
         out_count[q] = 0;
-        stats[q] = QueryStats{0, 0, 0, 0, s.status | kStatusEmptySeeds};
+        stats[q] = QueryStats{0, 0, 0, 0, status | kStatusEmptySeeds};
       }
       __syncthreads();
       continue;
@@ -366,7 +369,7 @@ qg_search_kernel(DevGraph g, DevQG qg, const uint4* __restrict__ queries, uint32
     __syncthreads();
     if (tid == 0) {
       uint32_t n = 0;
-      float radius = s.radius;
+      float radius = P.radius;
       for (uint32_t i = 0; i < nseeds; i++) {
         float d = key_dist(bsorted[i]);
         if (n < P.size && d <= radius) res[n++] = bsorted[i];
@@ -375,199 +378,191 @@ qg_search_kernel(DevGraph g, DevQG qg, const uint4* __restrict__ queries, uint32
       if (n >= P.size) radius = key_dist(res[n - 1]);
       s.nres = n;
       s.radius = radius;
-      s.dc = nseeds;
-      s.tail = nseeds;
     }
     for (uint32_t i = tid; i < nseeds; i += blockDim.x) {
       cand0[i] = bsorted[i];
       visit_insert(table, hmask, bitmap, false, key_id(bsorted[i]));
     }
-    if (tid == 0) s.nvisited = nseeds;
     __syncthreads();
 
     // ---- best-first loop -----------------------------------------------------
-    uint32_t guard = 0;
+    // Alike in every thread, as in the exact graph kernel.
+    uint32_t head = 0, tail = nseeds, cur = 0, ovf_n = 0;
+    unsigned long long ovf_min = ~0ull;
+    uint32_t nvisited = nseeds, dc = nseeds, expansions = 0, edges = 0;
+    bool spilled = false, have = false;
+    float radius = s.radius;
+    uint32_t e0 = 0, deg = 0, code0 = 0;          // the node to expand: its ids, its codes
+    uint32_t guard = 0, turn = 0;
+    auto node = [&](uint32_t id, uint32_t& first, uint32_t& count, uint32_t& code) {
+      const bool has = id < qg.nnodes;            // nodes beyond the quantized graph have no edges
+      first = has ? __ldg(qg.offsets + id) : 0u;
+      count = has ? __ldg(qg.offsets + id + 1) - first : 0u;
+      code = has ? __ldg(qg.code_off16 + id) : 0u;
+    };
     while (true) {
-      if (s.head >= s.tail && s.ovf_n > 0) {
-        const float expR0 = __fmul_rn(P.coef, s.radius);
-        const uint32_t r0 = s.ovf_n;
-        if (tid == 0) s.ovf_tmp = 0;
-        __syncthreads();
-        for (uint32_t i = tid; i < r0; i += blockDim.x) {
-          unsigned long long k = ovf[i];
-          if (key_dist(k) <= expR0) ovf_tmp[atomicAdd(&s.ovf_tmp, 1u)] = k;
+      if (!have) {
+        if (head >= tail && ovf_n > 0) {
+          head = 0;
+          tail = exact_refill<kExactThreads>(cur ? cand1 : cand0, cfg.ccap, ovf, ovf_tmp, ovf_n, ovf_min,
+                                             __fmul_rn(P.coef, radius), s);
         }
-        __syncthreads();
-        const uint32_t r = s.ovf_tmp;
-        unsigned long long* cl = s.cur ? cand1 : cand0;
-        if (r <= cfg.ccap) {
-          for (uint32_t i = tid; i < r; i += blockDim.x) cl[i] = ovf_tmp[i];
-          __syncthreads();
-          bitonic_sort(cl, r, cfg.ccap);
-          if (tid == 0) { s.head = 0; s.tail = r; s.ovf_n = 0; s.ovf_min = ~0ull; }
-        } else {
-          unsigned long long prefix = 0, mask = 0;
-          uint32_t need = cfg.ccap;
-          for (int shift = 56; shift >= 0; shift -= 8) {
-            for (uint32_t i = tid; i < 256; i += blockDim.x) s.hist[i] = 0;
-            __syncthreads();
-            for (uint32_t i = tid; i < r; i += blockDim.x) {
-              unsigned long long k = ovf_tmp[i];
-              if ((k & mask) == prefix) atomicAdd(&s.hist[(uint32_t)(k >> shift) & 255u], 1u);
-            }
-            __syncthreads();
-            if (tid == 0) {
-              uint32_t acc = 0, b;
-              for (b = 0; b < 255; b++) {
-                if (acc + s.hist[b] >= need) break;
-                acc += s.hist[b];
-              }
-              s.sel_prefix = prefix | ((unsigned long long)b << shift);
-              s.sel_need = need - acc;
-            }
-            __syncthreads();
-            prefix = s.sel_prefix;
-            need = s.sel_need;
-            mask |= 255ull << shift;
-            __syncthreads();
-          }
-          if (tid == 0) { s.ovf_n = 0; s.nnew = 0; s.ovf_min = ~0ull; }
-          __syncthreads();
-          for (uint32_t i = tid; i < r; i += blockDim.x) {
-            unsigned long long k = ovf_tmp[i];
-            if (k <= prefix) {
-              cl[atomicAdd(&s.nnew, 1u)] = k;
-            } else {
-              ovf[atomicAdd(&s.ovf_n, 1u)] = k;
-              atomicMin(&s.ovf_min, k);
-            }
-          }
-          __syncthreads();
-          bitonic_sort(cl, cfg.ccap, cfg.ccap);
-          if (tid == 0) { s.head = 0; s.tail = cfg.ccap; }
-        }
-        __syncthreads();
+        if (head >= tail) break;
+        const unsigned long long t = (cur ? cand1 : cand0)[head];
+        if (key_dist(t) > __fmul_rn(P.coef, radius)) break;
+        head++;
+        node(key_id(t), e0, deg, code0);
       }
-      if (tid == 0) {
-        unsigned long long* cl = s.cur ? cand1 : cand0;
-        float expR = __fmul_rn(P.coef, s.radius);
-        if (s.head >= s.tail) {
-          s.done = 1;
-        } else {
-          unsigned long long t = cl[s.head++];
-          if (key_dist(t) > expR) s.done = 1;
-          else { s.target = key_id(t); s.expansions++; }
-        }
-      }
-      __syncthreads();
-      if (s.done) break;
-      if (++guard > g.nrows + 8) {
-        if (tid == 0) s.status |= kStatusIterationLimit;
+      have = false;
+      const unsigned long long guess = head < tail ? (cur ? cand1 : cand0)[head] : ~0ull;
+      uint32_t ge0 = 0, gdeg = 0, gcode = 0;
+      if (head < tail) node(key_id(guess), ge0, gdeg, gcode);
+      if (guard++ > g.nrows + 8) {
+        status |= kStatusIterationLimit;
         break;
       }
-      const uint32_t target = s.target;
-      const bool has_node = target < qg.nnodes;       // nodes beyond the quantized graph have no edges
-      const uint32_t e0 = has_node ? qg.offsets[target] : 0u;
-      const uint32_t deg = has_node ? qg.offsets[target + 1] - e0 : 0u;
-      const uint8_t* stream = qg.codes + (has_node ? (size_t)qg.code_off16[target] * 16 : 0);
-      if (tid == 0) { s.edges += deg; s.dc += deg; }
-      for (uint32_t c0 = 0; c0 < deg; c0 += kExactChunk) {
-        const uint32_t clen = min((uint32_t)kExactChunk, deg - c0);
-        // quantized distances of the chunk: one 16-neighbour block per warp at a time
-        const uint32_t nblk = (clen + 15) / 16;
-        for (uint32_t bi = (uint32_t)warp; bi < nblk; bi += kExactWarps) {
-          const uint8_t* blk = stream + (size_t)(c0 / 16 + bi) * 8 * qg.ma;
-          int o;
-          float d = qg_block_distance<SPL>(blk, L, M, qg.ma, lscale, loffset, lane, &o);
-          if (o >= 0 && bi * 16 + (uint32_t)o < clen) qd[bi * 16 + o] = d;
-        }
-        if (!s.spilled && s.nvisited + clen > (cfg.hcap >> 1)) {
+      expansions++;
+      edges += deg;
+      dc += deg;
+      bool finished = false;
+      const uint32_t n_edges = deg;
+      const uint8_t* stream = qg.codes + (size_t)code0 * 16;
+      for (uint32_t c0 = 0; c0 < n_edges; c0 += kExactChunk) {
+        const uint32_t clen = min((uint32_t)kExactChunk, n_edges - c0);
+        const bool last = c0 + kExactChunk >= n_edges;
+        if (!spilled && nvisited + clen > (cfg.hcap >> 1)) {
           for (uint32_t i = tid; i < cfg.hcap; i += blockDim.x) {
             uint32_t id = table[i];
             if (id) atomicOr(&bitmap[id >> 5], 1u << (id & 31u));
           }
           __threadfence_block();
           __syncthreads();
-          if (tid == 0) { s.spilled = 1; s.status |= kStatusVisitedSpill; }
+          spilled = true;
+          status |= kStatusVisitedSpill;
         }
-        __syncthreads();
-        const bool spilled = s.spilled != 0;
-        // within the exploration radius and not visited yet: new, in edge order
-        const float expR0 = __fmul_rn(P.coef, s.radius);
-        bool isnew = false;
-        uint32_t id = 0;
-        float dq = 0.f;
-        if ((uint32_t)tid < clen) {
-          dq = qd[tid];
-          id = qg.ids[e0 + c0 + tid];
-          if (dq <= expR0) isnew = visit_insert(table, hmask, bitmap, spilled, id);
-        }
-        unsigned ballot = __ballot_sync(0xffffffffu, isnew);
-        if (lane == 0) s.warp_cnt[warp] = __popc(ballot);
-        __syncthreads();
-        uint32_t base = 0;
-        for (int w = 0; w < warp; w++) base += s.warp_cnt[w];
-        if (isnew) {
-          const uint32_t pos = base + __popc(ballot & ((1u << lane) - 1u));
-          nid[pos] = id;
-          nd[pos] = dq;
-        }
-        __syncthreads();
-        uint32_t nnew = 0;
-        for (int w = 0; w < kExactWarps; w++) nnew += s.warp_cnt[w];
-        // sequential replay of the result-set updates (warp 0): a neighbour joins
-        // when within both the exploration radius and the radius of that moment
-        if (warp == 0) {
-          float radius = s.radius;
-          uint32_t n = s.nres;
-          for (uint32_t b = 0; b < nnew; b += 32) {
-            uint32_t i = b + lane;
-            float d = i < nnew ? nd[i] : FLT_MAX;
-            float lim = fminf(radius, __fmul_rn(P.coef, radius));
-            unsigned m = __ballot_sync(0xffffffffu, i < nnew && d <= lim);
-            while (m) {
-              int src = __ffs(m) - 1;
-              float dj = __shfl_sync(0xffffffffu, d, src);
-              uint32_t idj = nid[b + src];
-              if (dj <= radius && dj <= __fmul_rn(P.coef, radius))
-                result_insert(res, n, radius, P.size, (uint32_t)GraphMode::Updatable, pack_key(dj, idj), lane);
-              m &= (src == 31) ? 0u : ~((2u << src) - 1u);
-              lim = fminf(radius, __fmul_rn(P.coef, radius));
-              m &= __ballot_sync(0xffffffffu, i < nnew && d <= lim);
+        // quantized distances of the chunk, a 16-neighbour block per warp at a time; within
+        // the exploration radius and not visited yet: new
+        const float expR0 = __fmul_rn(P.coef, radius);
+        const uint32_t nblk = (clen + 15) / 16;
+        const int o = qg_lane_object(M, lane);
+        bool pass = false;
+        for (uint32_t bi = (uint32_t)warp; bi < nblk; bi += kExactWarps) {
+          uint2 w[SPL];
+          qg_block_words<SPL>(stream + (size_t)(c0 / 16 + bi) * 8 * qg.ma, qg.ma, lane, w);
+          const uint32_t pos = bi * 16 + (uint32_t)o;
+          const bool mine = o >= 0 && pos < clen;
+          const uint32_t id = mine ? __ldg(qg.ids + e0 + c0 + pos) : 0u;
+          if (last && bi == (uint32_t)warp) {
+            // the guess's code lines (and ids) are asked for beside this node's
+            const uint32_t bytes = (gdeg + 15) / 16 * 8 * qg.ma;
+            if ((uint32_t)tid * 128u < bytes)
+              asm volatile("prefetch.global.L2 [%0];" ::"l"(qg.codes + (size_t)gcode * 16 + (uint32_t)tid * 128u));
+            if ((uint32_t)tid * 32u < gdeg) asm volatile("prefetch.global.L2 [%0];" ::"l"(qg.ids + ge0 + tid * 32));
+          }
+          int oo;
+          const float d = qg_block_distance_words<SPL>(w, L, M, lscale, loffset, lane, &oo);
+          if (mine) {
+            const bool isnew = d <= expR0 && visit_insert(table, hmask, bitmap, spilled, id);
+            if (isnew) {
+              bkeys[atomicAdd(&s.keep[turn], 1u)] = pack_key(d, id);
+              pass = pass || d <= radius;
+            }
+            if (!(P.coef >= 1.0f)) {               // the replay below goes through them in edge order
+              nd[pos] = isnew ? d : INFINITY;
+              nid[pos] = id;
             }
           }
-          if (lane == 0) {
-            s.radius = radius;
-            s.nres = n;
-            s.nvisited += nnew;
+        }
+        const bool replay = __syncthreads_or(pass ? 1 : 0) != 0;
+        uint32_t m = s.keep[turn];
+        // one barrier a round: the counter cleared is the one last read a round ago, and first
+        // used again after the next barrier
+        if (tid == 0) s.keep[turn == 0 ? 2 : turn - 1] = 0;
+        turn = turn == 2 ? 0 : turn + 1;
+        nvisited += m;
+        // result-set updates: a neighbour joins when within both the exploration radius and
+        // the radius of that moment
+        if (replay) {
+          rank_sort_split<kExactThreads>(bkeys, bsorted, m);
+          __syncthreads();
+          if (!(P.coef >= 1.0f) || !merge_results<kExactThreads>(res, P.size, (uint32_t)GraphMode::Updatable, radius,
+                                                                 bsorted, m, nullptr, nullptr, 0, s)) {
+            if (warp == 0) {
+              float rad = radius;
+              uint32_t n = s.nres;
+              for (uint32_t b = 0; b < clen; b += 32) {
+                uint32_t i = b + lane;
+                float d = i < clen ? nd[i] : INFINITY;
+                float lim = fminf(rad, __fmul_rn(P.coef, rad));
+                unsigned m = __ballot_sync(0xffffffffu, i < clen && d <= lim);
+                while (m) {
+                  int src = __ffs(m) - 1;
+                  float dj = __shfl_sync(0xffffffffu, d, src);
+                  uint32_t idj = nid[b + src];
+                  if (dj <= rad && dj <= __fmul_rn(P.coef, rad))
+                    result_insert(res, n, rad, P.size, (uint32_t)GraphMode::Updatable, pack_key(dj, idj), lane);
+                  m &= (src == 31) ? 0u : ~((2u << src) - 1u);
+                  lim = fminf(rad, __fmul_rn(P.coef, rad));
+                  m &= __ballot_sync(0xffffffffu, i < clen && d <= lim);
+                }
+              }
+              if (lane == 0) {
+                s.radius = rad;
+                s.nres = n;
+              }
+            }
+            __syncthreads();
+          }
+          radius = s.radius;
+        }
+        const float expR = __fmul_rn(P.coef, radius);
+        unsigned long long* cl = cur ? cand1 : cand0;
+        if (m == 0) {
+          // no candidate came: the list stays, and its head is the guess unless an earlier
+          // round of this node brought a nearer one (which is popped at the top then)
+          if (last && head < tail && cl[head] == guess) {
+            have = !(key_dist(guess) > expR);
+            finished = !have;
+            if (have) {
+              head++;
+              e0 = ge0;
+              deg = gdeg;
+              code0 = gcode;
+            }
+          }
+          continue;
+        }
+        if (tid == 0) s.evict_min = ~0ull;
+        unsigned long long* cn = cur ? cand0 : cand1;
+        const unsigned long long* old = cl + head;
+        if (!replay) rank_sort_split<kExactThreads>(bkeys, bsorted, m);
+        if (replay && tid == kExactThreads - 1) s.live_old = upper_bound_dist(old, tail - head, expR);
+        __syncthreads();
+        uint32_t nold = tail - head;
+        if (replay) {
+          nold = s.live_old;
+          m = upper_bound_dist(bsorted, m, expR);
+        }
+        const uint32_t mk = ovf_n && m && bsorted[m - 1] >= ovf_min ? lower_bound_keys(bsorted, m, ovf_min) : m;
+        if (last) {
+          unsigned long long t = nold ? old[0] : ~0ull;
+          if (mk && bsorted[0] < t) t = bsorted[0];
+          if (nold + mk > 0) {
+            have = !(key_dist(t) > expR);
+            finished = !have;
+          }
+          if (have) {
+            if (t == guess) {
+              e0 = ge0;
+              deg = gdeg;
+              code0 = gcode;
+            } else {
+              node(key_id(t), e0, deg, code0);     // under way while the list is merged
+            }
           }
         }
-        __syncthreads();
-        const float expR = __fmul_rn(P.coef, s.radius);
-        {
-          bool keep = (uint32_t)tid < nnew && nd[tid] <= expR;
-          unsigned kb = __ballot_sync(0xffffffffu, keep);
-          if (lane == 0) s.warp_cnt[warp] = __popc(kb);
-          __syncthreads();
-          uint32_t kbase = 0;
-          for (int w = 0; w < warp; w++) kbase += s.warp_cnt[w];
-          if (keep) bkeys[kbase + __popc(kb & ((1u << lane) - 1u))] = pack_key(nd[tid], nid[tid]);
-          __syncthreads();
-        }
-        uint32_t m = 0;
-        for (int w = 0; w < kExactWarps; w++) m += s.warp_cnt[w];
-        rank_sort(bkeys, bsorted, m);
-        unsigned long long* cl = s.cur ? cand1 : cand0;
-        unsigned long long* cn = s.cur ? cand0 : cand1;
-        if (tid == 0) s.live_old = upper_bound_dist(cl + s.head, s.tail - s.head, expR);
-        __syncthreads();
-        const uint32_t nold = s.live_old;
-        const unsigned long long* old = cl + s.head;
-        const uint32_t mk = s.ovf_n ? lower_bound_keys(bsorted, m, s.ovf_min) : m;
-        const uint32_t obase = s.ovf_n;
+        const uint32_t obase = ovf_n;
         const uint32_t nevict = (nold + mk > cfg.ccap) ? nold + mk - cfg.ccap : 0u;
-        if (tid == 0) s.evict_min = ~0ull;
-        __syncthreads();
         for (uint32_t i = tid; i < m - mk; i += blockDim.x) {
           uint32_t o = obase + i;
           if (o < cfg.ocap) ovf[o] = bsorted[mk + i];
@@ -593,23 +588,19 @@ qg_search_kernel(DevGraph g, DevQG qg, const uint4* __restrict__ queries, uint32
           }
         }
         __syncthreads();
-        if (tid == 0) {
-          uint32_t added = (m - mk) + nevict;
-          if (added) {
-            unsigned long long mn = s.evict_min;
-            if (mk < m && bsorted[mk] < mn) mn = bsorted[mk];
-            if (mn < s.ovf_min) s.ovf_min = mn;
-            uint32_t n2 = s.ovf_n + added;
-            if (n2 > cfg.ocap) { n2 = cfg.ocap; s.status |= kStatusCandidateOverflow; }
-            s.ovf_n = n2;
-          }
-          s.head = 0;
-          s.tail = nold + mk - nevict;
-          s.cur ^= 1u;
+        const uint32_t added = (m - mk) + nevict;
+        if (added) {
+          unsigned long long mn = s.evict_min;
+          if (mk < m && bsorted[mk] < mn) mn = bsorted[mk];
+          if (mn < ovf_min) ovf_min = mn;
+          ovf_n += added;
+          if (ovf_n > cfg.ocap) { ovf_n = cfg.ocap; status |= kStatusCandidateOverflow; }
         }
-        __syncthreads();
+        head = have ? 1u : 0u;
+        tail = nold + mk - nevict;
+        cur ^= 1u;
       }
-      __syncthreads();
+      if (finished) break;
     }
     // ---- results ---------------------------------------------------------------
     __syncthreads();
@@ -617,12 +608,19 @@ qg_search_kernel(DevGraph g, DevQG qg, const uint4* __restrict__ queries, uint32
     if (P.rerank) {
       // exact L2 of every result, sorted by (distance, id); kept while distance <
       // radius (upper_bound at (0, radius)); at most k
-      for (uint32_t b = (uint32_t)(warp * (32 / G)); b < n; b += ngroups) {
-        uint32_t i = b + (uint32_t)(lane / G);
-        bool valid = i < n;
-        uint32_t id = valid ? key_id(res[i]) : 0u;
-        float d = group_distance<ObjType::Float, Metric::L2>(qv, g.objects + (size_t)id * rc, (int)rc, gl, G);
-        if (valid && gl == 0) cand0[i] = pack_key(d, id);
+      const int pw = packed_width(G);
+      for (uint32_t b = (uint32_t)(warp * (32 / pw)); b < n; b += 2 * (kExactThreads / pw)) {
+        uint32_t id[2], at[2];
+        Acc<ObjType::Float, Metric::L2> sum[2];
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+          at[u] = b + u * (kExactThreads / pw) + (uint32_t)(lane / pw);
+          id[u] = at[u] < n ? key_id(res[at[u]]) : 0u;
+        }
+        packed_sums<ObjType::Float, Metric::L2, 2>(qv, g.objects, id, (int)rc, lane & (pw - 1), G, sum);
+#pragma unroll
+        for (int u = 0; u < 2; u++)
+          if (at[u] < n && (lane & (pw - 1)) == 0) cand0[at[u]] = pack_key(sum[u].finish(), id[u]);
       }
       __syncthreads();
       bitonic_sort(cand0, n, cfg.ccap);
@@ -632,10 +630,10 @@ qg_search_kernel(DevGraph g, DevQG qg, const uint4* __restrict__ queries, uint32
           keep = 0;
           while (keep < n && key_dist(cand0[keep]) < P.radius) keep++;
         }
-        s.nnew = min(keep, P.k);
+        qs.nkept = min(keep, P.k);
       }
       __syncthreads();
-      n = s.nnew;
+      n = qs.nkept;
       for (uint32_t i = tid; i < n; i += blockDim.x) {
         unsigned long long k = cand0[i];
         out[P.out_off + i] = ObjDist{key_id(k), key_dist(k)};
@@ -648,9 +646,9 @@ qg_search_kernel(DevGraph g, DevQG qg, const uint4* __restrict__ queries, uint32
     }
     if (tid == 0) {
       out_count[q] = n;
-      stats[q] = QueryStats{s.dc, s.expansions, s.nvisited, s.edges, s.status};
+      stats[q] = QueryStats{dc, expansions, nvisited, edges, status};
     }
-    if (s.spilled) {
+    if (spilled) {
       for (uint32_t i = tid; i < cfg.bitmap_words; i += blockDim.x) bitmap[i] = 0u;
       __threadfence();
     }
