@@ -1363,6 +1363,8 @@ void GraphEngine::read_qg() {
 }
 
 void GraphEngine::upload_qg() {
+  for (uint32_t i = 0; i < qg_.nnodes; i++)
+    qg_max_degree_ = std::max(qg_max_degree_, qg_.offsets[i + 1] - qg_.offsets[i]);
   NGT_CUDA(cudaSetDevice(device_));
   auto up = [&](const void* src, size_t bytes) {
     void* p = dmalloc_copy<void>(src, bytes);
@@ -1509,8 +1511,7 @@ void GraphEngine::qg_search_device_relaxed(const uint4* d_rows, size_t nq, const
   cfg.list_cap = L;
   cfg.parents = tuning_.parents ? std::min<uint32_t>(tuning_.parents, 32) : 8;
   // neighbour slots: the code blocks of the largest node, and about P typical nodes
-  uint32_t maxdeg = 0;
-  for (uint32_t i = 0; i < qg_.nnodes; i++) maxdeg = std::max(maxdeg, qg_.offsets[i + 1] - qg_.offsets[i]);
+  const uint32_t maxdeg = qg_max_degree_;
   const uint32_t meandeg = qg_.nnodes ? (uint32_t)(qg_.offsets[qg_.nnodes] / qg_.nnodes) : 0u;
   uint32_t NB = next_pow2(std::max<uint32_t>({512u, (maxdeg + 15) / 16 * 16,
                                               cfg.parents * ((meandeg + 15) / 16 * 16), L}));

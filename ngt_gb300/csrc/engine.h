@@ -406,6 +406,7 @@ class GraphEngine {
   // quantized graph
   HostQG qg_;
   bool qg_loaded_ = false;
+  uint32_t qg_max_degree_ = 0;
   DevQG dqg_;
   std::vector<void*> qg_buffers_;
   int device_ = 0;

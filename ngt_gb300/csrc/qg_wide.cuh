@@ -43,7 +43,7 @@ struct QGWideShared {
   uint32_t q, n, cur, np, nblk, cnt, pend, status, dc, expansions, edges, visited, seed_leaf;
   float lut_min, lut_scale, limit;
   float wmin[kQGWideWarps], wmax[kQGWideWarps];
-  uint32_t parents[32], pdeg[32], poff[32], pblk[33];
+  uint32_t parents[32], pdeg[32], poff[32], pcode[32], pblk[33];
 };
 
 // bytes of the work region (new keys, ids, distances), which also holds the float
@@ -93,7 +93,7 @@ qg_wide_kernel(DevGraph g, DevQG qg, const uint4* __restrict__ queries, uint32_t
   uint8_t* lexp = reinterpret_cast<uint8_t*>(lists + 2 * (size_t)L);
   unsigned long long* nkey = reinterpret_cast<unsigned long long*>(lexp + ((size_t)L * 2 + 15) / 16 * 16);
   uint32_t* nid = reinterpret_cast<uint32_t*>(nkey + NB);
-  float* nd = reinterpret_cast<float*>(nid + NB);
+  unsigned long long* fresh = reinterpret_cast<unsigned long long*>(nid);   // NB keys
   float* flut = reinterpret_cast<float*>(nkey);          // only while the table is built
   QGWideShared& s =
       *reinterpret_cast<QGWideShared*>(reinterpret_cast<unsigned char*>(nkey) + qg_wide_work_bytes(NB, M));
@@ -259,46 +259,59 @@ qg_wide_kernel(DevGraph g, DevQG qg, const uint4* __restrict__ queries, uint32_t
         uint8_t* flags = lexp + (size_t)s.cur * L;
         const float rk = n >= P.size ? fminf(key_dist(list[P.size - 1]), user_radius) : user_radius;
         const float limit = __fmul_rn(P.coef, rk);
-        uint32_t np = 0, nblk = 0;
-        bool full = false;
-        for (uint32_t b = 0; b < n && !full; b += 32) {
+        // the first P unexpanded entries within the limit, a lane each
+        uint32_t found = 0, mine = 0, at = 0;
+        for (uint32_t b = 0; b < n && found < cfg.parents; b += 32) {
           const uint32_t i = b + (uint32_t)lane;
           const unsigned long long k = i < n ? list[i] : ~0ull;
           const bool beyond = i < n && key_dist(k) > limit;
           unsigned bal = __ballot_sync(0xffffffffu, i < n && !beyond && flags[i] == 0);
-          while (bal) {
+          for (; bal && found < cfg.parents; bal &= bal - 1, found++) {
             const int src = __ffs(bal) - 1;
-            bal &= bal - 1;
-            const uint32_t p = key_id(__shfl_sync(0xffffffffu, k, src));
-            const bool has = p < qg.nnodes;
-            const uint32_t e0 = has ? qg.offsets[p] : 0u;
-            uint32_t dg = has ? qg.offsets[p + 1] - e0 : 0u;
-            if (np == 0) dg = min(dg, NB);                 // a node beyond the slots keeps its first NB
-            const uint32_t nb = (dg + 15) / 16;
-            if (np > 0 && (nblk + nb) * 16 > NB) { full = true; break; }
-            if (lane == 0) {
-              s.parents[np] = p;
-              s.pdeg[np] = dg;
-              s.poff[np] = e0;
-              s.pblk[np] = nblk;
-              flags[b + (uint32_t)src] = 1;
+            const uint32_t id = __shfl_sync(0xffffffffu, (uint32_t)k, src);
+            if ((uint32_t)lane == found) {
+              mine = id;
+              at = b + (uint32_t)src;
             }
-            np++;
-            nblk += nb;
-            if (np == cfg.parents) { full = true; break; }
           }
           if (__any_sync(0xffffffffu, beyond)) break;     // the list is sorted: nothing later qualifies
         }
+        // their nodes' offsets, all at once; kept up to the first whose code blocks do not fit
+        // the neighbour slots (the first always: a node beyond the slots keeps its first NB)
+        const bool has = (uint32_t)lane < found && mine < qg.nnodes;
+        const uint32_t e0 = has ? __ldg(qg.offsets + mine) : 0u;
+        uint32_t dg = has ? __ldg(qg.offsets + mine + 1) - e0 : 0u;
+        const uint32_t code = has ? __ldg(qg.code_off16 + mine) : 0u;
+        if (lane == 0) dg = min(dg, NB);
+        uint32_t blocks = (dg + 15) / 16, edges = dg;
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+          const uint32_t y = __shfl_up_sync(0xffffffffu, blocks, off), z = __shfl_up_sync(0xffffffffu, edges, off);
+          if (lane >= off) {
+            blocks += y;
+            edges += z;
+          }
+        }
+        const unsigned over = __ballot_sync(0xffffffffu, lane > 0 && blocks * 16 > NB);
+        const uint32_t np = min(found, over ? (uint32_t)__ffs(over) - 1u : 32u);
+        if ((uint32_t)lane < np) {
+          s.parents[lane] = mine;
+          s.pdeg[lane] = dg;
+          s.poff[lane] = e0;
+          s.pcode[lane] = code;
+          s.pblk[lane + 1] = blocks;
+          flags[at] = 1;
+        }
+        const uint32_t nblk = np ? __shfl_sync(0xffffffffu, blocks, np - 1) : 0u;
+        const uint32_t e = np ? __shfl_sync(0xffffffffu, edges, np - 1) : 0u;
         if (lane == 0) {
           s.np = np;
           s.nblk = nblk;
-          s.pblk[np] = nblk;
+          s.pblk[0] = 0;
           s.limit = limit;
           s.expansions += np;
           s.cnt = 0;
           s.pend = 0;
-          uint32_t e = 0;
-          for (uint32_t j = 0; j < np; j++) e += s.pdeg[j];
           s.edges += e;
           s.dc += e;
         }
@@ -327,8 +340,7 @@ qg_wide_kernel(DevGraph g, DevQG qg, const uint4* __restrict__ queries, uint32_t
             pj[u] = j;
             lbk[u] = on[u] ? bi - s.pblk[j] : 0u;
             if (on[u]) {
-              const uint32_t p = s.parents[j];
-              qg_block_words<SPL>(qg.codes + (size_t)qg.code_off16[p] * 16 + (size_t)lbk[u] * 8 * qg.ma, qg.ma,
+              qg_block_words<SPL>(qg.codes + (size_t)s.pcode[j] * 16 + (size_t)lbk[u] * 8 * qg.ma, qg.ma,
                                   lane, w[u]);
               const uint32_t e = lbk[u] * 16u + (uint32_t)lane;
               idv[u] = (lane < 16 && e < s.pdeg[j]) ? qg.ids[s.poff[j] + e] : 0u;
@@ -357,7 +369,7 @@ qg_wide_kernel(DevGraph g, DevQG qg, const uint4* __restrict__ queries, uint32_t
       }
       __syncthreads();
       // visited bits of the pending neighbours, eight atomics in flight per thread; the
-      // fresh ones (ids and distances) are compacted into nid / nd
+      // fresh ones' keys are compacted
       {
         const uint32_t npend = s.pend;
         const unsigned long long* pend = nkey;
@@ -374,15 +386,14 @@ qg_wide_kernel(DevGraph g, DevQG qg, const uint4* __restrict__ queries, uint32_t
           }
 #pragma unroll
           for (int r = 0; r < 8; r++) {
-            const bool fresh = (old[r] & bit[r]) == 0u;
-            const unsigned bal = __ballot_sync(0xffffffffu, fresh);
+            const bool is_new = (old[r] & bit[r]) == 0u;
+            const unsigned bal = __ballot_sync(0xffffffffu, is_new);
             uint32_t base = 0;
             if (lane == 0 && bal) base = atomicAdd(&s.cnt, (uint32_t)__popc(bal));
             base = __shfl_sync(0xffffffffu, base, 0);
-            if (fresh) {
+            if (is_new) {
               const uint32_t pos = base + (uint32_t)__popc(bal & ((1u << lane) - 1u));
-              nid[pos] = (uint32_t)kv[r];
-              nd[pos] = __uint_as_float((uint32_t)(kv[r] >> 32));
+              fresh[pos] = pack_key(__uint_as_float((uint32_t)(kv[r] >> 32)), (uint32_t)kv[r]);
             }
           }
         }
@@ -391,9 +402,15 @@ qg_wide_kernel(DevGraph g, DevQG qg, const uint4* __restrict__ queries, uint32_t
       // merge the new keys into the list (keeps the L best)
       const uint32_t m = s.cnt;
       if (m > 0) {
-        for (uint32_t i = tid; i < m; i += blockDim.x) nkey[i] = pack_key(nd[i], nid[i]);
-        __syncthreads();
-        cta_bitonic_sort(nkey, m, NB);
+        // sorted by rank (up to 128 keys: no barrier between its steps), else bitonic
+        if (m <= kQGWideThreads) {
+          rank_sort_split<(int)kQGWideThreads>(fresh, nkey, m);
+          __syncthreads();
+        } else {
+          for (uint32_t i = tid; i < m; i += blockDim.x) nkey[i] = fresh[i];
+          __syncthreads();
+          cta_bitonic_sort(nkey, m, NB);
+        }
         const uint32_t n = s.n, cur = s.cur;
         const unsigned long long* ol = lists + (size_t)cur * L;
         const uint8_t* of = lexp + (size_t)cur * L;
@@ -436,15 +453,29 @@ qg_wide_kernel(DevGraph g, DevQG qg, const uint4* __restrict__ queries, uint32_t
     __syncthreads();
     uint32_t n = s.cnt;
     if (P.rerank) {
-      for (uint32_t b = (uint32_t)(warp * (32 / G)); b < n; b += (uint32_t)ngroups) {
-        const uint32_t i = b + (uint32_t)(lane / G);
-        const bool valid = i < n;
-        const uint32_t id = valid ? key_id(list[i]) : 0u;
-        const float d = group_distance<ObjType::Float, Metric::L2>(qv, g.objects + (size_t)id * rc, (int)rc, gl, G);
-        if (valid && gl == 0) nkey[i] = pack_key(d, id);
+      const int pw = packed_width(G);
+      const uint32_t step = kQGWideThreads / (uint32_t)pw;
+      const bool few = n <= kQGWideThreads;
+      for (uint32_t b = (uint32_t)(warp * (32 / pw)); b < n; b += 2 * step) {
+        uint32_t id[2], at[2];
+        Acc<ObjType::Float, Metric::L2> sum[2];
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+          at[u] = b + (uint32_t)u * step + (uint32_t)(lane / pw);
+          id[u] = at[u] < n ? key_id(list[at[u]]) : 0u;
+        }
+        packed_sums<ObjType::Float, Metric::L2, 2>(qv, g.objects, id, (int)rc, lane & (pw - 1), G, sum);
+#pragma unroll
+        for (int u = 0; u < 2; u++)
+          if (at[u] < n && (lane & (pw - 1)) == 0) (few ? fresh : nkey)[at[u]] = pack_key(sum[u].finish(), id[u]);
       }
       __syncthreads();
-      cta_bitonic_sort(nkey, n, NB);
+      if (few) {
+        rank_sort_split<(int)kQGWideThreads>(fresh, nkey, n);
+        __syncthreads();
+      } else {
+        cta_bitonic_sort(nkey, n, NB);
+      }
       if (tid == 0) {
         uint32_t keep = n;
         if (P.radius < FLT_MAX) {
