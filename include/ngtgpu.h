@@ -19,9 +19,8 @@ extern "C" {
 #define NGTGPU_KERNEL_BATCHED 1u   /* warp per query, persistent, bf16 search rows for float objects,
                                       exact re-rank of the best candidates (checked by recall) */
 #define NGTGPU_KERNEL_BATCHED_FP32 2u  /* the batched kernel on the full-precision rows */
-#define NGTGPU_KERNEL_WIDE 3u      /* the same search with one query per 256-thread CTA: rows of an
-                                      iteration copied to shared memory all at once (low latency per
-                                      query; float L2 and uint8 L2 indexes) */
+#define NGTGPU_KERNEL_WIDE 3u      /* the same search with one query per CTA of 64 to 512 threads, all
+                                      rows of an iteration in flight at once (low latency per query) */
 
 /* Per-query statistics: distance computations, expanded nodes, visited ids,
  * adjacency entries read, and status bits (1: candidate overflow tier full,
@@ -104,8 +103,8 @@ bool ngtgpu_set_batched_rows_in_flight(NGTIndex, uint32_t rows, NGTError);
  * neighbour slots of one iteration (each parent reads at most
  * neighbour_capacity / parents edges) and sets the shared memory per query.
  * parents: at most 32 (the warp-per-query kernel uses at most 16 of them).
- * NGTGPU_KERNEL_WIDE reads rows_in_flight as the rows each lane group scores at
- * once from shared memory (1, 2 or 4; default 4). */
+ * NGTGPU_KERNEL_WIDE reads rows_in_flight as the rows each lane group keeps in
+ * flight (1, 2 or 4; default 8 for 8-bit rows, else 4). */
 typedef struct {
   uint32_t list_capacity;
   uint32_t parents;
@@ -113,10 +112,11 @@ typedef struct {
   uint32_t rows_in_flight;
   uint32_t ctas_per_sm;
   uint32_t neighbour_capacity;
-  uint32_t cta_threads;        /* NGTGPU_KERNEL_WIDE: 64, 128 or 256 threads per query (64: float L2 only) */
-  uint32_t stage_kilobytes;    /* NGTGPU_KERNEL_WIDE: shared memory for staged rows (default 64) */
+  uint32_t cta_threads;        /* NGTGPU_KERNEL_WIDE: 64, 128 or 256 threads per query (64: float L2 only);
+                                  0: by the number of queries, 512 while each has an SM to itself */
+  uint32_t stage_kilobytes;    /* NGTGPU_KERNEL_WIDE: no effect (rows are loaded into registers) */
   uint32_t l2_policy;          /* NGTGPU_KERNEL_WIDE: 1 plain caching, 2 visited bitmaps kept in L2,
-                                  3 (default) as 2 and staged rows streamed through L2 (evict-first) */
+                                  3 (default) as 2 and search rows streamed through L2 (evict-first) */
   uint32_t search_rows;        /* NGTGPU_KERNEL_WIDE, float L2 objects: 0 automatic (8-bit codes when they
                                   are lossless, else bf16), 1 bf16, 2 8-bit codes */
 } NGTGPUBatchedTuning;
@@ -126,7 +126,7 @@ bool ngtgpu_set_batched_tuning_ex(NGTIndex, const NGTGPUBatchedTuning *tuning, N
  * (or, epsilon < 0, the smallest epsilon of a sweep from 0 to 0.3 reaching the floor,
  * chosen per configuration and returned in *best_epsilon, which may be NULL):
  * a fixed list of configurations (the warp-per-query kernel's row pipelines and
- * register budgets, the CTA-per-query kernel's threads, staged rows and parents per
+ * register budgets, the CTA-per-query kernel's threads and parents per
  * step) is timed on the nq sample queries (CUDA events, median of three launches),
  * and the fastest whose tie-aware recall@k against the exhaustive search of the
  * sample is >= recall_floor -- or, with recall_floor < 0, >= the exact-order kernel's

@@ -68,7 +68,6 @@ std::vector<Candidate> candidates(bool float_l2) {
   warp(3, 4, 5, 256);
   if (float_l2) warp(4, 6, 4, 0);
   for (uint32_t P : {8u, 10u, 12u, 16u}) wide(P, 128, 16);
-  wide(8, 128, 32);
   if (float_l2) {
     wide(16, 256, 32);
     wide(32, 256, 64);

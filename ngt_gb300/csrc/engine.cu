@@ -803,7 +803,23 @@ void GraphEngine::launch_wide(const uint4* d_rows, size_t nq, const QueryParams*
                               cudaStream_t stream, FastScratch& scratch) {
   const SearchRows rows = wide_search_rows();
   const bool bf16 = rows == SearchRows::Bf16, sq8 = rows == SearchRows::Sq8;
-  const uint32_t threads = tuning_.cta_threads ? tuning_.cta_threads : 256u;
+  int sms = 0;
+  NGT_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device_));
+  // Threads per query: the tuning's, or by how many queries share the SMs.  512 while each
+  // has an SM to itself (152 queries, 1M x 128, 10 parents: 1.21 ms, with 256 threads
+  // 1.55 ms; 200k x 100 cosine 0.20 and 0.27 ms), and up to two per SM on large indexes,
+  // whose visited bitmaps then stay in shared memory (304 queries: 1.42 and 1.63 ms; 200k:
+  // 0.33 and 0.28 ms).  128 from six per SM on, where there is such a kernel and few parents
+  // a step (10,000 queries: 15.1 ms, with 256 threads 16.0 ms; 50k x 64: 1.07 and 1.25 ms;
+  // with 32 parents 41.4 and 29.6 ms).
+  uint32_t threads = tuning_.cta_threads;
+  if (!threads) {
+    const size_t own_sm = host_.nrows >= (1u << 18) ? 2 * (size_t)sms : (size_t)sms;
+    const bool few_parents = tuning_.parents <= 16;
+    threads = nq <= own_sm ? 512u : 256u;
+    if (nq >= 6 * (size_t)sms && few_parents && wide_kernel(host_.prop.otype, host_.prop.metric, rows, 128))
+      threads = 128;
+  }
   WideKernelFn fn = wide_kernel(host_.prop.otype, host_.prop.metric, rows, threads);
   if (!fn) throw std::runtime_error("the wide kernel does not support this index type or CTA size");
   if (bf16) ensure_bf16_rows();
@@ -828,10 +844,9 @@ void GraphEngine::launch_wide(const uint4* d_rows, size_t nq, const QueryParams*
     cfg.sq_offset = sq8_offset_;
     cfg.sq_in = 256.f / sq8_scale_;
     cfg.sq_out = sq8_scale_ / 256.f;
+    // whole codes: scale 1, and every squared distance below 2^24 (255^2 x 256)
+    cfg.sq_dot = sq8_lossless_ && host_.prop.dimension <= 256 ? 1u : 0u;
   }
-  // 64 KB of staged rows by default (two 256-thread CTAs share an SM)
-  const uint32_t stage_bytes = (tuning_.stage_kb ? tuning_.stage_kb : 64u) * 1024u;
-  cfg.stage_rows = std::max<uint32_t>(16, std::min<uint32_t>(512, stage_bytes / (cfg.search_chunks * 16)));
   // two chunks per lane; one for 8-bit rows (whose unpacked query chunk is 16 floats)
   cfg.sgroup = std::min<uint32_t>(32, next_pow2(sq8 ? cfg.search_chunks : (cfg.search_chunks + 1) / 2));
   cfg.ngroup = std::min<uint32_t>(32, next_pow2(dev_.row_chunks));
@@ -841,19 +856,36 @@ void GraphEngine::launch_wide(const uint4* d_rows, size_t nq, const QueryParams*
   cfg.spill_cap = kSpillCapacity;
   // default: visited bitmaps kept in L2, staged rows streamed through it
   cfg.l2_policy = tuning_.l2_policy ? tuning_.l2_policy - 1 : 2u;
-  // rows_in_flight: rows per lane group scored at once (1, 2 or 4; default 4)
-  cfg.score_rows = tuning_.rows_in_flight ? std::min<uint32_t>(tuning_.rows_in_flight, 4) : 4u;
-  size_t smem = wide_kernel_smem_bytes(dev_.row_chunks, cfg);
-  int max_smem = 0, per_sm = 0, sms = 0;
+  // rows_in_flight: rows per lane group in flight (default 8 for 8-bit rows, else 4)
+  cfg.score_rows = tuning_.rows_in_flight ? std::min<uint32_t>(tuning_.rows_in_flight, 4) : 8u;
+  int max_smem = 0, per_sm = 0;
   NGT_CUDA(cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, device_));
-  while (smem > (size_t)max_smem && cfg.stage_rows > 16) {
-    cfg.stage_rows /= 2;
-    smem = wide_kernel_smem_bytes(dev_.row_chunks, cfg);
-  }
+  auto ctas_per_sm = [&](size_t smem) {
+    int n = 0;
+    NGT_CUDA(cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    NGT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, (const void*)fn, (int)threads, smem));
+    return n;
+  };
+  size_t smem = wide_kernel_smem_bytes(dev_.row_chunks, cfg);
   if (smem > (size_t)max_smem) throw std::runtime_error("wide search state does not fit in shared memory");
+  per_sm = ctas_per_sm(smem);
+  // the visited bitmap lies in shared memory where that costs no CTA of an SM (200k x 100
+  // cosine, 10,000 queries: 4.26 ms, in global memory 4.54 ms), with 512 threads wherever
+  // it fits (up to about 1.5M objects)
+  cfg.smem_bitmap = 1;
+  const size_t smem_with = wide_kernel_smem_bytes(dev_.row_chunks, cfg);
+  if (smem_with <= (size_t)max_smem) {
+    const int n = ctas_per_sm(smem_with);
+    if (n >= 1 && (n >= per_sm || threads == 512)) {
+      smem = smem_with;
+      per_sm = n;
+    } else {
+      cfg.smem_bitmap = 0;
+    }
+  } else {
+    cfg.smem_bitmap = 0;
+  }
   NGT_CUDA(cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  NGT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)fn, (int)threads, smem));
-  NGT_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device_));
   size_t grid = std::min<size_t>(nq, (size_t)std::max(1, per_sm) * sms);
   ensure_fast_scratch(scratch, grid, stream);
   NGT_CUDA(cudaMemsetAsync(scratch.work, 0, 4, stream));

@@ -6,12 +6,14 @@
 //   * the P parents' edge slots are read, filtered against the query's
 //     visited bitmap and compacted by all threads of the CTA (128 or 256);
 //   * the new neighbours' search rows (bf16 or 8-bit copies of float objects, or
-//     the objects themselves) are copied into a shared-memory stage with 16-byte
-//     cp.async in two halves, the next half in flight while the current one is
-//     scored, several rows per lane group at once;
+//     the objects themselves) are loaded straight into registers, several rows per
+//     lane group in flight, and scored; a row within the limit goes to the new
+//     keys (or the spill tier) at once;
 //   * every survivor's place in the list is its rank among the new keys (counted
-//     when there are at most T of them, else after a CTA bitonic sort) plus its
-//     rank in the list; keys land in a second list buffer.
+//     when there are few, else after a sort) plus its rank in the list; keys land
+//     in a second list buffer.
+// A step takes four CTA barriers: parents chosen, new ids gathered, rows scored,
+// list merged (with a shared-memory row stage, two more per 64 rows).
 // One warp (warp 0) owns the control decisions (parent selection, the refill
 // from the spill tier), exactly as the warp-per-query kernel makes them.
 // Per-query latency is set by a few memory round trips per iteration instead of
@@ -26,62 +28,58 @@
 
 namespace ngtg {
 
-constexpr int kWideMaxThreads = 256;
+constexpr int kWideMaxThreads = 512;
 constexpr int kWideMaxWarps = kWideMaxThreads / 32;
 
 struct WideConfig {
   uint32_t list_cap;       // L: power of two
   uint32_t nbr_cap;        // neighbour slots per iteration (power of two >= L)
   uint32_t parents;        // P (<= 32)
-  uint32_t stage_rows;     // search rows staged in shared memory per round
   uint32_t sgroup;         // lanes per search distance (power of two <= 32)
   uint32_t ngroup;         // lanes per full-precision distance
   uint32_t search_chunks;  // 16-byte chunks per search row
   uint32_t rerank_x16;
   uint32_t bitmap_words;   // per CTA, multiple of 4
+  uint32_t smem_bitmap;    // 1: the visited bitmap lies in shared memory
   uint32_t max_iters;
   uint32_t spill_cap;
   uint32_t l2_policy;      // 0: default caching; 1: visited bitmap kept in L2 (evict_last);
-                           // 2: as 1, and staged rows streamed through L2 (evict_first)
-  uint32_t score_rows;     // rows per lane group scored at once (1, 2 or 4)
+                           // 2: as 1, and search rows streamed through L2 (evict_first)
+  uint32_t score_rows;     // rows per lane group in flight (1, 2, 4, or 8 for 8-bit rows)
   // 8-bit search rows of float objects: code = rint((x - sq_offset) / s), the query
   // mapped the same way in 1/256 steps; distance = sqrt(sum) * sq_out (s / 256)
   uint32_t sq8, dim;
+  uint32_t sq_dot;         // 1: integer dot products give the same distances for whole queries
   float sq_offset, sq_in, sq_out;   // sq_in = 256 / s
 };
 
 struct WideShared {
-  uint32_t q, n, cur, np, total, cnt, kept, scan0, spill_n, stop, done, refill, first_new;
-  uint32_t status, dc, expansions, edges, visited;
-  unsigned long long spill_min, worst;
-  float limit, insert_limit;
+  uint32_t q, n, np, total, cnt, kept, spill_n, done, refill, first_new;
+  uint32_t status, dc, expansions, edges;
+  uint32_t qnorm, fraction;      // 8-bit rows: the query codes' squared sum; 1: not all whole
+  unsigned long long spill_min;
+  float limit;
   uint32_t parents[32], pexcl[32], pbase[32];
-  unsigned long long wmin[kWideMaxWarps];
 };
 
-// 16-byte chunks of the row stage, which also holds the NB candidate keys
-__host__ __device__ inline size_t wide_stage_chunks(uint32_t search_chunks, uint32_t stage_rows, uint32_t nbr_cap) {
-  const size_t rows = (size_t)stage_rows * search_chunks, keys = ((size_t)nbr_cap * 8 + 15) / 16;
-  return rows > keys ? rows : keys;
-}
-
 inline size_t wide_smem_bytes(uint32_t row_chunks, const WideConfig& c) {
-  size_t b = (size_t)row_chunks * 16 + (size_t)c.search_chunks * (c.sq8 ? 64 : 16);
+  size_t b = (size_t)row_chunks * 16 + (size_t)c.search_chunks * (c.sq8 ? 64 + 16 : 16);
   b += (size_t)c.list_cap * 16;                                   // list, double-buffered
-  b += (size_t)c.nbr_cap * 8;                                     // nid, nd
-  b += wide_stage_chunks(c.search_chunks, c.stage_rows, c.nbr_cap) * 16;   // row staging / nkey
-  b += sizeof(WideShared) + 16;
+  b += (size_t)c.nbr_cap * 4;                                     // new ids
+  b += (size_t)kWideMaxThreads * 8;                               // sorted new keys / histogram
+  b += (size_t)c.nbr_cap * 8;                                     // new keys
+  b += (sizeof(WideShared) + 15) / 16 * 16 + 16;
+  if (c.smem_bitmap) b += (size_t)c.bitmap_words * 4;
   return b;
 }
 
-__device__ __forceinline__ void cp_async16(void* smem_dst, const void* gmem_src) {
-  const uint32_t d = (uint32_t)__cvta_generic_to_shared(smem_dst);
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(gmem_src) : "memory");
-}
-__device__ __forceinline__ void cp_async16_hint(void* smem_dst, const void* gmem_src, uint64_t policy) {
-  const uint32_t d = (uint32_t)__cvta_generic_to_shared(smem_dst);
-  asm volatile("cp.async.cg.shared.global.L2::cache_hint [%0], [%1], 16, %2;\n" ::"r"(d), "l"(gmem_src), "l"(policy)
-               : "memory");
+// A 16-byte chunk of a search row, read once: no place in L1, and L2 by `policy`.
+__device__ __forceinline__ uint4 load_row_chunk(const uint4* p, uint64_t policy) {
+  uint4 v;
+  asm("ld.global.nc.L1::no_allocate.L2::cache_hint.v4.u32 {%0, %1, %2, %3}, [%4], %5;"
+      : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+      : "l"(p), "l"(policy));
+  return v;
 }
 // atomicOr on a visited-bitmap word, with an L2 eviction-priority hint when `hint`
 __device__ __forceinline__ uint32_t visit_or(uint32_t* word, uint32_t bit, bool hint, uint64_t policy) {
@@ -99,6 +97,11 @@ __device__ __forceinline__ void store_zero16(uint4* p, bool hint, uint64_t polic
 __device__ __forceinline__ uint64_t l2_policy_evict_last() {
   uint64_t p;
   asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;\n" : "=l"(p));
+  return p;
+}
+__device__ __forceinline__ uint64_t l2_policy_evict_normal() {
+  uint64_t p;
+  asm volatile("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;\n" : "=l"(p));
   return p;
 }
 __device__ __forceinline__ uint64_t l2_policy_evict_first() {
@@ -178,9 +181,33 @@ struct WideDot {
   }
 };
 
-// T: threads per CTA (64, 128 or 256), one query per CTA.
+// The m <= T unique keys in[0..m) sorted to out by their ranks, several threads per key
+// where the CTA has them to spare.
+template <int T>
+__device__ __forceinline__ void rank_sort_keys(const unsigned long long* in, unsigned long long* out, uint32_t m) {
+  uint32_t split = 1;
+  while (split < 8 && m * split * 2 <= (uint32_t)T) split *= 2;
+  const uint32_t i = threadIdx.x / split, sub = threadIdx.x & (split - 1);
+  const unsigned long long k = i < m ? in[i] : 0ull;
+  uint32_t r = 0;
+  if (i < m)
+    for (uint32_t j = sub; j < m; j += split) r += in[j] < k ? 1u : 0u;
+  for (uint32_t off = 1; off < split; off <<= 1) r += __shfl_xor_sync(0xffffffffu, r, off);
+  if (i < m && sub == 0) out[r] = k;
+}
+
+// T: threads per CTA (64, 128, 256 or 512), one query per CTA.
+// Bound by the dependent round trips of a step (parents' offsets, edges, visited bits,
+// rows) and by instruction issue: 0.97M warp instructions per query of 22,400 rows before
+// the integer dot products, 0.55 issued per cycle and scheduler.  Measured on 1M x 128,
+// 8-bit rows, k = 10, epsilon 0.08, 10,000 queries, 128 threads: 15.35 ms with a shared-memory
+// row stage (two barriers per 64 rows); rows loaded into registers 15.1 ms; dot products
+// 14.2 ms.  152 queries: 2.0 ms with 128 threads, 1.1 ms with 512 and the visited bitmap in
+// shared memory.  200k x 100 cosine, 1,500 queries from host buffers: 1.80 -> 1.2 ms (packed
+// lanes, three CTAs per SM instead of two).  Not kept: prefetching a step's rows into L2
+// when they are gathered (5 % slower), 1,024 threads (8 % slower than 512).
 template <ObjType ST, ObjType OT, Metric M, int T>
-__global__ void __launch_bounds__(T, T == 64 ? 10 : T == 128 ? 6 : 2)
+__global__ void __launch_bounds__(T, T == 64 ? 10 : T == 128 ? 6 : T == 256 ? 3 : 1)
 graph_search_wide_kernel(DevGraph g, const uint4* __restrict__ srows, const uint4* __restrict__ queries,
                          uint32_t nq, const QueryParams* __restrict__ params, const uint32_t* __restrict__ seed_list,
                          ObjDist* __restrict__ out, uint32_t* __restrict__ out_count, QueryStats* __restrict__ stats,
@@ -189,177 +216,239 @@ graph_search_wide_kernel(DevGraph g, const uint4* __restrict__ srows, const uint
   extern __shared__ __align__(16) unsigned char smem[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint32_t rc = g.row_chunks, sc = cfg.search_chunks;
-  const uint32_t L = cfg.list_cap, NB = cfg.nbr_cap, SR = cfg.stage_rows;
+  const uint32_t L = cfg.list_cap, NB = cfg.nbr_cap;
   uint4* qn = reinterpret_cast<uint4*>(smem);
   typedef WideDot<ST, OT, M> Dot;
   uint4* qs = qn + rc;                                                           // sc (x 4 for Sq8) chunks
   unsigned long long* lists = reinterpret_cast<unsigned long long*>(qs + (Dot::kSq8 ? 4 * sc : sc));   // 2 x L
-  uint32_t* nid = reinterpret_cast<uint32_t*>(lists + 2 * (size_t)L);
-  float* nd = reinterpret_cast<float*>(nid + NB);
-  uint4* stage = reinterpret_cast<uint4*>(nd + NB);
-  // the candidate keys share the row stage: rows are staged only inside a score
-  // phase, keys are built after it and consumed before the next one
-  unsigned long long* nkey = reinterpret_cast<unsigned long long*>(stage);
-  WideShared& s = *reinterpret_cast<WideShared*>(stage + wide_stage_chunks(sc, SR, NB));
+  unsigned long long* nkey = lists + 2 * (size_t)L;                              // NB new keys
+  unsigned long long* nsorted = nkey + NB;                                       // up to T of them, sorted
+  uint32_t* nid = reinterpret_cast<uint32_t*>(nsorted + kWideMaxThreads);        // NB new ids
+  uint8_t* qcode = reinterpret_cast<uint8_t*>(nid + NB);                         // Sq8: 16 sc query codes
+  WideShared& s = *reinterpret_cast<WideShared*>(qcode + (Dot::kSq8 ? 16 * sc : 0));
+  uint32_t* sbitmap = reinterpret_cast<uint32_t*>(reinterpret_cast<unsigned char*>(&s) + (sizeof(WideShared) + 15) / 16 * 16);
   uint32_t* bitmap = bitmaps + (size_t)blockIdx.x * cfg.bitmap_words;
   unsigned long long* spill = spills + (size_t)blockIdx.x * 2 * cfg.spill_cap;
   unsigned long long* spill_tmp = spill + cfg.spill_cap;
   const int SG = (int)cfg.sgroup, NG = (int)cfg.ngroup;
-  const int sgl = lane & (SG - 1), ngl = lane & (NG - 1);
+  const int sgl = lane & (SG - 1);
   const bool keep_visited = cfg.l2_policy >= 1, stream_rows = cfg.l2_policy >= 2;
   const uint64_t pol_keep = keep_visited ? l2_policy_evict_last() : 0ull;
-  const uint64_t pol_stream = stream_rows ? l2_policy_evict_first() : 0ull;
+  const uint64_t pol_stream = stream_rows ? l2_policy_evict_first() : l2_policy_evict_normal();
 
-  // distances of nid[0..cnt) into nd[], rows staged through shared memory
-  // distances of nid[0..cnt) into nd[]: rows staged through shared memory in two
-  // halves, the next half's copies in flight while the current half is scored
-  const uint32_t SRH = SR / 2;
-  // each thread copies chunk (tid % sc) of every (T / sc)-th row when sc divides T
-  const bool rows_split = ((uint32_t)T % sc) == 0;
-  const uint32_t my_chunk = (uint32_t)tid % sc, my_row = (uint32_t)tid / sc, row_step = (uint32_t)T / sc;
-  auto issue = [&](uint32_t r0, uint32_t nr, uint4* buf) {
-    if (rows_split) {
-      if (stream_rows) {
-        for (uint32_t i = my_row; i < nr; i += row_step)
-          cp_async16_hint(buf + (size_t)i * sc + my_chunk, srows + (size_t)nid[r0 + i] * sc + my_chunk, pol_stream);
-      } else {
-        for (uint32_t i = my_row; i < nr; i += row_step)
-          cp_async16(buf + (size_t)i * sc + my_chunk, srows + (size_t)nid[r0 + i] * sc + my_chunk);
-      }
-    } else {
-      for (uint32_t idx = tid; idx < nr * sc; idx += blockDim.x) {
-        const uint32_t i = idx / sc, c = idx - i * sc;
-        cp_async16(buf + idx, srows + (size_t)nid[r0 + i] * sc + c);
-      }
-    }
-    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  // A scored row within the limit: below the list's worst entry it joins the new keys,
+  // else the spill tier.  Rows past the limit are not kept (their sums need no root).
+  struct Limits {
+    float limit;                 // largest distance kept
+    float far;                   // sums past it are past the limit beyond doubt
+    unsigned long long worst;    // keys from here on go to the spill tier
+    bool all;                    // seeds: every distance is kept
   };
-  auto score = [&](uint32_t cnt) {
-    if (cnt == 0) return;
-    // the query chunks this lane reads (c = sgl + j * SG), negated and unpacked once
-    // the host sets sgroup so that every lane reads at most two chunks (one for 8-bit rows)
+  auto place = [&](float d, uint32_t id, const Limits& w) {
+    if (!(d <= w.limit) && !w.all) return;
+    const unsigned long long key = pack_key(d, id);
+    if (key < w.worst || w.all) {
+      nkey[atomicAdd(&s.kept, 1u)] = key;
+    } else {
+      const uint32_t o = atomicAdd(&s.spill_n, 1u);
+      if (o < cfg.spill_cap) spill[o] = key;
+      atomicMin(&s.spill_min, key);
+    }
+  };
+  // scores nid[0..cnt): every lane group loads the chunks of several rows before it adds
+  // any up.  Lanes, chunks and the order of summation are the same for every number of rows.
+  auto score = [&](uint32_t cnt, const Limits& w) {
+    const uint32_t gpb = (uint32_t)T / SG;
+    const uint32_t gi = (uint32_t)(tid / SG);
     constexpr int kQC = Dot::kSq8 ? 1 : 2;
-    float2 nqc[kQC][Dot::NQ];
-    if constexpr (Dot::kOn) {
+    if (Dot::kOn && sc <= (uint32_t)(kQC * SG)) {
+      // the query chunks this lane reads (c = sgl + j * SG), negated and unpacked once; the
+      // host sets sgroup so that a lane reads at most two chunks (one for 8-bit rows)
+      float2 nqc[kQC][Dot::NQ];
 #pragma unroll
       for (int j = 0; j < kQC; j++) {
         const uint32_t c = (uint32_t)sgl + (uint32_t)(j * SG);
         if (c < sc) Dot::prepare(qs, c, nqc[j]);
         else Dot::zero(nqc[j]);
       }
-    }
-    uint4* buf[2] = {stage, stage + (size_t)SRH * sc};
-    issue(0, min(SRH, cnt), buf[0]);
-    if (cnt > SRH) issue(SRH, min(SRH, cnt - SRH), buf[1]);
-    uint32_t h = 0;
-    for (uint32_t r0 = 0; r0 < cnt; r0 += SRH, h ^= 1u) {
-      const uint32_t nr = min(SRH, cnt - r0);
-      if (r0 + SRH < cnt) {
-        asm volatile("cp.async.wait_group 1;\n" ::: "memory");   // this half landed
-      } else {
-        asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-      }
-      __syncthreads();
-      const uint4* stg = buf[h];
-      const uint32_t gpb = (uint32_t)T / SG;
-      const uint32_t gi = (uint32_t)(tid / SG);
-      if (Dot::kOn && sc <= (uint32_t)(kQC * SG)) {
-        // KR rows per lane group at once: their shared-memory loads first, then 2 x KR
-        // independent accumulations (one per chunk) and interleaved shuffle reductions
-        auto rows_at_once = [&](auto kr_tag) {
-          constexpr int KR = decltype(kr_tag)::value;
-          for (uint32_t b = 0; b < nr; b += gpb * KR) {    // uniform trip count per warp
-            uint4 x[KR][kQC];
+      const bool dots = Dot::kSq8 && s.fraction == 0;
+      const uint4 qc = dots && (uint32_t)sgl < sc ? reinterpret_cast<const uint4*>(qcode)[sgl] : make_uint4(0, 0, 0, 0);
+      auto rows_at_once = [&](auto kr_tag, uint32_t b) {
+        constexpr int KR = decltype(kr_tag)::value;
+        uint4 x[KR][kQC];
+        uint32_t id[KR];
+#pragma unroll
+        for (int u = 0; u < KR; u++) {
+          const uint32_t i = b + (uint32_t)u * gpb + gi;
+          id[u] = i < cnt ? nid[i] : 0u;
+#pragma unroll
+          for (int j = 0; j < kQC; j++) {
+            const uint32_t c = (uint32_t)sgl + (uint32_t)(j * SG);
+            x[u][j] = c < sc ? load_row_chunk(srows + (size_t)id[u] * sc + c, pol_stream) : make_uint4(0, 0, 0, 0);
+          }
+        }
+        float v[KR];
+        if constexpr (Dot::kSq8) {
+          if (dots) {
+            // sum (c - q)^2 = sum c c - 2 sum c q + sum q q over whole codes, exact in 32 bits;
+            // times 2^16 it is the sum of the squared 1/256 steps that the float form adds up
+            // (exact there too, below 2^24 steps of one)
+            int t[KR];
 #pragma unroll
             for (int u = 0; u < KR; u++) {
-              const uint32_t i = b + (uint32_t)u * gpb + gi;
-              const uint4* row = stg + (size_t)(i < nr ? i : 0u) * sc;
+              const uint32_t xw[4] = {x[u][0].x, x[u][0].y, x[u][0].z, x[u][0].w};
+              const uint32_t qw[4] = {qc.x, qc.y, qc.z, qc.w};
+              uint32_t cc = 0, cq = 0;
 #pragma unroll
-              for (int j = 0; j < kQC; j++) {
-                const uint32_t c = (uint32_t)sgl + (uint32_t)(j * SG);
-                x[u][j] = c < sc ? row[c] : make_uint4(0, 0, 0, 0);
+              for (int i = 0; i < 4; i++) {
+                cc = __dp4a(xw[i], xw[i], cc);
+                cq = __dp4a(xw[i], qw[i], cq);
               }
-            }
-            float v[KR];
-#pragma unroll
-            for (int u = 0; u < KR; u++) {
-              float2 acc[kQC];
-#pragma unroll
-              for (int j = 0; j < kQC; j++) {
-                acc[j] = make_float2(0.f, 0.f);
-                if ((uint32_t)sgl + (uint32_t)(j * SG) < sc) acc[j] = Dot::add(acc[j], nqc[j], x[u][j]);
-              }
-              float t = acc[0].x + acc[0].y;
-#pragma unroll
-              for (int j = 1; j < kQC; j++) t += acc[j].x + acc[j].y;
-              v[u] = t;
+              t[u] = (int)(cc - 2u * cq);
             }
 #pragma unroll
             for (int off = 16; off > 0; off >>= 1)
               if (off < SG) {
 #pragma unroll
-                for (int u = 0; u < KR; u++) v[u] += __shfl_xor_sync(0xffffffffu, v[u], off);
+                for (int u = 0; u < KR; u++) t[u] += __shfl_xor_sync(0xffffffffu, t[u], off);
               }
 #pragma unroll
             for (int u = 0; u < KR; u++) {
               const uint32_t i = b + (uint32_t)u * gpb + gi;
-              if (i < nr && sgl == 0) nd[r0 + i] = Dot::kSq8 ? sqrtf(v[u]) * cfg.sq_out : sqrtf(v[u]);
+              const float vu = (float)(t[u] + (int)s.qnorm) * 65536.f;
+              if (i < cnt && sgl == 0 && !(vu > w.far)) place(sqrtf(vu) * cfg.sq_out, id[u], w);
             }
+            return;
           }
-        };
-        const uint32_t kr = min(cfg.score_rows, (nr + gpb - 1) / gpb);   // uniform
-        if (kr >= 4) rows_at_once(std::integral_constant<int, 4>{});
-        else if (kr >= 2) rows_at_once(std::integral_constant<int, 2>{});
-        else rows_at_once(std::integral_constant<int, 1>{});
-      } else {
-        for (uint32_t b = 0; b < nr; b += gpb) {          // uniform trip count per warp
-          const uint32_t i = b + gi;
-          const bool valid = i < nr;
-          const uint4* row = stg + (size_t)(valid ? i : 0u) * sc;
-          float d;
-          if constexpr (Dot::kOn) {
-            float2 acc = make_float2(0.f, 0.f);
-            for (uint32_t c = (uint32_t)sgl; c < sc; c += (uint32_t)SG) {
-              float2 nq[Dot::NQ];
-              Dot::prepare(qs, c, nq);
-              acc = Dot::add(acc, nq, row[c]);
-            }
-            float v = acc.x + acc.y;
+        }
 #pragma unroll
-            for (int off = 16; off > 0; off >>= 1)
-              if (off < SG) v += __shfl_xor_sync(0xffffffffu, v, off);
-            d = Dot::kSq8 ? sqrtf(v) * cfg.sq_out : sqrtf(v);
-          } else {
-            Acc<ST, M> acc;
-            for (uint32_t c = (uint32_t)sgl; c < sc; c += (uint32_t)SG) acc.add(qs[c], row[c], (int)c);
-            acc.reduce(SG);
-            d = acc.finish();
+        for (int u = 0; u < KR; u++) {
+          float2 acc[kQC];
+#pragma unroll
+          for (int j = 0; j < kQC; j++) {
+            acc[j] = make_float2(0.f, 0.f);
+            if ((uint32_t)sgl + (uint32_t)(j * SG) < sc) acc[j] = Dot::add(acc[j], nqc[j], x[u][j]);
           }
-          if (valid && sgl == 0) nd[r0 + i] = d;
+          float t = acc[0].x + acc[0].y;
+#pragma unroll
+          for (int j = 1; j < kQC; j++) t += acc[j].x + acc[j].y;
+          v[u] = t;
+        }
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1)
+          if (off < SG) {
+#pragma unroll
+            for (int u = 0; u < KR; u++) v[u] += __shfl_xor_sync(0xffffffffu, v[u], off);
+          }
+#pragma unroll
+        for (int u = 0; u < KR; u++) {
+          const uint32_t i = b + (uint32_t)u * gpb + gi;
+          if (i < cnt && sgl == 0 && !(v[u] > w.far))
+            place(Dot::kSq8 ? sqrtf(v[u]) * cfg.sq_out : sqrtf(v[u]), id[u], w);
+        }
+      };
+      for (uint32_t b = 0; b < cnt;) {                    // uniform over the CTA
+        const uint32_t kr = min(cfg.score_rows, (cnt - b + gpb - 1) / gpb);
+        if (Dot::kSq8 && kr >= 8) {
+          rows_at_once(std::integral_constant<int, Dot::kSq8 ? 8 : 4>{}, b);
+          b += 8 * gpb;
+        } else if (kr >= 4) {
+          rows_at_once(std::integral_constant<int, 4>{}, b);
+          b += 4 * gpb;
+        } else if (kr >= 2) {
+          rows_at_once(std::integral_constant<int, 2>{}, b);
+          b += 2 * gpb;
+        } else {
+          rows_at_once(std::integral_constant<int, 1>{}, b);
+          b += gpb;
         }
       }
-      __syncthreads();                                   // the half is free again
-      if (r0 + 2 * SRH < cnt) issue(r0 + 2 * SRH, min(SRH, cnt - (r0 + 2 * SRH)), buf[h]);
+    } else if constexpr (Dot::kOn) {
+      // long rows: chunk after chunk, two rows at once
+      for (uint32_t b = 0; b < cnt; b += 2 * gpb) {
+        float2 acc[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+        uint32_t id[2];
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+          const uint32_t i = b + (uint32_t)u * gpb + gi;
+          id[u] = i < cnt ? nid[i] : 0u;
+        }
+#pragma unroll 2
+        for (uint32_t c = (uint32_t)sgl; c < sc; c += (uint32_t)SG) {
+          float2 nq[Dot::NQ];
+          uint4 x[2];
+#pragma unroll
+          for (int u = 0; u < 2; u++) x[u] = load_row_chunk(srows + (size_t)id[u] * sc + c, pol_stream);
+          Dot::prepare(qs, c, nq);
+#pragma unroll
+          for (int u = 0; u < 2; u++) acc[u] = Dot::add(acc[u], nq, x[u]);
+        }
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+          float v = acc[u].x + acc[u].y;
+#pragma unroll
+          for (int off = 16; off > 0; off >>= 1)
+            if (off < SG) v += __shfl_xor_sync(0xffffffffu, v, off);
+          const uint32_t i = b + (uint32_t)u * gpb + gi;
+          if (i < cnt && sgl == 0 && !(v > w.far)) place(Dot::kSq8 ? sqrtf(v) * cfg.sq_out : sqrtf(v), id[u], w);
+        }
+      }
+    } else {
+      // the objects' own comparator, the lanes of a group packed four to a thread
+      const int pw = packed_width(SG);
+      const uint32_t ppb = (uint32_t)T / (uint32_t)pw;
+      for (uint32_t b = 0; b < cnt; b += ppb) {
+        const uint32_t i = b + (uint32_t)(tid / pw);
+        const uint32_t id[1] = {i < cnt ? nid[i] : 0u};
+        Acc<ST, M> sum[1];
+        packed_sums<ST, M, 1>(qs, srows, id, (int)sc, lane & (pw - 1), SG, sum);
+        if (i < cnt && (lane & (pw - 1)) == 0) place(sum[0].finish(), id[0], w);
+      }
     }
   };
 
+  // true when `id` was not visited yet (and marks it)
+  auto visit = [&](uint32_t id) {
+    const uint32_t bit = 1u << (id & 31u);
+    if (cfg.smem_bitmap) return (atomicOr(&sbitmap[id >> 5], bit) & bit) == 0u;
+    return (visit_or(&bitmap[id >> 5], bit, keep_visited, pol_keep) & bit) == 0u;
+  };
   while (true) {
-    if (tid == 0) s.q = atomicAdd(work, 1u);
+    if (tid == 0) {
+      s.q = atomicAdd(work, 1u);
+      s.qnorm = 0;
+      s.fraction = 0;
+    }
     __syncthreads();
     const uint32_t q = s.q;
     if (q >= nq) break;
     const QueryParams P = params[q];
     for (uint32_t i = tid; i < rc; i += blockDim.x) qn[i] = queries[(size_t)q * rc + i];
+    if (cfg.smem_bitmap)
+      for (uint32_t i = tid; i < cfg.bitmap_words / 4; i += blockDim.x)
+        reinterpret_cast<uint4*>(sbitmap)[i] = make_uint4(0, 0, 0, 0);
     __syncthreads();
     if constexpr (Dot::kSq8) {
       // 16 negated values per row chunk: -(2^23 + rint(256 (q - offset) / s)), 0 past dim
       const float* qf = reinterpret_cast<const float*>(qn);
       float* qv = reinterpret_cast<float*>(qs);
+      bool whole = cfg.sq_dot != 0;
+      uint32_t qq = 0;
       for (uint32_t i = tid; i < sc * 16; i += blockDim.x) {
         float v = 0.f;
         if (i < cfg.dim) v = fminf(fmaxf(rintf((qf[i] - cfg.sq_offset) * cfg.sq_in), -8388607.f), 8388607.f);
         qv[i] = -(8388608.f + v);
+        // a query of whole codes 0..255 is scored by integer dot products
+        const float c = v * (1.f / 256.f);
+        const bool code = c >= 0.f && c <= 255.f && c == rintf(c);
+        whole = whole && code;
+        const uint32_t u = code ? (uint32_t)c : 0u;
+        qcode[i] = (uint8_t)u;
+        qq += u * u;
       }
+      qq = __reduce_add_sync(0xffffffffu, qq);
+      if (lane == 0 && qq) atomicAdd(&s.qnorm, qq);
+      if (!whole) s.fraction = 1;
     } else if constexpr (ST != OT) {
       const float* qf = reinterpret_cast<const float*>(qn);
       uint32_t* qb = reinterpret_cast<uint32_t*>(qs);
@@ -372,8 +461,8 @@ graph_search_wide_kernel(DevGraph g, const uint4* __restrict__ srows, const uint
       for (uint32_t i = tid; i < sc; i += blockDim.x) qs[i] = qn[i];
     }
     if (tid == 0) {
-      s.n = 0; s.cur = 0; s.scan0 = 0; s.spill_n = 0; s.spill_min = ~0ull; s.refill = 0; s.done = 0;
-      s.status = 0; s.dc = 0; s.expansions = 0; s.edges = 0; s.visited = 0;
+      s.spill_n = 0; s.spill_min = ~0ull; s.refill = 0; s.first_new = 0xffffffffu; s.kept = 0;
+      s.status = 0; s.dc = 0; s.expansions = 0; s.edges = 0;
     }
     __syncthreads();
     if (P.size == 0) {
@@ -420,27 +509,25 @@ graph_search_wide_kernel(DevGraph g, const uint4* __restrict__ srows, const uint
         uint32_t id = 0;
         if (i < nseeds) {
           id = seeds[i];
-          if (id < g.nrows) {
-            uint32_t bit = 1u << (id & 31u);
-            fresh = (visit_or(&bitmap[id >> 5], bit, keep_visited, pol_keep) & bit) == 0u;
-          }
+          if (id < g.nrows) fresh = visit(id);
         }
         unsigned bal = __ballot_sync(0xffffffffu, fresh);
         if (fresh) nid[m + __popc(bal & ((1u << lane) - 1u))] = id;
         m += __popc(bal);
       }
-      if (lane == 0) { s.cnt = m; s.status |= st; s.dc = m; s.visited = m; }
+      if (lane == 0) { s.cnt = m; s.status |= st; s.dc = m; }
     }
     __syncthreads();
+    // Alike in every thread: the list is lists[cur * L ..], n entries; warp 0 also keeps
+    // the first entry that may be unexpanded.
+    uint32_t n = 0, cur = 0, scan0 = 0;
     {
       const uint32_t m = s.cnt;
-      score(m);
-      for (uint32_t i = tid; i < m; i += blockDim.x) nkey[i] = pack_key(nd[i], nid[i]);
+      score(m, Limits{INFINITY, INFINITY, ~0ull, true});
       __syncthreads();
       cta_bitonic_sort(nkey, m, NB);
-      const uint32_t n0 = min(m, L);
-      for (uint32_t i = tid; i < n0; i += blockDim.x) lists[i] = nkey[i];
-      if (tid == 0) s.n = n0;
+      n = min(m, L);
+      for (uint32_t i = tid; i < n; i += blockDim.x) lists[i] = nkey[i];
       __syncthreads();
     }
     const float user_radius = P.radius;
@@ -449,10 +536,16 @@ graph_search_wide_kernel(DevGraph g, const uint4* __restrict__ srows, const uint
     for (uint32_t it = 0; it < cfg.max_iters; it++) {
       // control (warp 0): refill from the spill tier when flagged, then pick parents
       if (warp == 0) {
-        unsigned long long* list = lists + (size_t)s.cur * L;
-        uint32_t n = s.n, scan0 = s.scan0, spill_n = s.spill_n;
+        unsigned long long* list = lists + (size_t)cur * L;
+        uint32_t spill_n = s.spill_n;
         unsigned long long spill_min = s.spill_min;
-        bool refill = s.refill != 0;
+        const bool refill = s.refill != 0;
+        scan0 = min(scan0, s.first_new);
+        __syncwarp();
+        if (spill_n > cfg.spill_cap) {
+          spill_n = cfg.spill_cap;
+          if (lane == 0) s.status |= kStatusCandidateOverflow;
+        }
         float rk = (n >= P.size) ? fminf(key_dist(list[P.size - 1]), user_radius) : user_radius;
         const float limit = P.coef * rk;
         if (refill) {
@@ -472,7 +565,7 @@ graph_search_wide_kernel(DevGraph g, const uint4* __restrict__ srows, const uint
           if (r > room) {
             unsigned long long prefix = 0, mask = 0;
             uint32_t need = room;
-            uint32_t* hist = reinterpret_cast<uint32_t*>(nd);
+            uint32_t* hist = reinterpret_cast<uint32_t*>(nsorted);
             for (int shift = 56; shift >= 0; shift -= 8) {
               for (uint32_t i = lane; i < 256; i += 32) hist[i] = 0;
               __syncwarp();
@@ -519,24 +612,25 @@ graph_search_wide_kernel(DevGraph g, const uint4* __restrict__ srows, const uint
           n += moved;
           spill_n = stay;
           spill_min = smin;
-          refill = false;
         }
         uint32_t np = 0;
         bool stop = false;
         for (uint32_t b = scan0 & ~31u; b < n && !stop && np < cfg.parents; b += 32) {
           uint32_t i = b + lane;
           unsigned long long k = i < n ? list[i] : ~0ull;
-          unsigned ball = __ballot_sync(0xffffffffu, i < n && !key_expanded(k));
-          while (ball && np < cfg.parents) {
-            int j = __ffs(ball) - 1;
-            unsigned long long kj = __shfl_sync(0xffffffffu, k, j);
-            if (key_dist(kj) > limit) { stop = true; break; }
-            if (lane == j) list[i] = k | kExpandedBit;
-            if (lane == 0) s.parents[np] = key_rawid(kj);
-            np++;
-            scan0 = b + (uint32_t)j + 1;
-            ball &= ball - 1;
+          // the unexpanded entries within the limit, in order, as many as there is room for
+          const unsigned open = __ballot_sync(0xffffffffu, i < n && !key_expanded(k));
+          const unsigned within = open & __ballot_sync(0xffffffffu, i < n && !(key_dist(k) > limit));
+          const uint32_t rank = (uint32_t)__popc(within & ((1u << lane) - 1u));
+          const bool take = ((within >> lane) & 1u) && np + rank < cfg.parents;
+          if (take) {
+            list[i] = k | kExpandedBit;
+            s.parents[np + rank] = key_rawid(k);
           }
+          const unsigned taken = __ballot_sync(0xffffffffu, take);
+          if (taken) scan0 = b + 32u - (uint32_t)__clz((int)taken);
+          np += (uint32_t)__popc(taken);
+          stop = np < cfg.parents && open != within;       // the list is sorted: the rest is past the limit
         }
         __syncwarp();
         uint32_t done = 0, next_refill = 0;
@@ -571,21 +665,25 @@ graph_search_wide_kernel(DevGraph g, const uint4* __restrict__ srows, const uint
           if (lane == 0) { s.total = total; s.edges += total; s.expansions += np; }
         }
         if (lane == 0) {
-          s.n = n; s.scan0 = scan0; s.spill_n = spill_n; s.spill_min = spill_min;
+          s.n = n; s.spill_n = spill_n; s.spill_min = spill_min;
           s.refill = next_refill; s.done = done; s.np = np; s.limit = limit;
-          s.cnt = 0; s.kept = 0;              // counters of this step's gather and placement
+          // counters of this step's gather, placement and merge
+          s.cnt = 0; s.kept = 0; s.first_new = 0xffffffffu;
         }
       }
       __syncthreads();
       const uint32_t done = s.done, refill_next = s.refill, np = s.np, total = s.total;
-      __syncthreads();              // everyone has read the decision before warp 0 writes the next one
+      n = s.n;
       if (done) break;
-      if (refill_next) continue;
+      if (refill_next) {
+        __syncthreads();            // everyone has read the decision before warp 0 writes the next one
+        continue;
+      }
       // ---- gather: unvisited neighbours of the parents ----------------------------------
       // Every thread takes up to kGatherSlots edge slots (t = base + j*T + tid): all
       // edge loads, then all visited-bit atomics, then one CTA scan of the per-thread
       // counts places the new ids (their order does not matter to this search).
-      constexpr int kGatherSlots = 8;
+      constexpr int kGatherSlots = T >= 512 ? 2 : 8;
       for (uint32_t base0 = 0; base0 < total; base0 += kGatherSlots * (uint32_t)T) {
         uint32_t ids[kGatherSlots];
         uint32_t fm = 0, p2 = 0;
@@ -601,10 +699,7 @@ graph_search_wide_kernel(DevGraph g, const uint4* __restrict__ srows, const uint
 #pragma unroll
         for (int j = 0; j < kGatherSlots; j++) {
           const uint32_t t = base0 + (uint32_t)j * (uint32_t)T + (uint32_t)tid;
-          if (t < total) {
-            const uint32_t bit = 1u << (ids[j] & 31u);
-            if ((visit_or(&bitmap[ids[j] >> 5], bit, keep_visited, pol_keep) & bit) == 0u) fm |= 1u << j;
-          }
+          if (t < total && visit(ids[j])) fm |= 1u << j;
         }
         // places in nid: a warp scan of the per-thread counts and one counter
         // increment per warp (the order of the new ids does not matter to this search)
@@ -625,72 +720,50 @@ graph_search_wide_kernel(DevGraph g, const uint4* __restrict__ srows, const uint
       }
       __syncthreads();
       const uint32_t cnt = s.cnt;
-      if (tid == 0) { s.dc += cnt; s.visited += cnt; }
-      // ---- distances ------------------------------------------------------------------------
-      score(cnt);
-      // ---- placement: below the list's worst -> merged; else within the limit -> spill ---
-      const unsigned long long* list = lists + (size_t)s.cur * L;
-      const uint32_t n = s.n;
-      const unsigned long long worst = (n >= L) ? (list[L - 1] & ~(unsigned long long)kExpandedBit) : ~0ull;
-      const float rk2 = (n >= P.size) ? fminf(key_dist(list[P.size - 1]), user_radius) : user_radius;
-      const float insert_limit = P.coef * rk2;
-      // kept keys are appended through one counter increment per warp and round
-      // (their order does not matter: they are ranked or sorted before the merge)
-      unsigned long long smin = ~0ull;
-      for (uint32_t base0 = 0; base0 < cnt; base0 += blockDim.x) {
-        const uint32_t i = base0 + tid;
-        unsigned long long key = ~0ull;
-        bool live = false;
-        if (i < cnt) {
-          key = pack_key(nd[i], nid[i]);
-          live = nd[i] <= insert_limit;
-        }
-        const bool keep = live && key < worst;
-        const bool spl = live && key >= worst;
-        const unsigned kb = __ballot_sync(0xffffffffu, keep);
-        uint32_t kbase = 0;
-        if (lane == 0 && kb) kbase = atomicAdd(&s.kept, (uint32_t)__popc(kb));
-        kbase = __shfl_sync(0xffffffffu, kbase, 0);
-        if (keep) nkey[kbase + __popc(kb & ((1u << lane) - 1u))] = key;
-        if (spl) {
-          const uint32_t o = atomicAdd(&s.spill_n, 1u);
-          if (o < cfg.spill_cap) spill[o] = key;
-          smin = key < smin ? key : smin;
-        }
+      if (tid == 0) s.dc += cnt;
+      // ---- distances and placement: below the list's worst -> new keys; else spill ----------
+      const unsigned long long* list = lists + (size_t)cur * L;
+      {
+        const float rk = (n >= P.size) ? fminf(key_dist(list[P.size - 1]), user_radius) : user_radius;
+        Limits w;
+        w.limit = P.coef * rk;
+        const float root = Dot::kSq8 ? w.limit / cfg.sq_out : w.limit;
+        w.far = root * root * 1.0001f;
+        w.worst = (n >= L) ? (list[L - 1] & ~(unsigned long long)kExpandedBit) : ~0ull;
+        w.all = false;
+        score(cnt, w);
       }
-      for (int off = 16; off > 0; off >>= 1) {
-        unsigned long long o = __shfl_xor_sync(0xffffffffu, smin, off);
-        smin = o < smin ? o : smin;
-      }
-      if (lane == 0) s.wmin[warp] = smin;
       __syncthreads();
       const uint32_t kept = s.kept;
-      if (tid == 0) {
-        unsigned long long mn = s.spill_min;
-        for (int w = 0; w < T / 32; w++) mn = s.wmin[w] < mn ? s.wmin[w] : mn;
-        s.spill_min = mn;
-        if (s.spill_n > cfg.spill_cap) { s.spill_n = cfg.spill_cap; s.status |= kStatusCandidateOverflow; }
-        s.first_new = 0xffffffffu;
+      if (kept == 0) {
+        __syncthreads();            // everyone has read the counter before warp 0 clears it
+        continue;
       }
-      __syncthreads();
-      if (kept == 0) continue;
       // ---- merge into the other list buffer (entries compare without the expanded bit) ---
-      // Every key's place is its rank among the new keys plus its rank among the list's:
-      // up to T new keys are ranked by counting (no sort, no barrier), more are sorted
-      // first and ranked by binary search.
-      const bool by_count = kept <= (uint32_t)T;
-      if (!by_count) cta_bitonic_sort(nkey, kept, NB);
-      auto rank_new = [&](unsigned long long x, uint32_t j_hint) -> uint32_t {
-        if (!by_count) return j_hint;
+      // Every key's place is its rank among the new keys plus its rank among the list's.
+      // Few new keys are counted against (no barrier); more are sorted first, up to T by
+      // rank, and searched.
+      const bool by_count = kept <= 12;
+      const unsigned long long* nk = nkey;
+      if (!by_count) {
+        if (kept <= (uint32_t)T) {
+          rank_sort_keys<T>(nkey, nsorted, kept);
+          nk = nsorted;
+          __syncthreads();
+        } else {
+          cta_bitonic_sort(nkey, kept, NB);
+        }
+      }
+      auto rank_new = [&](unsigned long long x) -> uint32_t {
+        if (!by_count) return warp_lower_bound(nk, kept, x);
         uint32_t r = 0;
-        for (uint32_t t = 0; t < kept; t++) r += nkey[t] < x ? 1u : 0u;
+        for (uint32_t t = 0; t < kept; t++) r += nk[t] < x ? 1u : 0u;
         return r;
       };
-      unsigned long long* dst = lists + (size_t)(s.cur ^ 1u) * L;
+      unsigned long long* dst = lists + (size_t)(cur ^ 1u) * L;
       for (uint32_t i = tid; i < n; i += blockDim.x) {
         const unsigned long long k = list[i];
-        const unsigned long long km = k & ~(unsigned long long)kExpandedBit;
-        const uint32_t pos = i + (by_count ? rank_new(km, 0u) : warp_lower_bound(nkey, kept, km));
+        const uint32_t pos = i + rank_new(k & ~(unsigned long long)kExpandedBit);
         if (pos < L) dst[pos] = k;
         else if (!key_expanded(k)) {
           const uint32_t o = atomicAdd(&s.spill_n, 1u);
@@ -699,13 +772,13 @@ graph_search_wide_kernel(DevGraph g, const uint4* __restrict__ srows, const uint
         }
       }
       for (uint32_t j = tid; j < kept; j += blockDim.x) {
-        const unsigned long long k = nkey[j];
+        const unsigned long long k = nk[j];
         uint32_t lo = 0, hi = n;
         while (lo < hi) {
           uint32_t mid = (lo + hi) >> 1;
           if ((list[mid] & ~(unsigned long long)kExpandedBit) < k) lo = mid + 1; else hi = mid;
         }
-        const uint32_t pos = rank_new(k, j) + lo;
+        const uint32_t pos = (by_count ? rank_new(k) : j) + lo;
         if (pos < L) {
           dst[pos] = k;
           atomicMin(&s.first_new, pos);
@@ -716,26 +789,21 @@ graph_search_wide_kernel(DevGraph g, const uint4* __restrict__ srows, const uint
         }
       }
       __syncthreads();
-      if (tid == 0) {
-        s.cur ^= 1u;
-        s.n = min(n + kept, L);
-        if (s.first_new < s.scan0) s.scan0 = s.first_new;
-        if (s.spill_n > cfg.spill_cap) { s.spill_n = cfg.spill_cap; s.status |= kStatusCandidateOverflow; }
-      }
-      __syncthreads();
+      cur ^= 1u;
+      n = min(n + kept, L);
     }
     // ---- exact re-rank of the best entries with the full-precision rows --------------------
     {
-      const unsigned long long* list = lists + (size_t)s.cur * L;
-      const uint32_t n = s.n;
+      const unsigned long long* list = lists + (size_t)cur * L;
       const uint32_t R = min(n, max(P.size, (uint32_t)((P.size * cfg.rerank_x16 + 15) / 16)));
-      const uint32_t gpb = (uint32_t)T / NG;
+      const int pw = packed_width(NG);
+      const uint32_t gpb = (uint32_t)T / (uint32_t)pw;
       for (uint32_t b = 0; b < R; b += gpb) {
-        const uint32_t i = b + (uint32_t)(tid / NG);
-        const bool valid = i < R;
-        const uint32_t id = valid ? key_rawid(list[i]) : 0u;
-        float d = group_distance<OT, M>(qn, g.objects + (size_t)id * rc, (int)rc, ngl, NG);
-        if (valid && ngl == 0) nkey[i] = pack_key(d, id);
+        const uint32_t i = b + (uint32_t)(tid / pw);
+        const uint32_t id[1] = {i < R ? key_rawid(list[i]) : 0u};
+        Acc<OT, M> sum[1];
+        packed_sums<OT, M, 1>(qn, g.objects, id, (int)rc, lane & (pw - 1), NG, sum);
+        if (i < R && (lane & (pw - 1)) == 0) nkey[i] = pack_key(sum[0].finish(), id[0]);
       }
       __syncthreads();
       cta_bitonic_sort(nkey, R, NB);
@@ -751,12 +819,14 @@ graph_search_wide_kernel(DevGraph g, const uint4* __restrict__ srows, const uint
         }
         if (lane == 0) {
           out_count[q] = nout;
-          stats[q] = QueryStats{s.dc, s.expansions, s.visited, s.edges, s.status};
+          stats[q] = QueryStats{s.dc, s.expansions, s.dc, s.edges, s.status};
         }
       }
     }
-    uint4* bm4 = reinterpret_cast<uint4*>(bitmap);
-    for (uint32_t i = tid; i < cfg.bitmap_words / 4; i += blockDim.x) store_zero16(bm4 + i, keep_visited, pol_keep);
+    if (!cfg.smem_bitmap) {
+      uint4* bm4 = reinterpret_cast<uint4*>(bitmap);
+      for (uint32_t i = tid; i < cfg.bitmap_words / 4; i += blockDim.x) store_zero16(bm4 + i, keep_visited, pol_keep);
+    }
     __syncthreads();
   }
 }

@@ -1,15 +1,17 @@
 // Instantiations of the CTA-per-query ("wide") batched graph search for the
-// distances other than L2: the objects themselves are the search rows, 256
-// threads per query.  A translation unit of its own so that they compile in
+// distances other than L2: the objects themselves are the search rows, 256 or
+// 512 threads per query.  A translation unit of its own so that they compile in
 // parallel with the L2 instantiations.
 #include "graph_wide.cuh"
 #include "kernels.h"
 
 namespace ngtg {
 
-WideKernelFn wide_kernel_native(ObjType ot, Metric m) {
+WideKernelFn wide_kernel_native(ObjType ot, Metric m, uint32_t threads) {
 #define NGT_WIDE(OT, M) \
-  case Metric::M: return &graph_search_wide_kernel<ObjType::OT, ObjType::OT, Metric::M, 256>;
+  case Metric::M:                                                                             \
+    return threads == 512 ? &graph_search_wide_kernel<ObjType::OT, ObjType::OT, Metric::M, 512> \
+                          : &graph_search_wide_kernel<ObjType::OT, ObjType::OT, Metric::M, 256>;
   switch (ot) {
     case ObjType::Float:
       switch (m) {
