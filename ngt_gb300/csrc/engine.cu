@@ -91,6 +91,21 @@ bool is_normalized(Metric m) {
 
 }  // namespace
 
+// The engine's own memory pool for the buffers of one call.  The device's default pool
+// returns its memory to the driver at every synchronisation, so that each host-buffer call
+// mapped its few buffers anew (about 0.3 ms); this one keeps up to 64 MB until the engine
+// closes.
+void GraphEngine::create_pool() {
+  cudaMemPoolProps props{};
+  props.allocType = cudaMemAllocationTypePinned;
+  props.handleTypes = cudaMemHandleTypeNone;
+  props.location.type = cudaMemLocationTypeDevice;
+  props.location.id = device_;
+  NGT_CUDA(cudaMemPoolCreate(&pool_, &props));
+  uint64_t keep = 64ull << 20;
+  NGT_CUDA(cudaMemPoolSetAttribute(pool_, cudaMemPoolAttrReleaseThreshold, &keep));
+}
+
 GraphEngine::GraphEngine(const std::string& path, GraphMode mode, bool quantized) : mode_(mode) {
   load_index(path, host_);
   if (!exact_kernel(host_.prop.otype, host_.prop.metric))
@@ -100,6 +115,7 @@ GraphEngine::GraphEngine(const std::string& path, GraphMode mode, bool quantized
   if (quantized) read_qg();
   NGT_CUDA(cudaGetDevice(&device_));
   NGT_CUDA(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking));
+  create_pool();
   upload();
   if (quantized) upload_qg();
   // The no-allocation search's fixed scratch and the exact kernel live in modules
@@ -150,6 +166,7 @@ GraphEngine::GraphEngine(const std::string& qbg_dir, bool blobs) : mode_(GraphMo
   }
   NGT_CUDA(cudaGetDevice(&device_));
   NGT_CUDA(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking));
+  create_pool();
   upload();
   auto up = [&](const void* src, size_t bytes) {
     void* p = dmalloc_copy<void>(src, bytes);
@@ -216,6 +233,7 @@ GraphEngine::~GraphEngine() {
   if (linear_scratch_.pinned) cudaFreeHost(linear_scratch_.pinned);
   tc_release(tc_);
   if (stream_) cudaStreamDestroy(stream_);
+  if (pool_) cudaMemPoolDestroy(pool_);
 }
 
 void GraphEngine::upload() {
@@ -679,8 +697,8 @@ void GraphEngine::search_device(const uint4* d_rows, size_t nq, const SearchArgs
   QueryParams* d_params = nullptr;
   uint32_t* d_seeds = nullptr;
   // the launch's own work counter lies behind its parameters
-  NGT_CUDA(cudaMallocAsync(&d_params, nq * sizeof(QueryParams) + 4, stream));
-  NGT_CUDA(cudaMallocAsync(&d_seeds, seeds.size() * 4, stream));
+  NGT_CUDA(dev_alloc(&d_params, nq * sizeof(QueryParams) + 4, stream));
+  NGT_CUDA(dev_alloc(&d_seeds, seeds.size() * 4, stream));
   NGT_CUDA(cudaMemcpyAsync(d_params, params.data(), nq * sizeof(QueryParams), cudaMemcpyHostToDevice, stream));
   NGT_CUDA(cudaMemcpyAsync(d_seeds, seeds.data(), seeds.size() * 4, cudaMemcpyHostToDevice, stream));
   if (kernel == Kernel::Exact)
@@ -710,8 +728,8 @@ void GraphEngine::search_device_slot(const uint4* d_rows, size_t nq, const Searc
   build_params(args, nargs, nq, kmax, params, seeds, max_size);
   QueryParams* d_params = nullptr;
   uint32_t* d_seeds = nullptr;
-  NGT_CUDA(cudaMallocAsync(&d_params, nq * sizeof(QueryParams), stream));
-  NGT_CUDA(cudaMallocAsync(&d_seeds, seeds.size() * 4, stream));
+  NGT_CUDA(dev_alloc(&d_params, nq * sizeof(QueryParams), stream));
+  NGT_CUDA(dev_alloc(&d_seeds, seeds.size() * 4, stream));
   NGT_CUDA(cudaMemcpyAsync(d_params, params.data(), nq * sizeof(QueryParams), cudaMemcpyHostToDevice, stream));
   NGT_CUDA(cudaMemcpyAsync(d_seeds, seeds.data(), seeds.size() * 4, cudaMemcpyHostToDevice, stream));
   if (kernel == Kernel::Wide)
@@ -981,10 +999,10 @@ void GraphEngine::search(const void* queries, QueryType qt, size_t nq, size_t qd
   uint32_t* d_counts = nullptr;
   QueryStats* d_stats = nullptr;
   cudaStream_t s = stream_;
-  NGT_CUDA(cudaMallocAsync(&d_rows, row_total, s));
-  NGT_CUDA(cudaMallocAsync(&d_out, nq * kmax * sizeof(ObjDist), s));
-  NGT_CUDA(cudaMallocAsync(&d_counts, nq * 4, s));
-  NGT_CUDA(cudaMallocAsync(&d_stats, nq * sizeof(QueryStats), s));
+  NGT_CUDA(dev_alloc(&d_rows, row_total, s));
+  NGT_CUDA(dev_alloc(&d_out, nq * kmax * sizeof(ObjDist), s));
+  NGT_CUDA(dev_alloc(&d_counts, nq * 4, s));
+  NGT_CUDA(dev_alloc(&d_stats, nq * sizeof(QueryStats), s));
   NGT_CUDA(cudaMemcpyAsync(d_rows, staging_, row_total, cudaMemcpyHostToDevice, s));
   search_device(d_rows, nq, args, nargs, d_out, d_counts, d_stats, kmax, s, kernel);
   NGT_CUDA(cudaMemcpyAsync(out.results.data(), d_out, nq * kmax * sizeof(ObjDist), cudaMemcpyDeviceToHost, s));
@@ -1017,7 +1035,7 @@ void GraphEngine::linear_search_tc_host(const float* queries, size_t nq, size_t 
   const size_t o_st = o_cnt + al(nq * 4), total = o_st + al(nq * 4);
   cudaStream_t s = stream_;
   uint8_t* d = nullptr;
-  NGT_CUDA(cudaMallocAsync(&d, total, s));
+  NGT_CUDA(dev_alloc(&d, total, s));
   try {
     NGT_CUDA(cudaMemcpyAsync(d, staging_, row_total, cudaMemcpyHostToDevice, s));
     linear_search_tc_device(reinterpret_cast<const uint4*>(d), nq, size, candidates,
@@ -1073,12 +1091,12 @@ void GraphEngine::search_refined(const void* queries, QueryType qt, size_t nq, s
   ObjDist *d_cand = nullptr, *d_out = nullptr;
   uint32_t *d_cc = nullptr, *d_exact = nullptr, *d_counts = nullptr;
   float* d_q = nullptr;
-  NGT_CUDA(cudaMallocAsync(&d_cand, cand.results.size() * sizeof(ObjDist), s));
-  NGT_CUDA(cudaMallocAsync(&d_cc, nq * 4, s));
-  NGT_CUDA(cudaMallocAsync(&d_exact, nq * 4, s));
-  NGT_CUDA(cudaMallocAsync(&d_q, nq * qdim * 4, s));
-  NGT_CUDA(cudaMallocAsync(&d_out, nq * kmax * sizeof(ObjDist), s));
-  NGT_CUDA(cudaMallocAsync(&d_counts, nq * 4, s));
+  NGT_CUDA(dev_alloc(&d_cand, cand.results.size() * sizeof(ObjDist), s));
+  NGT_CUDA(dev_alloc(&d_cc, nq * 4, s));
+  NGT_CUDA(dev_alloc(&d_exact, nq * 4, s));
+  NGT_CUDA(dev_alloc(&d_q, nq * qdim * 4, s));
+  NGT_CUDA(dev_alloc(&d_out, nq * kmax * sizeof(ObjDist), s));
+  NGT_CUDA(dev_alloc(&d_counts, nq * 4, s));
   NGT_CUDA(cudaMemcpyAsync(d_cand, cand.results.data(), cand.results.size() * sizeof(ObjDist),
                            cudaMemcpyHostToDevice, s));
   NGT_CUDA(cudaMemcpyAsync(d_cc, cand.counts.data(), nq * 4, cudaMemcpyHostToDevice, s));
@@ -1488,8 +1506,8 @@ void GraphEngine::qg_search_device(const uint4* d_rows, size_t nq, const QGArgs*
   QGParams* d_params = nullptr;
   uint32_t* d_seeds = nullptr;
   // the launch's own work counter lies behind its parameters
-  NGT_CUDA(cudaMallocAsync(&d_params, nq * sizeof(QGParams) + 4, stream));
-  NGT_CUDA(cudaMallocAsync(&d_seeds, seeds.size() * 4, stream));
+  NGT_CUDA(dev_alloc(&d_params, nq * sizeof(QGParams) + 4, stream));
+  NGT_CUDA(dev_alloc(&d_seeds, seeds.size() * 4, stream));
   NGT_CUDA(cudaMemcpyAsync(d_params, params.data(), nq * sizeof(QGParams), cudaMemcpyHostToDevice, stream));
   NGT_CUDA(cudaMemcpyAsync(d_seeds, seeds.data(), seeds.size() * 4, cudaMemcpyHostToDevice, stream));
   if (grid < nq) {
@@ -1568,8 +1586,8 @@ void GraphEngine::qg_search_device_relaxed(const uint4* d_rows, size_t nq, const
   NGT_CUDA(cudaMemsetAsync(scratch.work, 0, 4, stream));
   QGParams* d_params = nullptr;
   uint32_t* d_seeds = nullptr;
-  NGT_CUDA(cudaMallocAsync(&d_params, nq * sizeof(QGParams), stream));
-  NGT_CUDA(cudaMallocAsync(&d_seeds, seeds.size() * 4, stream));
+  NGT_CUDA(dev_alloc(&d_params, nq * sizeof(QGParams), stream));
+  NGT_CUDA(dev_alloc(&d_seeds, seeds.size() * 4, stream));
   NGT_CUDA(cudaMemcpyAsync(d_params, params.data(), nq * sizeof(QGParams), cudaMemcpyHostToDevice, stream));
   NGT_CUDA(cudaMemcpyAsync(d_seeds, seeds.data(), seeds.size() * 4, cudaMemcpyHostToDevice, stream));
   fn<<<(unsigned)grid, kQGWideThreads, smem, stream>>>(dev_, dqg_, d_rows, (uint32_t)nq, d_params, d_seeds,
@@ -1600,10 +1618,10 @@ void GraphEngine::qg_search(const void* queries, QueryType qt, size_t nq, size_t
   uint32_t* d_counts = nullptr;
   QueryStats* d_stats = nullptr;
   cudaStream_t s = stream_;
-  NGT_CUDA(cudaMallocAsync(&d_rows, rows.size(), s));
-  NGT_CUDA(cudaMallocAsync(&d_out, nq * kmax * sizeof(ObjDist), s));
-  NGT_CUDA(cudaMallocAsync(&d_counts, nq * 4, s));
-  NGT_CUDA(cudaMallocAsync(&d_stats, nq * sizeof(QueryStats), s));
+  NGT_CUDA(dev_alloc(&d_rows, rows.size(), s));
+  NGT_CUDA(dev_alloc(&d_out, nq * kmax * sizeof(ObjDist), s));
+  NGT_CUDA(dev_alloc(&d_counts, nq * 4, s));
+  NGT_CUDA(dev_alloc(&d_stats, nq * sizeof(QueryStats), s));
   NGT_CUDA(cudaMemcpyAsync(d_rows, rows.data(), rows.size(), cudaMemcpyHostToDevice, s));
   if (relaxed) qg_search_device_relaxed(d_rows, nq, args, nargs, d_out, d_counts, d_stats, kmax, s);
   else qg_search_device(d_rows, nq, args, nargs, d_out, d_counts, d_stats, kmax, s);
@@ -1705,9 +1723,9 @@ void GraphEngine::qbg_probe_blobs(const uint4* d_rows, size_t nq, const QBGArgs*
     QueryParams* d_params = nullptr;
     uint32_t* d_seeds = nullptr;
     QueryStats* d_st = nullptr;
-    NGT_CUDA(cudaMallocAsync(&d_params, nq * sizeof(QueryParams) + 4, stream));
-    NGT_CUDA(cudaMallocAsync(&d_seeds, seeds.size() * 4, stream));
-    NGT_CUDA(cudaMallocAsync(&d_st, nq * sizeof(QueryStats), stream));
+    NGT_CUDA(dev_alloc(&d_params, nq * sizeof(QueryParams) + 4, stream));
+    NGT_CUDA(dev_alloc(&d_seeds, seeds.size() * 4, stream));
+    NGT_CUDA(dev_alloc(&d_st, nq * sizeof(QueryStats), stream));
     NGT_CUDA(cudaMemcpyAsync(d_params, params.data(), nq * sizeof(QueryParams), cudaMemcpyHostToDevice, stream));
     NGT_CUDA(cudaMemcpyAsync(d_seeds, seeds.data(), seeds.size() * 4, cudaMemcpyHostToDevice, stream));
     uint32_t* work = reinterpret_cast<uint32_t*>(d_params + nq);
@@ -1795,13 +1813,13 @@ void GraphEngine::qbg_search_device(const uint4* d_rows, size_t nq, const QBGArg
   ObjDist* d_sout = d_out;
   uint32_t* d_scount = d_counts;
   if (refine) {
-    NGT_CUDA(cudaMallocAsync(&d_sout, nq * stride * sizeof(ObjDist), stream));
-    NGT_CUDA(cudaMallocAsync(&d_scount, nq * 4, stream));
+    NGT_CUDA(dev_alloc(&d_sout, nq * stride * sizeof(ObjDist), stream));
+    NGT_CUDA(dev_alloc(&d_scount, nq * 4, stream));
   }
   QBGParams* d_params = nullptr;
   uint32_t* d_seeds = nullptr;
-  NGT_CUDA(cudaMallocAsync(&d_params, nq * sizeof(QBGParams), stream));
-  NGT_CUDA(cudaMallocAsync(&d_seeds, seeds.size() * 4, stream));
+  NGT_CUDA(dev_alloc(&d_params, nq * sizeof(QBGParams), stream));
+  NGT_CUDA(dev_alloc(&d_seeds, seeds.size() * 4, stream));
   NGT_CUDA(cudaMemcpyAsync(d_params, params.data(), nq * sizeof(QBGParams), cudaMemcpyHostToDevice, stream));
   NGT_CUDA(cudaMemcpyAsync(d_seeds, seeds.data(), seeds.size() * 4, cudaMemcpyHostToDevice, stream));
   auto ensure_blob_dist = [&](size_t grid, uint32_t ocap) {
@@ -1821,8 +1839,8 @@ void GraphEngine::qbg_search_device(const uint4* d_rows, size_t nq, const QBGArg
   if (two_step) {
     ObjDist* d_blobs = nullptr;
     uint32_t* d_bcounts = nullptr;
-    NGT_CUDA(cudaMallocAsync(&d_blobs, nq * max_probes * sizeof(ObjDist), stream));
-    NGT_CUDA(cudaMallocAsync(&d_bcounts, nq * 4, stream));
+    NGT_CUDA(dev_alloc(&d_blobs, nq * max_probes * sizeof(ObjDist), stream));
+    NGT_CUDA(dev_alloc(&d_bcounts, nq * 4, stream));
     qbg_probe_blobs(d_rows, nq, args, nargs, d_blobs, d_bcounts, max_probes, stream, slot);
     QBGScanKernelFn fn = qbg_scan_kernel_for(qb_.m);
     if (!fn) throw std::runtime_error("too many subspaces in the QBG index");
@@ -1891,7 +1909,7 @@ void GraphEngine::qbg_search_device(const uint4* d_rows, size_t nq, const QBGArg
   }
   if (refine) {
     uint32_t* d_exact = nullptr;
-    NGT_CUDA(cudaMallocAsync(&d_exact, nq * 4, stream));
+    NGT_CUDA(dev_alloc(&d_exact, nq * 4, stream));
     NGT_CUDA(cudaMemcpyAsync(d_exact, exact.data(), nq * 4, cudaMemcpyHostToDevice, stream));
     const uint32_t P = next_pow2(std::max<uint32_t>(max_size, 2));
     const size_t smem = (size_t)olist_chunks_ * 16 + (size_t)P * 8;
@@ -1939,10 +1957,10 @@ void GraphEngine::qbg_search(const void* queries, QueryType qt, size_t nq, size_
   uint32_t* d_counts = nullptr;
   QueryStats* d_stats = nullptr;
   cudaStream_t s = stream_;
-  NGT_CUDA(cudaMallocAsync(&d_rows, rows.size(), s));
-  NGT_CUDA(cudaMallocAsync(&d_out, nq * kmax * sizeof(ObjDist), s));
-  NGT_CUDA(cudaMallocAsync(&d_counts, nq * 4, s));
-  NGT_CUDA(cudaMallocAsync(&d_stats, nq * sizeof(QueryStats), s));
+  NGT_CUDA(dev_alloc(&d_rows, rows.size(), s));
+  NGT_CUDA(dev_alloc(&d_out, nq * kmax * sizeof(ObjDist), s));
+  NGT_CUDA(dev_alloc(&d_counts, nq * 4, s));
+  NGT_CUDA(dev_alloc(&d_stats, nq * sizeof(QueryStats), s));
   NGT_CUDA(cudaMemcpyAsync(d_rows, rows.data(), rows.size(), cudaMemcpyHostToDevice, s));
   qbg_search_device(d_rows, nq, args, nargs, d_out, d_counts, d_stats, kmax, s);
   NGT_CUDA(cudaMemcpyAsync(out.results.data(), d_out, nq * kmax * sizeof(ObjDist), cudaMemcpyDeviceToHost, s));

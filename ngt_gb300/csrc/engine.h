@@ -411,6 +411,13 @@ class GraphEngine {
   std::vector<void*> qg_buffers_;
   int device_ = 0;
   cudaStream_t stream_ = nullptr;
+  cudaMemPool_t pool_ = nullptr;
+  void create_pool();
+  // stream-ordered allocation from the engine's pool (freed with cudaFreeAsync)
+  template <typename T>
+  cudaError_t dev_alloc(T** p, size_t bytes, cudaStream_t s) {
+    return cudaMallocFromPoolAsync(reinterpret_cast<void**>(p), bytes, pool_, s);
+  }
   std::mutex mu_;
   std::mutex staging_mu_;                                 // the pinned query staging of search()
   void* staging_ = nullptr;
