@@ -19,7 +19,7 @@
 //      pipeline, accumulators double-buffered in TMEM (2 x 256 columns) and
 //      read back with tcgen05.ld by sixteen epilogue warps (four per TMEM lane
 //      quadrant).  The first `first_rows` rows are written out densely; on the
-//      remaining rows, taken in parts that double in size, the epilogue keeps
+//      remaining rows, taken in growing parts (part_growth), the epilogue keeps
 //      only scores that beat the query's threshold, and tc_compact_kernel cuts
 //      each list back to the C best and raises the threshold between two parts.
 //      A two-SM form (cta_group::2, M = 256 over a pair of CTAs, each staging
@@ -47,6 +47,7 @@
 #include <algorithm>
 #include <array>
 #include <cfloat>
+#include <cmath>
 #include <memory>
 #include <stdexcept>
 #include <string>
@@ -78,28 +79,36 @@ constexpr uint32_t SMEM_BYTES = STAGES * STAGE_BYTES + 1024;   // + slack for 10
 // one half (128 queries) of the query tile, 32 KB per k-block, in 6 stages.
 constexpr uint32_t STAGES2 = 6;
 constexpr uint32_t STAGE2_BYTES = A_BYTES + B_BYTES / 2;
-constexpr uint32_t MAX_STAGES = STAGES2 > STAGES ? STAGES2 : STAGES;
+// Up to 64 queries take tiles of 64 (SMALL_BN), 24 KB per k-block in 8 stages: the rows are
+// then what bounds the kernel (HBM), and a tile of 256 would move 32 KB of query padding
+// from L2 beside each 16 KB of rows and keep half as many rows in flight (33 queries over
+// 476K x 768: 155 us, 4.7 TB/s, before).
+constexpr uint32_t SMALL_BN = 64;
+constexpr uint32_t STAGES_SMALL = 8;
+constexpr uint32_t STAGE_SMALL_BYTES = A_BYTES + SMALL_BN * BK * 2;
+constexpr uint32_t MAX_STAGES = STAGES_SMALL;
 static_assert(STAGES2 * STAGE2_BYTES + 1024 <= SMEM_BYTES, "two-SM stages fit the same shared memory");
-constexpr uint32_t EPI_WARPS = 16;      // four per TMEM lane quadrant, each a quarter of the columns
-constexpr uint32_t EPI_PARTS = EPI_WARPS / 4;
-constexpr uint32_t THREADS = 64 + 32 * EPI_WARPS;   // warp 0 TMA, warp 1 MMA, warps 2.. epilogue
-constexpr uint32_t TMEM_COLS = 2 * BN;
+static_assert(STAGES_SMALL * STAGE_SMALL_BYTES + 1024 <= SMEM_BYTES, "small-tile stages fit the same shared memory");
+// epilogue warps: four (small tiles: two) per TMEM lane quadrant, each a part of the columns
+constexpr uint32_t epi_warps(uint32_t bn) { return bn == SMALL_BN ? 8 : 16; }
+constexpr uint32_t tc_threads(uint32_t bn) { return 64 + 32 * epi_warps(bn); }   // warp 0 TMA, 1 MMA, 2.. epilogue
 constexpr uint32_t kInvalidKey = 0xff800000u;   // score key of -inf; valid keys are smaller
 constexpr uint64_t kWaitNs = 2000000000ull;     // bound of every wait (2 s)
+constexpr uint32_t kErrorOverflow = 8u;         // bit of the error word: a candidate list overflowed
 constexpr int kDeferQueries = 8;                // filter epilogue: see tc_score_kernel
 
 // Instruction descriptor of tcgen05.mma kind::f16: D fp32 (bits 4-5 = 1), A and
 // B bf16 (bits 7-9, 10-12 = 1), both K-major (bits 15, 16 = 0), N >> 3 at bits
 // 17-22, M >> 4 at bits 24-28.
-constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((BN >> 3) << 17) | ((BM >> 4) << 24);
+constexpr uint32_t idesc_bf16(uint32_t bn) { return (1u << 4) | (1u << 7) | (1u << 10) | ((bn >> 3) << 17) | ((BM >> 4) << 24); }
 // kind::f8f6f4 with A and B E4M3 (format 0 at bits 7-9 and 10-12), D fp32.  One MMA
 // consumes K = 32 one-byte elements, the same 32 bytes of each 128-byte swizzle
 // row as a bf16 MMA's K = 16, so staging, descriptors and k-steps are shared.
-constexpr uint32_t kIdescF8 = (1u << 4) | ((BN >> 3) << 17) | ((BM >> 4) << 24);
+constexpr uint32_t idesc_f8(uint32_t bn) { return (1u << 4) | ((bn >> 3) << 17) | ((BM >> 4) << 24); }
 // The same with M = 256 for a pair of CTAs (cta_group::2): rows 0-127 from the
 // first CTA's A tile, 128-255 from the second's; each accumulates its own 128 rows.
-constexpr uint32_t kIdesc2 = (kIdesc & ~(0x1Fu << 24)) | (((2 * BM) >> 4) << 24);
-constexpr uint32_t kIdescF8_2 = (kIdescF8 & ~(0x1Fu << 24)) | (((2 * BM) >> 4) << 24);
+constexpr uint32_t kIdesc2 = (idesc_bf16(BN) & ~(0x1Fu << 24)) | (((2 * BM) >> 4) << 24);
+constexpr uint32_t kIdescF8_2 = (idesc_f8(BN) & ~(0x1Fu << 24)) | (((2 * BM) >> 4) << 24);
 constexpr float kE4M3Max = 448.f;       // largest finite E4M3 value
 
 struct ScoreArgs {
@@ -115,7 +124,7 @@ struct ScoreArgs {
   uint32_t* cand_count;
   uint32_t cap;
   uint32_t* status;                     // bit 1: candidate list overflow
-  uint32_t* error;                      // bit 1: producer wait, 2: MMA wait, 4: epilogue wait ran out
+  uint32_t* error;                      // bit 1: producer wait, 2: MMA wait, 4: epilogue wait ran out (8: overflow)
   const float* qscale;                  // fp8 scores: per-query dequantisation scale (bf16: unused)
 };
 
@@ -226,16 +235,18 @@ __device__ __forceinline__ uint64_t sw128_desc(uint32_t saddr) {
          ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
 }
 
+template <uint32_t kBN>
 __device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t accumulate) {
   asm volatile(
       "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}"
-      ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(kIdesc), "r"(accumulate)
+      ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc_bf16(kBN)), "r"(accumulate)
       : "memory");
 }
+template <uint32_t kBN>
 __device__ __forceinline__ void mma_f8(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t accumulate) {
   asm volatile(
       "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n}"
-      ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(kIdescF8), "r"(accumulate)
+      ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc_f8(kBN)), "r"(accumulate)
       : "memory");
 }
 __device__ __forceinline__ void mma_commit(uint32_t bar) {
@@ -328,19 +339,24 @@ __device__ __forceinline__ float key_score(uint32_t key) {
 // stage barrier; the MMA commits arrive on both CTAs' stage-empty and
 // accumulator-full barriers; both CTAs' epilogue warps arrive on the first
 // CTA's accumulator-empty barrier.
-template <bool kDense, bool kFp8, bool kPair>
-__global__ void __launch_bounds__(THREADS, 1)
+// kBN: queries per tile (BN, or SMALL_BN without kPair).
+template <bool kDense, bool kFp8, bool kPair, uint32_t kBN>
+__global__ void __launch_bounds__(tc_threads(kBN), 1)
 tc_score_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB, ScoreArgs a) {
-  constexpr uint32_t NST = kPair ? STAGES2 : STAGES;
-  constexpr uint32_t SBYTES = kPair ? STAGE2_BYTES : STAGE_BYTES;
+  static_assert(kBN == BN || (kBN == SMALL_BN && !kPair), "tile widths");
+  constexpr uint32_t NST = kPair ? STAGES2 : kBN == SMALL_BN ? STAGES_SMALL : STAGES;
+  constexpr uint32_t SBYTES = kPair ? STAGE2_BYTES : kBN == SMALL_BN ? STAGE_SMALL_BYTES : STAGE_BYTES;
+  constexpr uint32_t EPI_WARPS = epi_warps(kBN), EPI_PARTS = EPI_WARPS / 4, TMEM_COLS = 2 * kBN;
   extern __shared__ __align__(1024) unsigned char dsmem[];
   __shared__ __align__(8) uint64_t bar_full[MAX_STAGES], bar_empty[MAX_STAGES], bar_tfull[2], bar_tempty[2], bar_drain;
   __shared__ uint32_t tmem_base_sh;
   __shared__ volatile uint32_t abort_sh;
+  // thresholds of each epilogue warp's queries, read back four to a broadcast load
+  __shared__ __align__(16) float thr_sh[kDense ? 1 : epi_warps(kBN)][kDense ? 4 : kBN / (epi_warps(kBN) / 4)];
   const uint32_t base = (smem_u32(dsmem) + 1023u) & ~1023u;
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t mtiles = (a.row_end - a.row_begin + BM - 1) / BM;
-  const uint32_t ntiles = (a.nq + BN - 1) / BN;
+  const uint32_t ntiles = (a.nq + kBN - 1) / kBN;
   // work units: tiles, or (kPair) pairs of row tiles of one query tile per CTA pair
   const uint32_t rank = kPair ? cluster_ctarank() : 0u;
   const uint32_t unit0 = kPair ? blockIdx.x >> 1 : blockIdx.x;
@@ -390,7 +406,7 @@ tc_score_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
       uint32_t pending = 0, last_parity = 0;     // per stage: a load in flight, parity of its phase
       for (uint32_t t = unit0; t < units && !abort_sh; t += ustep) {
         const int row0 = (int)(a.row_begin + row_tile(t) * BM);
-        const int q0 = (int)((t % ntiles) * BN);
+        const int q0 = (int)((t % ntiles) * kBN);
         for (uint32_t kb = 0; kb < a.kblocks; kb++) {
           if (!mbar_wait(smem_u32(&bar_empty[stage]), phase ^ 1u, &abort_sh)) {
             atomicOr(a.error, 1u);
@@ -406,7 +422,7 @@ tc_score_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
             tma_load_2d_pair(sA, &mapA, fb0, (int)(kb * BK), row0);
             tma_load_2d_pair(sB, &mapB, fb0, (int)(kb * BK), q0 + (int)(rank * (BN / 2)));
           } else {
-            mbar_expect_tx(fb, STAGE_BYTES);
+            mbar_expect_tx(fb, SBYTES);
             tma_load_2d(sA, &mapA, fb, (int)(kb * BK), row0);
             tma_load_2d(sB, &mapB, fb, (int)(kb * BK), q0);
           }
@@ -442,7 +458,7 @@ tc_score_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
           break;
         }
         tc_fence_after();
-        const uint32_t d = tmem + buf * BN;
+        const uint32_t d = tmem + buf * kBN;
         bool ok = true;
         for (uint32_t kb = 0; kb < a.kblocks; kb++) {
           if (!mbar_wait(smem_u32(&bar_full[stage]), phase, &abort_sh)) {
@@ -459,8 +475,8 @@ tc_score_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
             const uint32_t acc = (kb | k) != 0 ? 1u : 0u;
             if constexpr (kPair && kFp8) mma_f8_pair(d, da, db, acc);
             else if constexpr (kPair) mma_bf16_pair(d, da, db, acc);
-            else if constexpr (kFp8) mma_f8(d, da, db, acc);
-            else mma_bf16(d, da, db, acc);
+            else if constexpr (kFp8) mma_f8<kBN>(d, da, db, acc);
+            else mma_bf16<kBN>(d, da, db, acc);
           }
           if constexpr (kPair) mma_commit_pair_both(smem_u32(&bar_empty[stage]));
           else mma_commit(smem_u32(&bar_empty[stage]));
@@ -480,7 +496,7 @@ tc_score_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
     }
   } else {
     // epilogue: warp w reads TMEM lanes 32 * (w % 4) .. + 31 (one row per
-    // thread) and one of EPI_PARTS column ranges of the 256 columns
+    // thread) and one of EPI_PARTS column ranges of the kBN columns
     const uint32_t quad = warp & 3u;
     const uint32_t part = (warp - 2u) >> 2;
     uint32_t local = 0;
@@ -488,7 +504,7 @@ tc_score_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
       const uint32_t buf = local & 1u, tphase = (local >> 1) & 1u;
       // what does not depend on the accumulator is loaded before the wait
       const uint32_t row0 = a.row_begin + row_tile(t) * BM;
-      const uint32_t q0 = (t % ntiles) * BN;
+      const uint32_t q0 = (t % ntiles) * kBN;
       const uint32_t row = row0 + quad * 32 + lane;
       const bool in_range = row < a.row_end;
       const bool rvalid = in_range && row != 0 && a.present[row];
@@ -496,14 +512,20 @@ tc_score_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
       const float bi = rvalid ? a.row_bias[row] : 0.f;
       // per chunk of 32 queries of this warp's columns: lane j holds the
       // threshold (+inf past the last query) and the scale of query qb + j
-      constexpr uint32_t CH = BN / (32 * EPI_PARTS);
-      static_assert(CH * 32 * EPI_PARTS == BN, "whole chunks of 32 queries per epilogue warp");
+      constexpr uint32_t CH = kBN / (32 * EPI_PARTS);
+      static_assert(CH * 32 * EPI_PARTS == kBN, "whole chunks of 32 queries per epilogue warp");
       float thr_c[CH], qs_c[CH];
 #pragma unroll
       for (uint32_t i = 0; i < CH; i++) {
         const uint32_t qj = q0 + (part * CH + i) * 32 + lane;
         thr_c[i] = (!kDense && qj < a.nq) ? __ldg(a.thr + qj) : INFINITY;
         qs_c[i] = (kFp8 && qj < a.nq) ? __ldg(a.qscale + qj) : 1.f;
+      }
+      if constexpr (!kDense) {
+        __syncwarp();                            // the previous tile's thresholds are read
+#pragma unroll
+        for (uint32_t i = 0; i < CH; i++) thr_sh[warp - 2][i * 32 + lane] = thr_c[i];
+        __syncwarp();
       }
       uint32_t ok = 1;
       if (lane == 0) ok = mbar_wait(smem_u32(&bar_tfull[buf]), tphase, &abort_sh) ? 1u : 0u;
@@ -515,7 +537,7 @@ tc_score_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
       }
       tc_fence_after();
       // this warp's first TMEM column: lanes 32 * quad.., its column range
-      const uint32_t tcol = tmem + ((quad * 32u) << 16) + buf * BN + part * CH * 32;
+      const uint32_t tcol = tmem + ((quad * 32u) << 16) + buf * kBN + part * CH * 32;
       // rolled loops over the chunks keep the epilogue's code small (per-chunk
       // values shift down into index 0 of their arrays)
       if constexpr (kDense) {
@@ -553,25 +575,28 @@ tc_score_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
 #pragma unroll 1
         for (uint32_t i = 0; i < CH; i++) {
           const uint32_t qb = q0 + (part * CH + i) * 32;
-          const float thr = thr_c[0], qs = qs_c[0];
+          const float qs = qs_c[0];
 #pragma unroll
-          for (uint32_t c = 0; c + 1 < CH; c++) {
-            thr_c[c] = thr_c[c + 1];
-            qs_c[c] = qs_c[c + 1];
-          }
+          for (uint32_t c = 0; c + 1 < CH; c++) qs_c[c] = qs_c[c + 1];
           uint32_t v[32];
           tmem_ld32(tcol + i * 32, v);
           tmem_ld_wait(v);
           // passed: the queries of the chunk whose threshold this lane's row
           // passes (none past the last query: its threshold is +inf)
           uint32_t passed = 0;
+          const float4* thr4 = reinterpret_cast<const float4*>(&thr_sh[warp - 2][i * 32]);
 #pragma unroll
-          for (uint32_t j = 0; j < 32; j++) {
-            const float t = __shfl_sync(0xffffffffu, thr, j);
-            const float scj = kFp8 ? sc * __shfl_sync(0xffffffffu, qs, j) : sc;
-            const float s = fmaf(__uint_as_float(v[j]), scj, bi);
-            passed |= (rvalid && s > t) ? 1u << j : 0u;
+          for (uint32_t j = 0; j < 32; j += 4) {
+            const float4 t4 = thr4[j / 4];
+            const float t[4] = {t4.x, t4.y, t4.z, t4.w};
+#pragma unroll
+            for (uint32_t x = 0; x < 4; x++) {
+              const float scj = kFp8 ? sc * __shfl_sync(0xffffffffu, qs, j + x) : sc;
+              const float s = fmaf(__uint_as_float(v[j + x]), scj, bi);
+              passed |= s > t[x] ? 1u << (j + x) : 0u;
+            }
           }
+          if (!rvalid) passed = 0;
           uint32_t qany = __reduce_or_sync(0xffffffffu, passed);
           uint32_t base = 0;                     // lane j: first reserved slot of query qb + j
           if (__popc(qany) > kDeferQueries) {
@@ -673,130 +698,210 @@ tc_score_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
   }
 }
 
-// The k-th smallest (1-based, 1 <= k <= n) of n distinct 64-bit keys in shared
-// memory: up to eight 8-bit radix passes (warp 0 scans the 256-bin histogram),
-// ended early once the k-th key is the only key with the prefix found so far.
-__device__ unsigned long long block_select_u64(const unsigned long long* keys, uint32_t n, uint32_t k,
-                                               uint32_t* hist) {
-  __shared__ unsigned long long sh_prefix;
-  __shared__ uint32_t sh_need, sh_single;
-  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  unsigned long long prefix = 0, mask = 0;
-  uint32_t need = k;
-  for (int shift = 56; shift >= 0; shift -= 8) {
-    for (uint32_t i = threadIdx.x; i < 256; i += blockDim.x) hist[i] = 0;
-    __syncthreads();
-    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
-      const unsigned long long x = keys[i];
-      if ((x & mask) == prefix) atomicAdd(&hist[(uint32_t)(x >> shift) & 255u], 1u);
-    }
-    __syncthreads();
-    if (warp == 0) {
-      uint32_t c[8], sum = 0;
-#pragma unroll
-      for (int j = 0; j < 8; j++) {
-        c[j] = hist[lane * 8 + j];
-        sum += c[j];
-      }
-      uint32_t incl = sum;
-#pragma unroll
-      for (int off = 1; off < 32; off <<= 1) {
-        uint32_t y = __shfl_up_sync(0xffffffffu, incl, off);
-        if (lane >= (uint32_t)off) incl += y;
-      }
-      const uint32_t excl = incl - sum;
-      const unsigned here = __ballot_sync(0xffffffffu, excl < need && incl >= need);
-      if (lane == (uint32_t)(__ffs(here) - 1)) {
-        uint32_t acc = excl, j = 0;
-        for (j = 0; j < 7; j++) {
-          if (acc + c[j] >= need) break;
-          acc += c[j];
-        }
-        sh_prefix = prefix | ((unsigned long long)(lane * 8 + j) << shift);
-        sh_need = need - acc;
-        sh_single = c[j] == 1u ? 1u : 0u;
-      }
-    }
-    __syncthreads();
-    prefix = sh_prefix;
-    need = sh_need;
-    mask |= 255ull << shift;
-    const bool single = sh_single != 0u && shift > 0;
-    __syncthreads();
-    if (single) {
-      // one key has this prefix: it is the k-th
-      for (uint32_t i = threadIdx.x; i < n; i += blockDim.x)
-        if ((keys[i] & mask) == prefix) sh_prefix = keys[i];
-      __syncthreads();
-      const unsigned long long r = sh_prefix;
-      __syncthreads();
-      return r;
-    }
+// The k-th smallest (1-based, k <= the valid ones) of n distinct 64-bit keys key(0..n-1), by
+// the whole CTA of T threads: radix passes of 11 bits from the highest bit in which the keys
+// differ (scores share their leading bits), ended once a bin holds exactly the keys still
+// needed.  Returns a threshold: the keys up to it are the k smallest.  hist: 2048 words.
+// Bound by its passes' barriers and shared-memory atomics: with 8-bit digits from the top
+// byte, keys of one exponent met in one bin and a selection of 400 from 8,192 took 422 us for
+// 10,000 queries.
+// mn, mx: the smallest and largest valid key of those this thread has seen (together the
+// CTA's threads have seen all).
+template <int T, class Key>
+__device__ unsigned long long block_select_u64(Key key, uint32_t n, uint32_t k, unsigned long long mn,
+                                               unsigned long long mx, uint32_t* hist) {
+  constexpr uint32_t kBits = 11, kBins = 1u << kBits, kPer = kBins / T;
+  static_assert(kPer * T == kBins, "whole bins per thread");
+  __shared__ unsigned long long sh_min, sh_max, sh_thr;
+  __shared__ uint32_t sh_need, sh_done, sh_warp[T / 32];
+  const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if (tid == 0) {
+    sh_min = ~0ull;
+    sh_max = 0ull;
   }
-  return prefix;
+  for (int off = 16; off > 0; off >>= 1) {
+    const unsigned long long a = __shfl_xor_sync(0xffffffffu, mn, off), c = __shfl_xor_sync(0xffffffffu, mx, off);
+    mn = a < mn ? a : mn;
+    mx = c > mx ? c : mx;
+  }
+  __syncthreads();
+  if (lane == 0 && mn <= mx) {
+    atomicMin(&sh_min, mn);
+    atomicMax(&sh_max, mx);
+  }
+  __syncthreads();
+  const unsigned long long lo = sh_min, diff = lo ^ sh_max;
+  if (diff == 0) return lo;                        // one key
+  int top = 64 - __clzll((long long)diff);         // bits top.. are common
+  unsigned long long prefix = top == 64 ? 0ull : lo >> top << top;
+  uint32_t need = k;
+  while (true) {
+    const int shift = max(0, top - (int)kBits);
+    const uint32_t dmask = (1u << (top - shift)) - 1u;
+    const unsigned long long above = top == 64 ? 0ull : ~0ull << top;
+    for (uint32_t i = tid; i < kBins; i += T) hist[i] = 0;
+    __syncthreads();
+    for (uint32_t i = tid; i < n; i += T) {
+      const unsigned long long x = key(i);
+      if ((x & above) == prefix) atomicAdd(&hist[(uint32_t)(x >> shift) & dmask], 1u);
+    }
+    __syncthreads();
+    uint32_t c[kPer], sum = 0;
+#pragma unroll
+    for (uint32_t j = 0; j < kPer; j++) {
+      c[j] = hist[tid * kPer + j];
+      sum += c[j];
+    }
+    uint32_t incl = sum;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, incl, off);
+      if (lane >= (uint32_t)off) incl += y;
+    }
+    if (lane == 31) sh_warp[warp] = incl;
+    __syncthreads();
+    uint32_t before = 0;
+    for (uint32_t w = 0; w < warp; w++) before += sh_warp[w];
+    uint32_t acc = before + incl - sum;
+    if (acc < need && acc + sum >= need) {
+      uint32_t j = 0;
+      for (; j + 1 < kPer; j++) {
+        if (acc + c[j] >= need) break;
+        acc += c[j];
+      }
+      const unsigned long long p = prefix | ((unsigned long long)(tid * kPer + j) << shift);
+      const bool all = acc + c[j] == need;         // every key of the bin is wanted
+      sh_thr = all ? p | ((1ull << shift) - 1ull) : p;
+      sh_need = need - acc;
+      sh_done = all ? 1u : 0u;
+    }
+    __syncthreads();
+    prefix = sh_thr;
+    need = sh_need;
+    if (sh_done || shift == 0) return prefix;      // distinct keys: the last digit leaves one
+    top = shift;
+  }
 }
 
-// Per query: the C best keys of the dense part -> first candidates and threshold.
-__global__ void __launch_bounds__(512)
+// Per query: the C best keys of the dense part -> first candidates and threshold.  Keys are
+// made from the scores as they are read (L2 holds a query's few KB), so that four CTAs share
+// an SM.
+constexpr int kSelectThreads = 512;
+__global__ void __launch_bounds__(kSelectThreads)
 tc_first_select_kernel(const float* __restrict__ dense, uint32_t ld, uint32_t nrows, uint32_t C,
                        float* __restrict__ thr, unsigned long long* __restrict__ cand,
                        uint32_t* __restrict__ cand_count, uint32_t cap, uint32_t row_offset) {
   extern __shared__ __align__(16) unsigned char smem[];
-  unsigned long long* keys = reinterpret_cast<unsigned long long*>(smem);   // ld
-  __shared__ uint32_t hist[256];
-  __shared__ uint32_t sh_n, sh_m;
-  const uint32_t q = blockIdx.x;
-  if (threadIdx.x == 0) sh_n = sh_m = 0;
+  uint32_t* keys = reinterpret_cast<uint32_t*>(smem);                       // nrows score keys
+  __shared__ uint32_t hist[2048];
+  __shared__ uint32_t sh_n, sh_m, sh_worst;
+  const uint32_t q = blockIdx.x, lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) sh_n = sh_m = sh_worst = 0;
   __syncthreads();
   const float* S = dense + (size_t)q * ld;
-  for (uint32_t r = threadIdx.x; r < nrows; r += blockDim.x) {
+  uint32_t valid = 0, mn = 0xffffffffu, mx = 0;
+  for (uint32_t r = threadIdx.x; r < nrows; r += kSelectThreads) {
     const uint32_t key = score_key(S[r]);
-    if (key < kInvalidKey) keys[atomicAdd(&sh_n, 1u)] = ((unsigned long long)key << 32) | (r + row_offset);
+    keys[r] = key;
+    if (key < kInvalidKey) {
+      valid++;
+      mn = min(mn, key);
+      mx = max(mx, key);
+    }
   }
+  valid = __reduce_add_sync(0xffffffffu, valid);
+  if (lane == 0) atomicAdd(&sh_n, valid);
   __syncthreads();
   const uint32_t n = sh_n;
-  unsigned long long kth = ~0ull;
-  if (n > C) kth = block_select_u64(keys, n, C, hist);
+  auto key = [&](uint32_t r) { return ((unsigned long long)keys[r] << 32) | (r + row_offset); };
+  // valid keys are the smallest ones: with more than C of them the C-th is valid
+  unsigned long long kth = ((unsigned long long)kInvalidKey << 32) - 1ull;
+  // (any row id bounds the keys of the smallest and the largest score)
+  const bool any = mn <= mx;
+  if (n > C)
+    kth = block_select_u64<kSelectThreads>(key, nrows, C, any ? (unsigned long long)mn << 32 : ~0ull,
+                                           any ? ((unsigned long long)mx << 32) | 0xffffffffull : 0ull, hist);
   unsigned long long* out = cand + (size_t)q * cap;
-  for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
-    const unsigned long long x = keys[i];
-    if (x <= kth) out[atomicAdd(&sh_m, 1u)] = x;
+  uint32_t worst = 0;
+  for (uint32_t b = 0; b < nrows; b += kSelectThreads) {
+    const uint32_t r = b + threadIdx.x;
+    const unsigned long long x = r < nrows ? key(r) : ~0ull;
+    const uint32_t take = __ballot_sync(0xffffffffu, x <= kth);
+    if (take == 0) continue;
+    uint32_t at = 0;
+    if (lane == 0) at = atomicAdd(&sh_m, (uint32_t)__popc(take));
+    at = __shfl_sync(0xffffffffu, at, 0);
+    if (x <= kth) {
+      out[at + __popc(take & ((1u << lane) - 1u))] = x;
+      worst = max(worst, (uint32_t)(x >> 32));
+    }
   }
+  worst = __reduce_max_sync(0xffffffffu, worst);
+  if (lane == 0 && worst) atomicMax(&sh_worst, worst);
   __syncthreads();
   if (threadIdx.x == 0) {
     cand_count[q] = sh_m;
-    thr[q] = n > C ? key_score((uint32_t)(kth >> 32)) : -INFINITY;
+    thr[q] = n > C ? key_score(sh_worst) : -INFINITY;
   }
 }
 
 // Per query, between two parts of the filtered rows: the C best candidate keys
 // are kept (written back in place) and the threshold moves up to the C-th.  The
-// rows still to come have larger ids, so the strict filter stays exact.
-__global__ void __launch_bounds__(512)
+// rows still to come have larger ids, so the strict filter stays exact.  The first `held`
+// keys (at least C) are held in shared memory, the rest of a long list stays where it is.
+constexpr int kCompactThreads = 256;
+__global__ void __launch_bounds__(kCompactThreads)
 tc_compact_kernel(unsigned long long* __restrict__ cand, uint32_t* __restrict__ cand_count, uint32_t cap, uint32_t C,
-                  float* __restrict__ thr, uint32_t* __restrict__ status) {
+                  uint32_t held, float* __restrict__ thr, uint32_t* __restrict__ status,
+                  uint32_t* __restrict__ error) {
   extern __shared__ __align__(16) unsigned char smem[];
-  unsigned long long* keys = reinterpret_cast<unsigned long long*>(smem);   // cap
-  __shared__ uint32_t hist[256];
-  __shared__ uint32_t sh_m;
-  const uint32_t q = blockIdx.x;
+  unsigned long long* keys = reinterpret_cast<unsigned long long*>(smem);   // held
+  __shared__ uint32_t hist[2048];
+  __shared__ uint32_t sh_m, sh_worst;
+  const uint32_t q = blockIdx.x, lane = threadIdx.x & 31;
   uint32_t n = cand_count[q];
   if (n <= C) return;                                   // uniform over the CTA
   if (n > cap) {
-    if (threadIdx.x == 0) status[q] |= 1u;
+    if (threadIdx.x == 0) {
+      status[q] |= 1u;
+      atomicOr(error, kErrorOverflow);
+    }
     n = cap;
   }
   unsigned long long* list = cand + (size_t)q * cap;
-  for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) keys[i] = list[i];
-  if (threadIdx.x == 0) sh_m = 0;
+  unsigned long long mn = ~0ull, mx = 0ull;
+  for (uint32_t i = threadIdx.x; i < n; i += kCompactThreads) {
+    const unsigned long long x = list[i];
+    if (i < held) keys[i] = x;
+    mn = x < mn ? x : mn;
+    mx = x > mx ? x : mx;
+  }
+  if (threadIdx.x == 0) sh_m = sh_worst = 0;
   __syncthreads();
-  const unsigned long long kth = block_select_u64(keys, n, C, hist);
-  for (uint32_t i = threadIdx.x; i < n; i += blockDim.x)
-    if (keys[i] <= kth) list[atomicAdd(&sh_m, 1u)] = keys[i];
+  auto key = [&](uint32_t i) { return i < held ? keys[i] : list[i]; };
+  const unsigned long long kth = block_select_u64<kCompactThreads>(key, n, C, mn, mx, hist);
+  // the C keys land in the first C places, which are held: no key still to be read is there
+  uint32_t worst = 0;
+  for (uint32_t b = 0; b < n; b += kCompactThreads) {
+    const uint32_t i = b + threadIdx.x;
+    const unsigned long long x = i < n ? key(i) : ~0ull;
+    const bool take = x <= kth;
+    const uint32_t mask = __ballot_sync(0xffffffffu, take);
+    if (mask == 0) continue;
+    uint32_t at = 0;
+    if (lane == 0) at = atomicAdd(&sh_m, (uint32_t)__popc(mask));
+    at = __shfl_sync(0xffffffffu, at, 0);
+    if (take) {
+      list[at + __popc(mask & ((1u << lane) - 1u))] = x;
+      worst = max(worst, (uint32_t)(x >> 32));
+    }
+  }
+  worst = __reduce_max_sync(0xffffffffu, worst);
+  if (lane == 0 && worst) atomicMax(&sh_worst, worst);
   __syncthreads();
   if (threadIdx.x == 0) {
     cand_count[q] = C;
-    thr[q] = key_score((uint32_t)(kth >> 32));
+    thr[q] = key_score(sh_worst);
   }
 }
 
@@ -837,17 +942,17 @@ constexpr uint32_t kTieWindow = 64;     // largest tie window the FP64 check res
 // `size` are returned in those places (in fp32 (distance, id) order): the returned
 // set is then the FP64 ground truth's among the candidates.  A window wider than
 // kTieWindow entries keeps the fp32 result and sets status bit 4.
+constexpr int kFinalThreads = 256;
 template <Metric M, bool kTies>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(kFinalThreads)
 tc_final_kernel(DevGraph g, const uint4* __restrict__ queries, uint32_t q0, const unsigned long long* __restrict__ cand,
                 const uint32_t* __restrict__ cand_count, uint32_t cap, uint32_t C, uint32_t P, uint32_t size,
                 uint32_t group, ObjDist* __restrict__ out, uint32_t kmax, uint32_t* __restrict__ out_count,
-                uint32_t* __restrict__ status) {
+                uint32_t* __restrict__ status, uint32_t* __restrict__ error) {
   extern __shared__ __align__(16) unsigned char smem[];
   uint4* qv = reinterpret_cast<uint4*>(smem);                                        // row_chunks
-  unsigned long long* keys = reinterpret_cast<unsigned long long*>(qv + g.row_chunks);  // cap
-  unsigned long long* sel = keys + cap;                                               // P
-  __shared__ uint32_t hist[256];
+  unsigned long long* sel = reinterpret_cast<unsigned long long*>(qv + g.row_chunks);   // P
+  __shared__ uint32_t hist[2048];
   __shared__ uint32_t sh_m;
   const uint32_t qi = blockIdx.x, q = q0 + qi;
   const uint32_t rc = g.row_chunks;
@@ -855,43 +960,49 @@ tc_final_kernel(DevGraph g, const uint4* __restrict__ queries, uint32_t q0, cons
   uint32_t n = cand_count[qi];
   if (n > cap) n = cap;
   const unsigned long long* src = cand + (size_t)qi * cap;
-  for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) keys[i] = src[i];
   if (threadIdx.x == 0) sh_m = 0;
   __syncthreads();
   unsigned long long kth = ~0ull;
-  if (n > C) kth = block_select_u64(keys, n, C, hist);
-  for (uint32_t i = threadIdx.x; i < n; i += blockDim.x)
-    if (keys[i] <= kth) sel[atomicAdd(&sh_m, 1u)] = keys[i];
+  if (n > C) {
+    unsigned long long mn = ~0ull, mx = 0ull;
+    for (uint32_t i = threadIdx.x; i < n; i += kFinalThreads) {
+      const unsigned long long x = __ldg(src + i);
+      mn = x < mn ? x : mn;
+      mx = x > mx ? x : mx;
+    }
+    kth = block_select_u64<kFinalThreads>([&](uint32_t i) { return __ldg(src + i); }, n, C, mn, mx, hist);
+  }
+  for (uint32_t b = 0; b < n; b += kFinalThreads) {
+    const uint32_t i = b + threadIdx.x;
+    const unsigned long long x = i < n ? __ldg(src + i) : ~0ull;
+    const uint32_t mask = __ballot_sync(0xffffffffu, i < n && x <= kth);
+    if (mask == 0) continue;
+    uint32_t at = 0;
+    if ((threadIdx.x & 31) == 0) at = atomicAdd(&sh_m, (uint32_t)__popc(mask));
+    at = __shfl_sync(0xffffffffu, at, 0);
+    if (i < n && x <= kth) sel[at + __popc(mask & ((1u << (threadIdx.x & 31)) - 1u))] = x;
+  }
   __syncthreads();
   const uint32_t m = sh_m;
   for (uint32_t i = m + threadIdx.x; i < P; i += blockDim.x) sel[i] = ~0ull;
-  // exact distances: groups of `group` lanes per row, as the plain linear search
-  const int G = (int)group;
+  // exact distances with the plain linear search's lanes and order of summation, packed four
+  // lanes to a thread, two rows in flight each
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int gl = lane & (G - 1);
-  const uint32_t gpw = 32 / G, ngroups = blockDim.x / G;
-  // each group computes kRows rows at once (their loads in flight together);
-  // every row's lanes and summation order are those of group_distance
-  constexpr uint32_t kRows = 4;
-  for (uint32_t b = warp * gpw * kRows; b < m; b += ngroups * kRows) {
+  const int pw = packed_width((int)group);
+  const uint32_t step = kFinalThreads / (uint32_t)pw;
+  constexpr int kRows = Acc<ObjType::Float, M>::kUseF12 ? 1 : 2;
+  for (uint32_t b = (uint32_t)(warp * (32 / pw)); b < m; b += kRows * step) {
     uint32_t idx[kRows], row[kRows];
-    Acc<ObjType::Float, M> acc[kRows];
+    Acc<ObjType::Float, M> sum[kRows];
 #pragma unroll
     for (uint32_t r = 0; r < kRows; r++) {
-      idx[r] = b + r * gpw + (uint32_t)(lane / G);
+      idx[r] = b + r * step + (uint32_t)(lane / pw);
       row[r] = idx[r] < m ? (uint32_t)sel[idx[r]] : 0u;
     }
-    for (int c = gl; c < (int)rc; c += G) {
-      const uint4 qc = qv[c];
+    packed_sums<ObjType::Float, M, kRows>(qv, g.objects, row, (int)rc, lane & (pw - 1), (int)group, sum);
 #pragma unroll
-      for (uint32_t r = 0; r < kRows; r++) acc[r].add(qc, __ldg(g.objects + (size_t)row[r] * rc + c), c);
-    }
-#pragma unroll
-    for (uint32_t r = 0; r < kRows; r++) {
-      acc[r].reduce(G);
-      const float d = acc[r].finish();
-      if (idx[r] < m && gl == 0) sel[idx[r]] = pack_key(d, row[r]);
-    }
+    for (uint32_t r = 0; r < kRows; r++)
+      if (idx[r] < m && (lane & (pw - 1)) == 0) sel[idx[r]] = pack_key(sum[r].finish(), row[r]);
   }
   __syncthreads();
   // bitonic sort of P keys (P a power of two)
@@ -968,7 +1079,10 @@ tc_final_kernel(DevGraph g, const uint4* __restrict__ queries, uint32_t q0, cons
     out[(size_t)q * kmax + i] = ObjDist{key_id(sel[i]), key_dist(sel[i])};
   if (threadIdx.x == 0) {
     out_count[q] = kk;
-    if (status && cand_count[qi] > cap) status[q] |= 1u;
+    if (status && cand_count[qi] > cap) {
+      status[q] |= 1u;
+      atomicOr(error, kErrorOverflow);
+    }
   }
 }
 
@@ -1054,7 +1168,7 @@ __global__ void tc_queries_kernel(const float* __restrict__ rows, uint32_t dpad,
 }
 
 typedef void (*FinalFn)(DevGraph, const uint4*, uint32_t, const unsigned long long*, const uint32_t*, uint32_t,
-                        uint32_t, uint32_t, uint32_t, uint32_t, ObjDist*, uint32_t, uint32_t*, uint32_t*);
+                        uint32_t, uint32_t, uint32_t, uint32_t, ObjDist*, uint32_t, uint32_t*, uint32_t*, uint32_t*);
 
 template <bool kTies>
 FinalFn final_kernel_t(Metric m) {
@@ -1232,15 +1346,15 @@ void GraphEngine::ensure_tc_rows8() {
 
 namespace {
 
-template <bool kFp8, bool kPair>
+template <bool kFp8, bool kPair, uint32_t kBN>
 void launch_scores_t(const CUtensorMap& mapA, const CUtensorMap& mapB, const tc::ScoreArgs& a, bool dense,
                      cudaStream_t s, unsigned grid) {
-  auto fn = dense ? tc::tc_score_kernel<true, kFp8, kPair> : tc::tc_score_kernel<false, kFp8, kPair>;
+  auto fn = dense ? tc::tc_score_kernel<true, kFp8, kPair, kBN> : tc::tc_score_kernel<false, kFp8, kPair, kBN>;
   if constexpr (kPair) {
     // clusters of two CTAs (grid even)
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(tc::THREADS);
+    cfg.blockDim = dim3(tc::tc_threads(kBN));
     cfg.dynamicSmemBytes = tc::SMEM_BYTES;
     cfg.stream = s;
     cudaLaunchAttribute at[1];
@@ -1252,7 +1366,7 @@ void launch_scores_t(const CUtensorMap& mapA, const CUtensorMap& mapB, const tc:
     cfg.numAttrs = 1;
     TC_CUDA(cudaLaunchKernelEx(&cfg, fn, mapA, mapB, a));
   } else {
-    fn<<<grid, tc::THREADS, tc::SMEM_BYTES, s>>>(mapA, mapB, a);
+    fn<<<grid, tc::tc_threads(kBN), tc::SMEM_BYTES, s>>>(mapA, mapB, a);
   }
 }
 
@@ -1260,50 +1374,86 @@ void launch_scores_t(const CUtensorMap& mapA, const CUtensorMap& mapB, const tc:
 // (set before the launches, so that a launch sequence can be captured into a graph).
 void prepare_score_kernels() {
   {
-    const void* fns[] = {(const void*)tc::tc_score_kernel<true, false, false>,
-                         (const void*)tc::tc_score_kernel<false, false, false>,
-                         (const void*)tc::tc_score_kernel<true, true, false>,
-                         (const void*)tc::tc_score_kernel<false, true, false>,
-                         (const void*)tc::tc_score_kernel<true, false, true>,
-                         (const void*)tc::tc_score_kernel<false, false, true>,
-                         (const void*)tc::tc_score_kernel<true, true, true>,
-                         (const void*)tc::tc_score_kernel<false, true, true>};
+    const void* fns[] = {(const void*)tc::tc_score_kernel<true, false, false, tc::BN>,
+                         (const void*)tc::tc_score_kernel<false, false, false, tc::BN>,
+                         (const void*)tc::tc_score_kernel<true, true, false, tc::BN>,
+                         (const void*)tc::tc_score_kernel<false, true, false, tc::BN>,
+                         (const void*)tc::tc_score_kernel<true, false, true, tc::BN>,
+                         (const void*)tc::tc_score_kernel<false, false, true, tc::BN>,
+                         (const void*)tc::tc_score_kernel<true, true, true, tc::BN>,
+                         (const void*)tc::tc_score_kernel<false, true, true, tc::BN>,
+                         (const void*)tc::tc_score_kernel<true, false, false, tc::SMALL_BN>,
+                         (const void*)tc::tc_score_kernel<false, false, false, tc::SMALL_BN>,
+                         (const void*)tc::tc_score_kernel<true, true, false, tc::SMALL_BN>,
+                         (const void*)tc::tc_score_kernel<false, true, false, tc::SMALL_BN>};
     for (const void* f : fns)
       TC_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc::SMEM_BYTES));
   }
 }
 
-// mapB: the query tiles (256-row boxes); mapBh: the same with 128-row boxes, for
-// the two-CTA (pair) kernel, which runs when `pair` is set.
+// queries per tile of the single-CTA form for nq queries
+uint32_t tile_queries(size_t nq) { return nq <= tc::SMALL_BN ? tc::SMALL_BN : tc::BN; }
+
+// mapB: the query tiles (boxes of tile_queries(a.nq) rows, or 256 with `pair`); mapBh: the
+// same with 128-row boxes, for the two-CTA (pair) kernel, which runs when it is given.
 void launch_scores(const TcState& st, const CUtensorMap& mapB, const CUtensorMap* mapBh, tc::ScoreArgs a, bool dense,
                    cudaStream_t s, int sms, bool fp8 = false) {
+  const bool pair = mapBh != nullptr;
+  const uint32_t bn = pair ? tc::BN : tile_queries(a.nq);
   const uint32_t mtiles = (a.row_end - a.row_begin + tc::BM - 1) / tc::BM;
-  const uint32_t ntiles = (a.nq + tc::BN - 1) / tc::BN;
+  const uint32_t ntiles = (a.nq + bn - 1) / bn;
   const uint32_t tiles = mtiles * ntiles;
   if (tiles == 0) return;
-  const bool pair = mapBh != nullptr;
   const unsigned grid = pair ? 2u * (unsigned)std::min<uint32_t>((mtiles + 1) / 2 * ntiles, (uint32_t)sms / 2)
                              : (unsigned)std::min<uint32_t>(tiles, (uint32_t)sms);
   if (fp8) {
     a.row_scale = st.scale8;
     a.kblocks = st.kpad8 / 128;
-    if (pair) launch_scores_t<true, true>(st.mapA8, *mapBh, a, dense, s, grid);
-    else launch_scores_t<true, false>(st.mapA8, mapB, a, dense, s, grid);
+    if (pair) launch_scores_t<true, true, tc::BN>(st.mapA8, *mapBh, a, dense, s, grid);
+    else if (bn == tc::BN) launch_scores_t<true, false, tc::BN>(st.mapA8, mapB, a, dense, s, grid);
+    else launch_scores_t<true, false, tc::SMALL_BN>(st.mapA8, mapB, a, dense, s, grid);
   } else {
-    if (pair) launch_scores_t<false, true>(st.mapA, *mapBh, a, dense, s, grid);
-    else launch_scores_t<false, false>(st.mapA, mapB, a, dense, s, grid);
+    if (pair) launch_scores_t<false, true, tc::BN>(st.mapA, *mapBh, a, dense, s, grid);
+    else if (bn == tc::BN) launch_scores_t<false, false, tc::BN>(st.mapA, mapB, a, dense, s, grid);
+    else launch_scores_t<false, false, tc::SMALL_BN>(st.mapA, mapB, a, dense, s, grid);
   }
   TC_CUDA(cudaGetLastError());
 }
 
-void check_error(const TcState& st, cudaStream_t s) {
+// Growth of the filtered parts: a part has R times the rows seen before it, and then about
+// C x R entries per query beat the threshold of those rows.  Measured at 10,000 queries and
+// C = 400: an appended entry costs the launch about 27 ps, a key of the compaction (C of them
+// and the new ones) 13 ps, a part some 12 us besides (launch, first and last wave); R is the
+// one with the least sum over the log(rows) / log(1 + R) parts: 1 there (13.5 ms of score and
+// compaction launches, 13.7 ms with R = 2), 16 for 33 queries over 1M rows (390 us of score
+// launches in 8 parts, 280 us in 3).  A quarter of the list's capacity is not exceeded on rows
+// in no particular order; a list that overflows all the same (rows sorted by nearness) has
+// the whole search done again with R = 1, as searches inside a caller's capture always are.
+uint32_t part_growth(size_t nq, size_t C, uint32_t cap) {
+  uint32_t best = 1;
+  double least = 0.0;
+  for (uint32_t R : {1u, 2u, 3u, 4u, 6u, 8u, 12u, 16u}) {
+    if (R > 1 && C * R * 4 > cap) break;
+    const double us = ((double)nq * C * (40.0 * R + 13.0) * 1e-6 + 12.0) / std::log2(1.0 + R);
+    if (R == 1 || us < least) {
+      least = us;
+      best = R;
+    }
+  }
+  return best;
+}
+
+// Waits for the stream; throws when a pipeline wait ran out; true when a candidate list
+// overflowed.
+bool check_error(const TcState& st, cudaStream_t s) {
   uint32_t err = 0;
   TC_CUDA(cudaMemcpyAsync(&err, st.error, 4, cudaMemcpyDeviceToHost, s));
   TC_CUDA(cudaStreamSynchronize(s));
-  if (err) {
-    TC_CUDA(cudaMemsetAsync(st.error, 0, 4, s));
+  if (err) TC_CUDA(cudaMemsetAsync(st.error, 0, 4, s));
+  if (err & ~tc::kErrorOverflow) {
     throw std::runtime_error("tensor-core score kernel: a pipeline wait ran out (code " + std::to_string(err) + ")");
   }
+  return err != 0;
 }
 
 }  // namespace
@@ -1319,12 +1469,13 @@ void GraphEngine::tc_scores_device(const uint4* d_rows, size_t nq, float* d_scor
   int sms = 0;
   TC_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device_));
   __nv_bfloat16* qb = nullptr;
-  const size_t nq_pad = (nq + tc::BN - 1) / tc::BN * tc::BN;
+  const uint32_t bn = tile_queries(nq);
+  const size_t nq_pad = (nq + bn - 1) / bn * bn;
   TC_CUDA(cudaMallocAsync(&qb, nq_pad * st.kpad * 2, stream));
   tc::tc_queries_kernel<<<1024, 256, 0, stream>>>(reinterpret_cast<const float*>(d_rows), host_.dpad, (uint32_t)nq,
                                                   (uint32_t)nq_pad, st.kpad, qb);
   TC_CUDA(cudaGetLastError());
-  CUtensorMap mapB = tc::make_map(qb, nq_pad, st.kpad, tc::BN);
+  CUtensorMap mapB = tc::make_map(qb, nq_pad, st.kpad, bn);
   tc::ScoreArgs a{};
   a.row_begin = 0;
   a.row_end = (uint32_t)host_.nrows;
@@ -1407,29 +1558,32 @@ void GraphEngine::linear_search_tc_device(const uint4* d_rows, size_t nq, size_t
   const uint32_t rc = dev_.row_chunks;
   uint32_t group = 1;
   while (group < rc && group < 32) group <<= 1;
-  const size_t fin_smem = (size_t)rc * 16 + (size_t)cap * 8 + (size_t)P * 8;
+  const size_t fin_smem = (size_t)rc * 16 + (size_t)P * 8;
+  const uint32_t held = C <= 2048 ? 2048u : cap;           // keys a compaction holds in shared memory
   TC_CUDA(cudaFuncSetAttribute((const void*)fin, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fin_smem));
   TC_CUDA(cudaFuncSetAttribute((const void*)tc::tc_first_select_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)(first * 8)));
+                               (int)(first * 4)));
   TC_CUDA(cudaFuncSetAttribute((const void*)tc::tc_compact_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)(cap * 8)));
+                               (int)(held * 8)));
   prepare_score_kernels();
-  // the launch sequence (timing: phase events between its parts)
-  auto enqueue = [&](bool timing) {
+  const uint32_t growth = part_growth(nq, C, cap);
+  // the launch sequence (timing: phase events between its parts; R: growth of the parts)
+  auto enqueue = [&](bool timing, uint32_t R) {
   TC_CUDA(cudaMemsetAsync(d_status, 0, nq * 4, stream));
   for (size_t q0 = 0; q0 < nq; q0 += qbmax) {
     const uint32_t nb = (uint32_t)std::min(qbmax, nq - q0);
-    const uint32_t nbpad = (nb + tc::BN - 1) / tc::BN * tc::BN;
+    const uint32_t bn = pair ? tc::BN : tile_queries(nb);
+    const uint32_t nbpad = (nb + bn - 1) / bn * bn;
     if (timing) TC_CUDA(cudaEventRecord(st.ev[0], stream));
     const float* qrows = reinterpret_cast<const float*>(d_rows) + q0 * host_.dpad;
     CUtensorMap mapB, mapBh;
     if (fp8) {
       tc::tc_queries8_kernel<<<1024, 256, 0, stream>>>(qrows, host_.dpad, nb, nbpad, st.kpad8, qbuf8, qscale);
-      mapB = tc::make_map8(qbuf8, nbpad, st.kpad8, tc::BN);
+      mapB = tc::make_map8(qbuf8, nbpad, st.kpad8, bn);
       if (pair) mapBh = tc::make_map8(qbuf8, nbpad, st.kpad8, tc::BN / 2);
     } else {
       tc::tc_queries_kernel<<<1024, 256, 0, stream>>>(qrows, host_.dpad, nb, nbpad, st.kpad, qbuf);
-      mapB = tc::make_map(qbuf, nbpad, st.kpad, tc::BN);
+      mapB = tc::make_map(qbuf, nbpad, st.kpad, bn);
       if (pair) mapBh = tc::make_map(qbuf, nbpad, st.kpad, tc::BN / 2);
     }
     const CUtensorMap* half = pair ? &mapBh : nullptr;
@@ -1448,12 +1602,12 @@ void GraphEngine::linear_search_tc_device(const uint4* d_rows, size_t nq, size_t
     a.dense = dense;
     a.dense_ld = (uint32_t)first;
     launch_scores(st, mapB, half, a, true, stream, sms, fp8);
-    tc::tc_first_select_kernel<<<nb, 512, first * 8, stream>>>(dense, (uint32_t)first, r0 - rb, (uint32_t)C, thr,
+    tc::tc_first_select_kernel<<<nb, tc::kSelectThreads, first * 4, stream>>>(dense, (uint32_t)first, r0 - rb, (uint32_t)C, thr,
                                                                cand, ccount, cap, rb);
     TC_CUDA(cudaGetLastError());
     launches_ += 3;
     if (timing) TC_CUDA(cudaEventRecord(st.ev[1], stream));
-    // filtered rest, in parts that double in size; between two parts the
+    // filtered rest, in parts R times as large as the rows before them; between two parts the
     // candidate lists are cut back to C and the thresholds move up
     a.dense = nullptr;
     a.thr = thr;
@@ -1467,8 +1621,9 @@ void GraphEngine::linear_search_tc_device(const uint4* d_rows, size_t nq, size_t
     // most low ids removed); the presence flags are the same for every query.
     size_t valid = 0;
     for (uint32_t i = std::max<uint32_t>(rb, 1); i < r0; i++) valid += host_.present[i] ? 1 : 0;
-    for (uint32_t row = r0, part = std::max<uint32_t>(r0 - rb, tc::BM); row < nrows; part *= 2) {
-      uint32_t end = (uint32_t)std::min<uint64_t>(nrows, (uint64_t)row + part);
+    uint64_t part = (uint64_t)R * std::max<uint32_t>(r0 - rb, tc::BM);
+    for (uint32_t row = r0; row < nrows; part *= 1 + R) {
+      uint32_t end = (uint32_t)std::min<uint64_t>(nrows, (row + part) / tc::BM * tc::BM);
       if (valid < C) {
         const size_t room = cap - valid;          // >= 3 C and >= 6144: cap >= max(8192, 4 C), C <= 2048 there
         size_t v = 0;
@@ -1487,15 +1642,17 @@ void GraphEngine::linear_search_tc_device(const uint4* d_rows, size_t nq, size_t
       launch_scores(st, mapB, half, a, false, stream, sms, fp8);
       launches_++;
       if (end < nrows) {
-        tc::tc_compact_kernel<<<nb, 512, cap * 8, stream>>>(cand, ccount, cap, (uint32_t)C, thr, d_status + q0);
+        tc::tc_compact_kernel<<<nb, tc::kCompactThreads, held * 8, stream>>>(cand, ccount, cap, (uint32_t)C, held, thr,
+                                                                             d_status + q0,
+                                                            st.error);
         TC_CUDA(cudaGetLastError());
         launches_++;
       }
       row = end;
     }
     if (timing) TC_CUDA(cudaEventRecord(st.ev[2], stream));
-    fin<<<nb, 256, fin_smem, stream>>>(dev_, d_rows, (uint32_t)q0, cand, ccount, cap, (uint32_t)C, P,
-                                       (uint32_t)size, group, d_out, (uint32_t)kmax, d_counts, d_status);
+    fin<<<nb, tc::kFinalThreads, fin_smem, stream>>>(dev_, d_rows, (uint32_t)q0, cand, ccount, cap, (uint32_t)C, P,
+                                       (uint32_t)size, group, d_out, (uint32_t)kmax, d_counts, d_status, st.error);
     TC_CUDA(cudaGetLastError());
     if (timing) TC_CUDA(cudaEventRecord(st.ev[3], stream));
     launches_++;
@@ -1505,9 +1662,15 @@ void GraphEngine::linear_search_tc_device(const uint4* d_rows, size_t nq, size_t
   TC_CUDA(cudaStreamIsCapturing(stream, &capture));
   if (!tc_graphs_ || capture != cudaStreamCaptureStatusNone) {
     // launched directly (also into a capture the caller runs on this stream)
-    enqueue(capture == cudaStreamCaptureStatusNone);
-    if (capture != cudaStreamCaptureStatusNone) return;
-    check_error(st, stream);
+    if (capture != cudaStreamCaptureStatusNone) {
+      enqueue(false, 1);
+      return;
+    }
+    enqueue(true, growth);
+    if (check_error(st, stream) && growth > 1) {
+      enqueue(true, 1);
+      check_error(st, stream);
+    }
     for (int i = 0; i < 3; i++) TC_CUDA(cudaEventElapsedTime(&tc_->phase_ms[i], st.ev[i], st.ev[i + 1]));
     return;
   }
@@ -1531,7 +1694,7 @@ void GraphEngine::linear_search_tc_device(const uint4* d_rows, size_t nq, size_t
     TC_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
     cudaGraph_t graph = nullptr;
     try {
-      enqueue(false);
+      enqueue(false, growth);
     } catch (...) {
       cudaStreamEndCapture(stream, &graph);
       if (graph) cudaGraphDestroy(graph);
@@ -1550,7 +1713,11 @@ void GraphEngine::linear_search_tc_device(const uint4* d_rows, size_t nq, size_t
   TC_CUDA(cudaGraphLaunch(g->exec, stream));
   TC_CUDA(cudaEventRecord(st.ev[3], stream));
   launches_ += g->launches;
-  check_error(st, stream);
+  if (check_error(st, stream) && growth > 1) {
+    enqueue(false, 1);
+    TC_CUDA(cudaEventRecord(st.ev[3], stream));
+    check_error(st, stream);
+  }
   // one replay: its whole time is reported as the middle phase
   float total = 0.f;
   TC_CUDA(cudaEventElapsedTime(&total, st.ev[0], st.ev[3]));

@@ -1,0 +1,71 @@
+"""Tensor-core exhaustive search: query tiles of 64 and 256, growing parts, and the second
+pass after a candidate list overflowed, against the plain exhaustive search."""
+import numpy as np
+import pytest
+
+from test_gpu_linear_select import _index
+
+pytestmark = pytest.mark.gpu
+
+
+def _plain(ix, q, k):
+    r = [ix.linear_search(v, k=k) for v in q]
+    return (np.array([[o.id for o in x] for x in r], np.uint32),
+            np.array([[o.distance for o in x] for x in r], np.float32))
+
+
+@pytest.mark.parametrize("dim", [3, 64, 65, 200])
+@pytest.mark.parametrize("n", [100, 8193, 70_001])
+def test_tile_widths_and_parts(tmp_path, n, dim):
+    rng = np.random.default_rng(n + dim)
+    x = rng.integers(0, 100, (n, dim)).astype(np.float32)       # whole numbers: bf16 scores are exact
+    q = rng.integers(0, 100, (260, dim)).astype(np.float32)
+    k = 10
+    with _index(tmp_path, x) as ix:
+        ids, ds, cnt, st = ix.linear_search_tc(q, k=k, candidates=64)
+        assert (st == 0).all()
+        pi, pd = _plain(ix, q[:20], k)
+        assert np.array_equal(ids[:20], pi) and np.array_equal(ds[:20], pd)
+        for nq in (1, 63, 64, 65, 256, 257):                    # one tile of 64, of 256, two
+            for fp8 in ("bf16", "fp8"):
+                a = ix.linear_search_tc(q[:nq], k=k, candidates=64 if fp8 == "bf16" else 2000 if n > 2000 else 64,
+                                        precision=fp8)
+                if fp8 == "bf16":
+                    assert np.array_equal(a[0], ids[:nq]) and np.array_equal(a[1], ds[:nq]), nq
+                elif nq <= 64:
+                    b = ix.linear_search_tc(np.concatenate([q[:nq]] * 70)[:65 * nq], k=k, precision=fp8,
+                                            candidates=2000 if n > 2000 else 64)
+                    assert np.array_equal(a[0], b[0][:nq]) and np.array_equal(a[1], b[1][:nq]), nq
+        s64, s256 = ix.tc_scores(q[:64]), ix.tc_scores(q)
+        assert np.array_equal(s64, s256[:64])
+
+
+def test_rows_sorted_by_nearness_are_searched_again(tmp_path):
+    """Each doubling part opens with 5,000 rows nearer than all before: a list holds one
+    part's, but not those of a part sixteen times the rows before it."""
+    n = 150_000
+    rng = np.random.default_rng(3)
+    x = rng.integers(90, 100, (n, 4)).astype(np.float32)
+    row, near = 8192 - 1, 80                                     # objects have ids from 1
+    while row < n:
+        x[row:row + 5000] = rng.integers(near - 10, near, (min(5000, n - row), 4))
+        row, near = 2 * (row + 1) - 1, near - 15
+    q = rng.integers(0, 3, (40, 4)).astype(np.float32)
+    with _index(tmp_path, x) as ix:
+        pi, pd = _plain(ix, q, 10)
+        for graphs in (False, True):
+            ix.set_tc_graphs(graphs)
+            for _ in range(2):
+                ids, ds, cnt, st = ix.linear_search_tc(q, k=10, candidates=64)
+                assert (st == 0).all() and (cnt == 10).all()
+                assert np.array_equal(ids, pi) and np.array_equal(ds, pd)
+
+
+def test_a_part_beyond_the_list_still_reports_overflow(tmp_path):
+    """Rows that come nearer one by one overflow any schedule: status bit 1, as before."""
+    n = 120_000
+    x = np.zeros((n, 2), np.float32)
+    x[:, 0] = np.arange(n, 0, -1) // 2
+    with _index(tmp_path, x) as ix:
+        ids, ds, cnt, st = ix.linear_search_tc(np.zeros((3, 2), np.float32), k=10, candidates=64)
+        assert (st & 1 != 0).all()
