@@ -1685,7 +1685,7 @@ GraphEngine::QbgScratch& GraphEngine::qbg_slot(size_t slot, size_t grid, cudaStr
   NGT_CUDA(cudaMemsetAsync(q.bitmaps, 0, grid * words * 4, stream));     // the kernels leave them clear
   NGT_CUDA(cudaMalloc(&q.exact_ovf, grid * 2 * (size_t)kOverflowCapacity * 8));
   NGT_CUDA(cudaMalloc(&q.qbg_ovf, grid * 4 * qocap * 8));
-  NGT_CUDA(cudaMalloc(&q.blob_dist, grid * (size_t)blob_cap_ * 4));
+  NGT_CUDA(cudaMalloc(&q.blob_dist, grid * (size_t)qbg_scan_dist_cap(blob_cap_) * 4));
   NGT_CUDA(cudaStreamSynchronize(stream));
   q.grid = grid;
   return q;
@@ -1818,7 +1818,8 @@ void GraphEngine::qbg_search_device(const uint4* d_rows, size_t nq, const QBGArg
   }
   QBGParams* d_params = nullptr;
   uint32_t* d_seeds = nullptr;
-  NGT_CUDA(dev_alloc(&d_params, nq * sizeof(QBGParams), stream));
+  // the scan's own work counter lies behind the parameters
+  NGT_CUDA(dev_alloc(&d_params, nq * sizeof(QBGParams) + 4, stream));
   NGT_CUDA(dev_alloc(&d_seeds, seeds.size() * 4, stream));
   NGT_CUDA(cudaMemcpyAsync(d_params, params.data(), nq * sizeof(QBGParams), cudaMemcpyHostToDevice, stream));
   NGT_CUDA(cudaMemcpyAsync(d_seeds, seeds.data(), seeds.size() * 4, cudaMemcpyHostToDevice, stream));
@@ -1831,7 +1832,7 @@ void GraphEngine::qbg_search_device(const uint4* d_rows, size_t nq, const QBGArg
       d_blob_dist_ = nullptr;
       size_t g2 = std::max(grid, qbg_grid_);
       NGT_CUDA(cudaMalloc(&d_qbg_ovf_, g2 * 4 * (size_t)std::max<uint32_t>(ocap, 1) * 8));
-      NGT_CUDA(cudaMalloc(&d_blob_dist_, g2 * (size_t)blob_cap_ * 4));
+      NGT_CUDA(cudaMalloc(&d_blob_dist_, g2 * (size_t)qbg_scan_dist_cap(blob_cap_) * 4));
       qbg_grid_ = g2;
       qbg_ocap_ = ocap;
     }
@@ -1859,9 +1860,15 @@ void GraphEngine::qbg_search_device(const uint4* d_rows, size_t nq, const QBGArg
       grid = std::min(grid, q.grid);
       bdist = q.blob_dist;
     }
+    uint32_t* work = nullptr;
+    if (grid < nq) {
+      work = reinterpret_cast<uint32_t*>(d_params + nq);
+      NGT_CUDA(cudaMemsetAsync(work, 0, 4, stream));
+    }
     fn<<<(unsigned)grid, kExactThreads, smem, stream>>>(dqb_, d_blob_sid_, d_rows, dev_.row_chunks, (uint32_t)nq,
                                                          d_params, d_blobs, d_bcounts, (uint32_t)max_probes, d_sout,
-                                                         d_scount, d_stats, bdist, blob_cap_, max_size);
+                                                         d_scount, d_stats, bdist, qbg_scan_dist_cap(blob_cap_),
+                                                         max_size, work);
     NGT_CUDA(cudaGetLastError());
     launches_++;
     NGT_CUDA(cudaFreeAsync(d_blobs, stream));
