@@ -181,6 +181,35 @@ struct WideDot {
   }
 };
 
+// The KR sums over SG lanes of partial sums v (a group's lanes lie side by side; KR and SG
+// powers of two), the rows spread over the lanes: each exchange with the lane `off` away
+// halves the rows a lane still adds up, then the rest of the lanes are added to all.  A lane
+// ends with the sums of rows first .. in v[0 ..] (max(KR / SG, 1) of them); the lanes without
+// one of their own get first = 2^31 - 1.  The pairs added are a butterfly's.
+template <uint32_t KR, class Add>
+__device__ __forceinline__ uint32_t group_sums(uint32_t (&v)[KR], int SG, int lane, Add add) {
+  uint32_t first = 0;
+  int off = SG >> 1;
+#pragma unroll
+  for (uint32_t h = KR / 2; h > 0; h >>= 1) {
+    if (off > 0) {
+      const bool up = (lane & off) != 0;
+#pragma unroll
+      for (uint32_t i = 0; i < h; i++) {
+        const uint32_t send = up ? v[i] : v[i + h], keep = up ? v[i + h] : v[i];
+        v[i] = add(keep, __shfl_xor_sync(0xffffffffu, send, off));
+      }
+      if (up) first += h;
+      off >>= 1;
+    }
+  }
+  if (off > 0) {
+    if (lane & (2 * off - 1)) first = 0x7fffffffu;
+    for (; off > 0; off >>= 1) v[0] = add(v[0], __shfl_xor_sync(0xffffffffu, v[0], off));
+  }
+  return first;
+}
+
 // The m <= T unique keys in[0..m) sorted to out by their ranks, several threads per key
 // where the CTA has them to spare.
 template <int T>
@@ -202,7 +231,8 @@ __device__ __forceinline__ void rank_sort_keys(const unsigned long long* in, uns
 // the integer dot products, 0.55 issued per cycle and scheduler.  Measured on 1M x 128,
 // 8-bit rows, k = 10, epsilon 0.08, 10,000 queries, 128 threads: 15.35 ms with a shared-memory
 // row stage (two barriers per 64 rows); rows loaded into registers 15.1 ms; dot products
-// 14.2 ms.  152 queries: 2.0 ms with 128 threads, 1.1 ms with 512 and the visited bitmap in
+// 14.2 ms; one body for every number of rows, sums spread over the lanes 12.55 ms (0.41
+// issued; stalls per issue on instruction fetches 2.8 -> 0.4).  152 queries: 2.0 ms with 128 threads, 1.1 ms with 512 and the visited bitmap in
 // shared memory.  200k x 100 cosine, 1,500 queries from host buffers: 1.80 -> 1.2 ms (packed
 // lanes, three CTAs per SM instead of two).  Not kept: prefetching a step's rows into L2
 // when they are gathered (5 % slower), 1,024 threads (8 % slower than 512).
@@ -255,8 +285,11 @@ graph_search_wide_kernel(DevGraph g, const uint4* __restrict__ srows, const uint
       atomicMin(&s.spill_min, key);
     }
   };
-  // scores nid[0..cnt): every lane group loads the chunks of several rows before it adds
-  // any up.  Lanes, chunks and the order of summation are the same for every number of rows.
+  // scores nid[0..cnt): every lane group loads the chunks of several rows before it adds any
+  // up.  Lanes, chunks and the order of summation are the same for every number of rows.
+  // One body for every number of rows and one call of it in the kernel: with bodies for 8, 4,
+  // 2 and 1 rows, once for the seeds and once for the steps, a sixth of the warps' time went
+  // on instruction fetches, and a step's last rows took up to three round trips.
   auto score = [&](uint32_t cnt, const Limits& w) {
     const uint32_t gpb = (uint32_t)T / SG;
     const uint32_t gi = (uint32_t)(tid / SG);
@@ -265,37 +298,43 @@ graph_search_wide_kernel(DevGraph g, const uint4* __restrict__ srows, const uint
       // the query chunks this lane reads (c = sgl + j * SG), negated and unpacked once; the
       // host sets sgroup so that a lane reads at most two chunks (one for 8-bit rows)
       float2 nqc[kQC][Dot::NQ];
+      auto prepare = [&]() {
 #pragma unroll
-      for (int j = 0; j < kQC; j++) {
-        const uint32_t c = (uint32_t)sgl + (uint32_t)(j * SG);
-        if (c < sc) Dot::prepare(qs, c, nqc[j]);
-        else Dot::zero(nqc[j]);
-      }
+        for (int j = 0; j < kQC; j++) {
+          const uint32_t c = (uint32_t)sgl + (uint32_t)(j * SG);
+          if (c < sc) Dot::prepare(qs, c, nqc[j]);
+          else Dot::zero(nqc[j]);
+        }
+      };
+      if (!Dot::kSq8) prepare();                 // 8-bit rows: with each batch, the registers are needed
       const bool dots = Dot::kSq8 && s.fraction == 0;
       const uint4 qc = dots && (uint32_t)sgl < sc ? reinterpret_cast<const uint4*>(qcode)[sgl] : make_uint4(0, 0, 0, 0);
-      auto rows_at_once = [&](auto kr_tag, uint32_t b) {
-        constexpr int KR = decltype(kr_tag)::value;
+      constexpr uint32_t KR = Dot::kSq8 ? 8 : 4;
+      const uint32_t step = min(cfg.score_rows, KR);
+      for (uint32_t b = 0; b < cnt; b += step * gpb) {         // uniform over the CTA
+        const uint32_t nu = min(step, (cnt - b + gpb - 1) / gpb);
         uint4 x[KR][kQC];
-        uint32_t id[KR];
 #pragma unroll
-        for (int u = 0; u < KR; u++) {
-          const uint32_t i = b + (uint32_t)u * gpb + gi;
-          id[u] = i < cnt ? nid[i] : 0u;
+        for (uint32_t u = 0; u < KR; u++) {
+          if (u < nu) {
+            const uint32_t i = b + u * gpb + gi;
+            const uint32_t id = i < cnt ? nid[i] : 0u;
 #pragma unroll
-          for (int j = 0; j < kQC; j++) {
-            const uint32_t c = (uint32_t)sgl + (uint32_t)(j * SG);
-            x[u][j] = c < sc ? load_row_chunk(srows + (size_t)id[u] * sc + c, pol_stream) : make_uint4(0, 0, 0, 0);
+            for (int j = 0; j < kQC; j++) {
+              const uint32_t c = (uint32_t)sgl + (uint32_t)(j * SG);
+              x[u][j] = c < sc ? load_row_chunk(srows + (size_t)id * sc + c, pol_stream) : make_uint4(0, 0, 0, 0);
+            }
           }
         }
-        float v[KR];
-        if constexpr (Dot::kSq8) {
-          if (dots) {
-            // sum (c - q)^2 = sum c c - 2 sum c q + sum q q over whole codes, exact in 32 bits;
-            // times 2^16 it is the sum of the squared 1/256 steps that the float form adds up
-            // (exact there too, below 2^24 steps of one)
-            int t[KR];
+        uint32_t sum[KR];                                      // a lane's part of each row's sum, as bits
+        uint32_t first;                                        // the first of the rows whose sum it holds then
+        if (Dot::kSq8 && dots) {
+          // sum (c - q)^2 = sum c c - 2 sum c q + sum q q over whole codes, exact in 32 bits;
+          // times 2^16 it is the sum of the squared 1/256 steps that the float form adds up
+          // (exact there too, below 2^24 steps of one)
 #pragma unroll
-            for (int u = 0; u < KR; u++) {
+          for (uint32_t u = 0; u < KR; u++) {
+            if (u < nu) {
               const uint32_t xw[4] = {x[u][0].x, x[u][0].y, x[u][0].z, x[u][0].w};
               const uint32_t qw[4] = {qc.x, qc.y, qc.z, qc.w};
               uint32_t cc = 0, cq = 0;
@@ -304,63 +343,42 @@ graph_search_wide_kernel(DevGraph g, const uint4* __restrict__ srows, const uint
                 cc = __dp4a(xw[i], xw[i], cc);
                 cq = __dp4a(xw[i], qw[i], cq);
               }
-              t[u] = (int)(cc - 2u * cq);
+              sum[u] = cc - 2u * cq;
+            } else {
+              sum[u] = 0u;
             }
-#pragma unroll
-            for (int off = 16; off > 0; off >>= 1)
-              if (off < SG) {
-#pragma unroll
-                for (int u = 0; u < KR; u++) t[u] += __shfl_xor_sync(0xffffffffu, t[u], off);
-              }
-#pragma unroll
-            for (int u = 0; u < KR; u++) {
-              const uint32_t i = b + (uint32_t)u * gpb + gi;
-              const float vu = (float)(t[u] + (int)s.qnorm) * 65536.f;
-              if (i < cnt && sgl == 0 && !(vu > w.far)) place(sqrtf(vu) * cfg.sq_out, id[u], w);
-            }
-            return;
           }
-        }
-#pragma unroll
-        for (int u = 0; u < KR; u++) {
-          float2 acc[kQC];
-#pragma unroll
-          for (int j = 0; j < kQC; j++) {
-            acc[j] = make_float2(0.f, 0.f);
-            if ((uint32_t)sgl + (uint32_t)(j * SG) < sc) acc[j] = Dot::add(acc[j], nqc[j], x[u][j]);
-          }
-          float t = acc[0].x + acc[0].y;
-#pragma unroll
-          for (int j = 1; j < kQC; j++) t += acc[j].x + acc[j].y;
-          v[u] = t;
-        }
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1)
-          if (off < SG) {
-#pragma unroll
-            for (int u = 0; u < KR; u++) v[u] += __shfl_xor_sync(0xffffffffu, v[u], off);
-          }
-#pragma unroll
-        for (int u = 0; u < KR; u++) {
-          const uint32_t i = b + (uint32_t)u * gpb + gi;
-          if (i < cnt && sgl == 0 && !(v[u] > w.far))
-            place(Dot::kSq8 ? sqrtf(v[u]) * cfg.sq_out : sqrtf(v[u]), id[u], w);
-        }
-      };
-      for (uint32_t b = 0; b < cnt;) {                    // uniform over the CTA
-        const uint32_t kr = min(cfg.score_rows, (cnt - b + gpb - 1) / gpb);
-        if (Dot::kSq8 && kr >= 8) {
-          rows_at_once(std::integral_constant<int, Dot::kSq8 ? 8 : 4>{}, b);
-          b += 8 * gpb;
-        } else if (kr >= 4) {
-          rows_at_once(std::integral_constant<int, 4>{}, b);
-          b += 4 * gpb;
-        } else if (kr >= 2) {
-          rows_at_once(std::integral_constant<int, 2>{}, b);
-          b += 2 * gpb;
+          first = group_sums<KR>(sum, SG, lane, [](uint32_t p, uint32_t r) { return p + r; });
         } else {
-          rows_at_once(std::integral_constant<int, 1>{}, b);
-          b += gpb;
+          if (Dot::kSq8) prepare();
+#pragma unroll
+          for (uint32_t u = 0; u < KR; u++) {
+            float t = 0.f;
+            if (u < nu) {
+              float2 acc[kQC];
+#pragma unroll
+              for (int j = 0; j < kQC; j++) {
+                acc[j] = make_float2(0.f, 0.f);
+                if ((uint32_t)sgl + (uint32_t)(j * SG) < sc) acc[j] = Dot::add(acc[j], nqc[j], x[u][j]);
+              }
+              t = acc[0].x + acc[0].y;
+#pragma unroll
+              for (int j = 1; j < kQC; j++) t += acc[j].x + acc[j].y;
+            }
+            sum[u] = __float_as_uint(t);
+          }
+          first = group_sums<KR>(sum, SG, lane, [](uint32_t p, uint32_t r) {
+            return __float_as_uint(__uint_as_float(p) + __uint_as_float(r));
+          });
+        }
+        const uint32_t held = max(KR / (uint32_t)SG, 1u);
+        for (uint32_t r = 0; r < held && first + r < nu; r++) {
+          uint32_t bits = sum[0];
+#pragma unroll
+          for (uint32_t k = 1; k < KR; k++) bits = r == k ? sum[k] : bits;
+          const float v = dots ? (float)((int)bits + (int)s.qnorm) * 65536.f : __uint_as_float(bits);
+          const uint32_t i = b + (first + r) * gpb + gi;
+          if (i < cnt && !(v > w.far)) place(Dot::kSq8 ? sqrtf(v) * cfg.sq_out : sqrtf(v), nid[i], w);
         }
       }
     } else if constexpr (Dot::kOn) {
@@ -521,19 +539,11 @@ graph_search_wide_kernel(DevGraph g, const uint4* __restrict__ srows, const uint
     // Alike in every thread: the list is lists[cur * L ..], n entries; warp 0 also keeps
     // the first entry that may be unexpanded.
     uint32_t n = 0, cur = 0, scan0 = 0;
-    {
-      const uint32_t m = s.cnt;
-      score(m, Limits{INFINITY, INFINITY, ~0ull, true});
-      __syncthreads();
-      cta_bitonic_sort(nkey, m, NB);
-      n = min(m, L);
-      for (uint32_t i = tid; i < n; i += blockDim.x) lists[i] = nkey[i];
-      __syncthreads();
-    }
     const float user_radius = P.radius;
 
-    // ---- best-first iterations ---------------------------------------------------------
-    for (uint32_t it = 0; it < cfg.max_iters; it++) {
+    // ---- the seeds' step (it = 0), then best-first iterations ----------------------------
+    for (uint32_t it = 0; it == 0 || it - 1 < cfg.max_iters; it++) {
+      if (it > 0) {
       // control (warp 0): refill from the spill tier when flagged, then pick parents
       if (warp == 0) {
         unsigned long long* list = lists + (size_t)cur * L;
@@ -719,8 +729,9 @@ graph_search_wide_kernel(DevGraph g, const uint4* __restrict__ srows, const uint
           if (fm & (1u << j)) nid[pos++] = ids[j];
       }
       __syncthreads();
+      if (tid == 0) s.dc += s.cnt;
+      }
       const uint32_t cnt = s.cnt;
-      if (tid == 0) s.dc += cnt;
       // ---- distances and placement: below the list's worst -> new keys; else spill ----------
       const unsigned long long* list = lists + (size_t)cur * L;
       {
@@ -728,12 +739,19 @@ graph_search_wide_kernel(DevGraph g, const uint4* __restrict__ srows, const uint
         Limits w;
         w.limit = P.coef * rk;
         const float root = Dot::kSq8 ? w.limit / cfg.sq_out : w.limit;
-        w.far = root * root * 1.0001f;
+        w.far = it == 0 ? INFINITY : root * root * 1.0001f;
         w.worst = (n >= L) ? (list[L - 1] & ~(unsigned long long)kExpandedBit) : ~0ull;
-        w.all = false;
+        w.all = it == 0;                                       // every seed is kept
         score(cnt, w);
       }
       __syncthreads();
+      if (it == 0) {
+        cta_bitonic_sort(nkey, cnt, NB);
+        n = min(cnt, L);
+        for (uint32_t i = tid; i < n; i += blockDim.x) lists[i] = nkey[i];
+        __syncthreads();
+        continue;
+      }
       const uint32_t kept = s.kept;
       if (kept == 0) {
         __syncthreads();            // everyone has read the counter before warp 0 clears it
