@@ -89,6 +89,15 @@ __device__ __forceinline__ uint32_t visit_or(uint32_t* word, uint32_t bit, bool 
                : "=r"(old) : "l"(word), "r"(bit), "l"(policy) : "memory");
   return old;
 }
+// The same without a branch: where `on` is false nothing is touched and the bit reads as set.
+// A step's atomics then all go out before the first result is waited for.
+__device__ __forceinline__ uint32_t visit_or_if(bool on, uint32_t* word, uint32_t bit, uint64_t policy) {
+  uint32_t old;
+  asm volatile("{\n.reg .pred p;\nsetp.ne.u32 p, %4, 0;\nmov.u32 %0, %2;\n"
+               "@p atom.global.or.L2::cache_hint.b32 %0, [%1], %2, %3;\n}\n"
+               : "=&r"(old) : "l"(word), "r"(bit), "l"(policy), "r"((uint32_t)on) : "memory");
+  return old;
+}
 __device__ __forceinline__ void store_zero16(uint4* p, bool hint, uint64_t policy) {
   if (!hint) { *p = make_uint4(0, 0, 0, 0); return; }
   asm volatile("st.global.L2::cache_hint.v4.u32 [%0], {%1, %1, %1, %1}, %2;\n" ::"l"(p), "r"(0u), "l"(policy)
@@ -263,7 +272,7 @@ graph_search_wide_kernel(DevGraph g, const uint4* __restrict__ srows, const uint
   const int SG = (int)cfg.sgroup, NG = (int)cfg.ngroup;
   const int sgl = lane & (SG - 1);
   const bool keep_visited = cfg.l2_policy >= 1, stream_rows = cfg.l2_policy >= 2;
-  const uint64_t pol_keep = keep_visited ? l2_policy_evict_last() : 0ull;
+  const uint64_t pol_keep = keep_visited ? l2_policy_evict_last() : l2_policy_evict_normal();
   const uint64_t pol_stream = stream_rows ? l2_policy_evict_first() : l2_policy_evict_normal();
 
   // A scored row within the limit: below the list's worst entry it joins the new keys,
@@ -706,10 +715,22 @@ graph_search_wide_kernel(DevGraph g, const uint4* __restrict__ srows, const uint
             ids[j] = __ldg(g.edges + s.pbase[p2] + (t - s.pexcl[p2]));
           }
         }
+        if (cfg.smem_bitmap) {
 #pragma unroll
-        for (int j = 0; j < kGatherSlots; j++) {
-          const uint32_t t = base0 + (uint32_t)j * (uint32_t)T + (uint32_t)tid;
-          if (t < total && visit(ids[j])) fm |= 1u << j;
+          for (int j = 0; j < kGatherSlots; j++) {
+            const uint32_t t = base0 + (uint32_t)j * (uint32_t)T + (uint32_t)tid;
+            if (t < total && visit(ids[j])) fm |= 1u << j;
+          }
+        } else {
+          uint32_t old[kGatherSlots];
+#pragma unroll
+          for (int j = 0; j < kGatherSlots; j++) {
+            const uint32_t t = base0 + (uint32_t)j * (uint32_t)T + (uint32_t)tid;
+            old[j] = visit_or_if(t < total, &bitmap[ids[j] >> 5], 1u << (ids[j] & 31u), pol_keep);
+          }
+#pragma unroll
+          for (int j = 0; j < kGatherSlots; j++)
+            if (!((old[j] >> (ids[j] & 31u)) & 1u)) fm |= 1u << j;
         }
         // places in nid: a warp scan of the per-thread counts and one counter
         // increment per warp (the order of the new ids does not matter to this search)
