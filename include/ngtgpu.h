@@ -103,8 +103,8 @@ bool ngtgpu_set_batched_rows_in_flight(NGTIndex, uint32_t rows, NGTError);
  * neighbour slots of one iteration (each parent reads at most
  * neighbour_capacity / parents edges) and sets the shared memory per query.
  * parents: at most 32 (the warp-per-query kernel uses at most 16 of them).
- * NGTGPU_KERNEL_WIDE reads rows_in_flight as the rows each lane group keeps in
- * flight (1, 2 or 4; default 8 for 8-bit rows, else 4). */
+ * NGTGPU_KERNEL_WIDE takes no notice of rows_in_flight (8 rows a lane group for
+ * 8-bit rows, else 4). */
 typedef struct {
   uint32_t list_capacity;
   uint32_t parents;

@@ -874,8 +874,6 @@ void GraphEngine::launch_wide(const uint4* d_rows, size_t nq, const QueryParams*
   cfg.spill_cap = kSpillCapacity;
   // default: visited bitmaps kept in L2, staged rows streamed through it
   cfg.l2_policy = tuning_.l2_policy ? tuning_.l2_policy - 1 : 2u;
-  // rows_in_flight: rows per lane group in flight (default 8 for 8-bit rows, else 4)
-  cfg.score_rows = tuning_.rows_in_flight ? std::min<uint32_t>(tuning_.rows_in_flight, 4) : 8u;
   int max_smem = 0, per_sm = 0;
   NGT_CUDA(cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, device_));
   auto ctas_per_sm = [&](size_t smem) {

@@ -45,7 +45,6 @@ struct WideConfig {
   uint32_t spill_cap;
   uint32_t l2_policy;      // 0: default caching; 1: visited bitmap kept in L2 (evict_last);
                            // 2: as 1, and search rows streamed through L2 (evict_first)
-  uint32_t score_rows;     // rows per lane group in flight (1, 2, 4, or 8 for 8-bit rows)
   // 8-bit search rows of float objects: code = rint((x - sq_offset) / s), the query
   // mapped the same way in 1/256 steps; distance = sqrt(sum) * sq_out (s / 256)
   uint32_t sq8, dim;
@@ -240,11 +239,14 @@ __device__ __forceinline__ void rank_sort_keys(const unsigned long long* in, uns
 // the integer dot products, 0.55 issued per cycle and scheduler.  Measured on 1M x 128,
 // 8-bit rows, k = 10, epsilon 0.08, 10,000 queries, 128 threads: 15.35 ms with a shared-memory
 // row stage (two barriers per 64 rows); rows loaded into registers 15.1 ms; dot products
-// 14.2 ms; one body for every number of rows, sums spread over the lanes 12.55 ms (0.41
-// issued; stalls per issue on instruction fetches 2.8 -> 0.4).  152 queries: 2.0 ms with 128 threads, 1.1 ms with 512 and the visited bitmap in
-// shared memory.  200k x 100 cosine, 1,500 queries from host buffers: 1.80 -> 1.2 ms (packed
-// lanes, three CTAs per SM instead of two).  Not kept: prefetching a step's rows into L2
-// when they are gathered (5 % slower), 1,024 threads (8 % slower than 512).
+// 14.2 ms; one body for every number of rows, sums spread over the lanes 12.55 ms (stalls per
+// issue on instruction fetches 2.8 -> 0.4); visited-bit updates without a branch each 11.5 ms;
+// row loads likewise, a batch ahead 9.6 ms.  152 queries: 2.0 ms with 128 threads, 1.1 ms with
+// 512 and the visited bitmap in shared memory.  200k x 100 cosine, 1,500 queries from host
+// buffers: 1.80 -> 1.0 ms (packed lanes, three CTAs per SM instead of two).  Not kept:
+// prefetching a step's rows into L2 when they are gathered (5 % slower), 1,024 threads (8 %
+// slower than 512), seven and eight CTAs an SM (10 and 24 % slower: their visited bitmaps of
+// 125 KB no longer fit L2).
 template <ObjType ST, ObjType OT, Metric M, int T>
 __global__ void __launch_bounds__(T, T == 64 ? 10 : T == 128 ? 6 : T == 256 ? 3 : 1)
 graph_search_wide_kernel(DevGraph g, const uint4* __restrict__ srows, const uint4* __restrict__ queries,
@@ -318,64 +320,75 @@ graph_search_wide_kernel(DevGraph g, const uint4* __restrict__ srows, const uint
       if (!Dot::kSq8) prepare();                 // 8-bit rows: with each batch, the registers are needed
       const bool dots = Dot::kSq8 && s.fraction == 0;
       const uint4 qc = dots && (uint32_t)sgl < sc ? reinterpret_cast<const uint4*>(qcode)[sgl] : make_uint4(0, 0, 0, 0);
+      // KR rows a lane group and batch (8-bit rows: 4 take 14.0 ms on the sizes above, 8 take
+      // 11.5, 16 with four or five CTAs an SM as long as 8)
       constexpr uint32_t KR = Dot::kSq8 ? 8 : 4;
-      const uint32_t step = min(cfg.score_rows, KR);
-      for (uint32_t b = 0; b < cnt; b += step * gpb) {         // uniform over the CTA
-        const uint32_t nu = min(step, (cnt - b + gpb - 1) / gpb);
-        uint4 x[KR][kQC];
+      const uint32_t step = KR * gpb;
+      uint4 x[KR][kQC];
+      uint32_t id[KR];
+      // Without a branch: past cnt the last row, past a row's end its last chunk, neither of
+      // which counts.  The loads of a batch with a branch each cost 11.5 instead of 9.9 ms.
+      auto rows = [&](uint32_t b) {
 #pragma unroll
-        for (uint32_t u = 0; u < KR; u++) {
-          if (u < nu) {
-            const uint32_t i = b + u * gpb + gi;
-            const uint32_t id = i < cnt ? nid[i] : 0u;
+        for (uint32_t u = 0; u < KR; u++) id[u] = nid[min(b + u * gpb + gi, cnt - 1)];
+      };
+      auto load = [&](uint32_t u) {
 #pragma unroll
-            for (int j = 0; j < kQC; j++) {
-              const uint32_t c = (uint32_t)sgl + (uint32_t)(j * SG);
-              x[u][j] = c < sc ? load_row_chunk(srows + (size_t)id * sc + c, pol_stream) : make_uint4(0, 0, 0, 0);
-            }
-          }
-        }
+        for (int j = 0; j < kQC; j++)
+          x[u][j] = load_row_chunk(srows + (size_t)id[u] * sc + min((uint32_t)sgl + (uint32_t)(j * SG), sc - 1),
+                                   pol_stream);
+      };
+      if (cnt > 0) {
+        rows(0);
+#pragma unroll
+        for (uint32_t u = 0; u < KR; u++) load(u);
+      }
+      for (uint32_t b = 0; b < cnt; b += step) {               // uniform over the CTA
+        const bool more = b + step < cnt;
+        if (more) rows(b + step);
+        const uint32_t nu = min(KR, (cnt - b + gpb - 1) / gpb);
         uint32_t sum[KR];                                      // a lane's part of each row's sum, as bits
         uint32_t first;                                        // the first of the rows whose sum it holds then
+        // the next batch's rows are loaded as this one's are taken (9.9 -> 9.6 ms)
+        auto take = [&](auto part) {
+          if (more) {
+#pragma unroll
+            for (uint32_t u = 0; u < KR; u++) {
+              sum[u] = part(x[u]);
+              load(u);
+            }
+          } else {
+#pragma unroll
+            for (uint32_t u = 0; u < KR; u++) sum[u] = part(x[u]);
+          }
+        };
         if (Dot::kSq8 && dots) {
           // sum (c - q)^2 = sum c c - 2 sum c q + sum q q over whole codes, exact in 32 bits;
           // times 2^16 it is the sum of the squared 1/256 steps that the float form adds up
           // (exact there too, below 2^24 steps of one)
-#pragma unroll
-          for (uint32_t u = 0; u < KR; u++) {
-            if (u < nu) {
-              const uint32_t xw[4] = {x[u][0].x, x[u][0].y, x[u][0].z, x[u][0].w};
-              const uint32_t qw[4] = {qc.x, qc.y, qc.z, qc.w};
-              uint32_t cc = 0, cq = 0;
-#pragma unroll
-              for (int i = 0; i < 4; i++) {
-                cc = __dp4a(xw[i], xw[i], cc);
-                cq = __dp4a(xw[i], qw[i], cq);
-              }
-              sum[u] = cc - 2u * cq;
-            } else {
-              sum[u] = 0u;
-            }
-          }
+          take([&](const uint4 (&y)[kQC]) {
+            uint32_t cc = 0, cq = 0;
+            cc = __dp4a(y[0].x, y[0].x, cc); cq = __dp4a(y[0].x, qc.x, cq);
+            cc = __dp4a(y[0].y, y[0].y, cc); cq = __dp4a(y[0].y, qc.y, cq);
+            cc = __dp4a(y[0].z, y[0].z, cc); cq = __dp4a(y[0].z, qc.z, cq);
+            cc = __dp4a(y[0].w, y[0].w, cc); cq = __dp4a(y[0].w, qc.w, cq);
+            return (uint32_t)sgl < sc ? cc - 2u * cq : 0u;
+          });
           first = group_sums<KR>(sum, SG, lane, [](uint32_t p, uint32_t r) { return p + r; });
         } else {
           if (Dot::kSq8) prepare();
+          take([&](const uint4 (&y)[kQC]) {
+            float2 acc[kQC];
 #pragma unroll
-          for (uint32_t u = 0; u < KR; u++) {
-            float t = 0.f;
-            if (u < nu) {
-              float2 acc[kQC];
-#pragma unroll
-              for (int j = 0; j < kQC; j++) {
-                acc[j] = make_float2(0.f, 0.f);
-                if ((uint32_t)sgl + (uint32_t)(j * SG) < sc) acc[j] = Dot::add(acc[j], nqc[j], x[u][j]);
-              }
-              t = acc[0].x + acc[0].y;
-#pragma unroll
-              for (int j = 1; j < kQC; j++) t += acc[j].x + acc[j].y;
+            for (int j = 0; j < kQC; j++) {
+              acc[j] = make_float2(0.f, 0.f);
+              if ((uint32_t)sgl + (uint32_t)(j * SG) < sc) acc[j] = Dot::add(acc[j], nqc[j], y[j]);
             }
-            sum[u] = __float_as_uint(t);
-          }
+            float t = acc[0].x + acc[0].y;
+#pragma unroll
+            for (int j = 1; j < kQC; j++) t += acc[j].x + acc[j].y;
+            return __float_as_uint(t);
+          });
           first = group_sums<KR>(sum, SG, lane, [](uint32_t p, uint32_t r) {
             return __float_as_uint(__uint_as_float(p) + __uint_as_float(r));
           });
