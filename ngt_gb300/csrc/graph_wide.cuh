@@ -241,7 +241,7 @@ __device__ __forceinline__ void rank_sort_keys(const unsigned long long* in, uns
 // row stage (two barriers per 64 rows); rows loaded into registers 15.1 ms; dot products
 // 14.2 ms; one body for every number of rows, sums spread over the lanes 12.55 ms (stalls per
 // issue on instruction fetches 2.8 -> 0.4); visited-bit updates without a branch each 11.5 ms;
-// row loads likewise, a batch ahead 9.6 ms.  152 queries: 2.0 ms with 128 threads, 1.1 ms with
+// row loads likewise, a batch ahead 9.2 ms.  152 queries: 2.0 ms with 128 threads, 1.1 ms with
 // 512 and the visited bitmap in shared memory.  200k x 100 cosine, 1,500 queries from host
 // buffers: 1.80 -> 1.0 ms (packed lanes, three CTAs per SM instead of two).  Not kept:
 // prefetching a step's rows into L2 when they are gathered (5 % slower), 1,024 threads (8 %
@@ -325,37 +325,31 @@ graph_search_wide_kernel(DevGraph g, const uint4* __restrict__ srows, const uint
       constexpr uint32_t KR = Dot::kSq8 ? 8 : 4;
       const uint32_t step = KR * gpb;
       uint4 x[KR][kQC];
-      uint32_t id[KR];
       // Without a branch: past cnt the last row, past a row's end its last chunk, neither of
       // which counts.  The loads of a batch with a branch each cost 11.5 instead of 9.9 ms.
-      auto rows = [&](uint32_t b) {
-#pragma unroll
-        for (uint32_t u = 0; u < KR; u++) id[u] = nid[min(b + u * gpb + gi, cnt - 1)];
-      };
-      auto load = [&](uint32_t u) {
+      auto load = [&](uint32_t u, uint32_t b) {
+        const uint32_t id = nid[min(b + u * gpb + gi, cnt - 1)];
 #pragma unroll
         for (int j = 0; j < kQC; j++)
-          x[u][j] = load_row_chunk(srows + (size_t)id[u] * sc + min((uint32_t)sgl + (uint32_t)(j * SG), sc - 1),
+          x[u][j] = load_row_chunk(srows + (size_t)id * sc + min((uint32_t)sgl + (uint32_t)(j * SG), sc - 1),
                                    pol_stream);
       };
       if (cnt > 0) {
-        rows(0);
 #pragma unroll
-        for (uint32_t u = 0; u < KR; u++) load(u);
+        for (uint32_t u = 0; u < KR; u++) load(u, 0);
       }
       for (uint32_t b = 0; b < cnt; b += step) {               // uniform over the CTA
         const bool more = b + step < cnt;
-        if (more) rows(b + step);
         const uint32_t nu = min(KR, (cnt - b + gpb - 1) / gpb);
         uint32_t sum[KR];                                      // a lane's part of each row's sum, as bits
         uint32_t first;                                        // the first of the rows whose sum it holds then
-        // the next batch's rows are loaded as this one's are taken (9.9 -> 9.6 ms)
+        // the next batch's rows are loaded as this one's are taken (9.9 -> 9.2 ms)
         auto take = [&](auto part) {
           if (more) {
 #pragma unroll
             for (uint32_t u = 0; u < KR; u++) {
               sum[u] = part(x[u]);
-              load(u);
+              load(u, b + step);
             }
           } else {
 #pragma unroll
