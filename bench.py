@@ -55,12 +55,12 @@ RECALL_TARGET = 0.95
 QS8_EPS_SWEEP = [0.08, 0.1, 0.11, 0.12, 0.13, 0.14, 0.15, 0.17, 0.2, 0.25, 0.3]
 # Batched-kernel candidates of the autotuner.  kernel 1: warp per query (R rows per
 # lane group in flight, registers budgeted for C CTAs per SM, NB neighbour slots per
-# step; 0 = automatic); kernel 3: CTA per query (T threads, `stage` KB of staged rows).
+# step; 0 = automatic); kernel 3: CTA per query (T threads; `stage` has no effect).
 BATCHED_CANDIDATES = [
     dict(kernel=1, L=256, P=3, R=4, C=5, NB=256), dict(kernel=1, L=256, P=4, R=6, C=4, NB=0),
-    dict(kernel=3, L=256, P=8, T=128, stage=16), dict(kernel=3, L=256, P=8, T=128, stage=8),
+    dict(kernel=3, L=256, P=8, T=128, stage=16),
     dict(kernel=3, L=256, P=10, T=128, stage=16), dict(kernel=3, L=256, P=12, T=128, stage=16),
-    dict(kernel=3, L=256, P=8, T=128, stage=32), dict(kernel=3, L=256, P=16, T=128, stage=16),
+    dict(kernel=3, L=256, P=16, T=128, stage=16),
     dict(kernel=3, L=256, P=16, T=256, stage=32), dict(kernel=3, L=256, P=8, T=256, stage=32)]
 WIDE_PARENTS = 32                 # parents per step of the CTA-per-query kernel the serving loop uses
 # dram__bytes_read.sum + dram__bytes_write.sum of one launch of 2,000 queries on
@@ -1362,7 +1362,7 @@ def main():
                        "headline": ("batched kernel (%s, %s search rows, exact fp32 re-rank), epsilon=%g, "
                                     "autotuned settings %s"
                                     % ("warp per query" if head["config"]["kernel"] == KERNEL_BATCHED
-                                       else "CTA per query, rows of a step staged in shared memory",
+                                       else "CTA per query, rows of a step loaded into registers",
                                        rows_text, head["epsilon"], json.dumps(head["config"], sort_keys=True))),
                        "recall_at_k": round(head["recall"], 4), "epsilon_curve": curves[KERNEL_BATCHED],
                        "plain_fp32": {"qps": round(plain["qps"], 1), "epsilon": plain["epsilon"],
@@ -1386,7 +1386,7 @@ def main():
                          "peak_source": peak_kind,
                          "basis": "(%d*DC + 4*edges + %d query + re-rank %d*2k) bytes per query over the kernel's "
                                   "median event time" % (head["row_bytes"], row_bytes, row_bytes)},
-            "served": {"kernel": "CTA per query (%s search rows, rows of a step staged in shared memory), "
+            "served": {"kernel": "CTA per query (%s search rows, rows of a step loaded into registers), "
                                  "%d parents per step; up to 8 launches of at most 512 queries in flight, "
                                  "a launch holds requests of one shared-memory class" % (wide_rows, WIDE_PARENTS),
                        "stream": "Poisson arrivals, request sizes geometric on 1..256 (mean ~16), k 10 (3/4) or "
