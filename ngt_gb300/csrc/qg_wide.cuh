@@ -326,6 +326,7 @@ qg_wide_kernel(DevGraph g, DevQG qg, const uint4* __restrict__ queries, uint32_t
         const uint32_t nblk = s.nblk;
         const float limit = s.limit;
         unsigned long long* pend = nkey;
+        uint32_t j = 0;                                    // the parent of the block, in turn
         for (uint32_t b0 = (uint32_t)warp * BPI; b0 < nblk; b0 += (uint32_t)BPI * kQGWideWarps) {
           uint2 w[BPI][SPL];
           uint32_t idv[BPI], pj[BPI], lbk[BPI];
@@ -334,7 +335,6 @@ qg_wide_kernel(DevGraph g, DevQG qg, const uint4* __restrict__ queries, uint32_t
           for (int u = 0; u < BPI; u++) {
             const uint32_t bi = b0 + (uint32_t)u;
             on[u] = bi < nblk;
-            uint32_t j = 0;
             if (on[u])
               while (j + 1 < np && s.pblk[j + 1] <= bi) j++;
             pj[u] = j;
@@ -386,6 +386,7 @@ qg_wide_kernel(DevGraph g, DevQG qg, const uint4* __restrict__ queries, uint32_t
           }
 #pragma unroll
           for (int r = 0; r < 8; r++) {
+            if (b + (uint32_t)r * kQGWideThreads >= npend) break;        // alike in the CTA
             const bool is_new = (old[r] & bit[r]) == 0u;
             const unsigned bal = __ballot_sync(0xffffffffu, is_new);
             uint32_t base = 0;
