@@ -824,12 +824,12 @@ void GraphEngine::launch_wide(const uint4* d_rows, size_t nq, const QueryParams*
   int sms = 0;
   NGT_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device_));
   // Threads per query: the tuning's, or by how many queries share the SMs.  512 while each
-  // has an SM to itself (152 queries, 1M x 128, 10 parents: 1.21 ms, with 256 threads
-  // 1.55 ms; 200k x 100 cosine 0.20 and 0.27 ms), and up to two per SM on large indexes,
-  // whose visited bitmaps then stay in shared memory (304 queries: 1.42 and 1.63 ms; 200k:
-  // 0.33 and 0.28 ms).  128 from six per SM on, where there is such a kernel and few parents
-  // a step (10,000 queries: 15.1 ms, with 256 threads 16.0 ms; 50k x 64: 1.07 and 1.25 ms;
-  // with 32 parents 41.4 and 29.6 ms).
+  // has an SM to itself (152 queries, 1M x 128, 10 parents: 1.03 ms, with 256 threads
+  // 1.22 ms; 200k x 100 cosine 0.17 and 0.23 ms), and up to two per SM on large indexes,
+  // whose visited bitmaps then stay in shared memory (304 queries: 1.20 and 1.28 ms; 200k:
+  // 0.31 and 0.24 ms).  128 from six per SM on, where there is such a kernel and few parents
+  // a step (10,000 queries: 9.5 ms, with 256 threads 12.0 ms; 50k x 64: 0.80 and 1.25 ms;
+  // with 32 parents 30.2 and 25.0 ms).
   uint32_t threads = tuning_.cta_threads;
   if (!threads) {
     const size_t own_sm = host_.nrows >= (1u << 18) ? 2 * (size_t)sms : (size_t)sms;
@@ -886,7 +886,7 @@ void GraphEngine::launch_wide(const uint4* d_rows, size_t nq, const QueryParams*
   if (smem > (size_t)max_smem) throw std::runtime_error("wide search state does not fit in shared memory");
   per_sm = ctas_per_sm(smem);
   // the visited bitmap lies in shared memory where that costs no CTA of an SM (200k x 100
-  // cosine, 10,000 queries: 4.26 ms, in global memory 4.54 ms), with 512 threads wherever
+  // cosine, 10,000 queries: 4.21 ms, in global memory 4.39 ms), with 512 threads wherever
   // it fits (up to about 1.5M objects)
   cfg.smem_bitmap = 1;
   const size_t smem_with = wide_kernel_smem_bytes(dev_.row_chunks, cfg);

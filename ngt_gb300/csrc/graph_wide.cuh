@@ -241,7 +241,7 @@ __device__ __forceinline__ void rank_sort_keys(const unsigned long long* in, uns
 // row stage (two barriers per 64 rows); rows loaded into registers 15.1 ms; dot products
 // 14.2 ms; one body for every number of rows, sums spread over the lanes 12.55 ms (stalls per
 // issue on instruction fetches 2.8 -> 0.4); visited-bit updates without a branch each 11.5 ms;
-// row loads likewise, a batch ahead 9.2 ms.  152 queries: 2.0 ms with 128 threads, 1.1 ms with
+// row loads likewise, a batch ahead 9.2 ms.  152 queries: 1.22 ms with 256 threads, 1.03 ms with
 // 512 and the visited bitmap in shared memory.  200k x 100 cosine, 1,500 queries from host
 // buffers: 1.80 -> 1.0 ms (packed lanes, three CTAs per SM instead of two).  Not kept:
 // prefetching a step's rows into L2 when they are gathered (5 % slower), 1,024 threads (8 %
