@@ -246,7 +246,10 @@ __device__ __noinline__ bool merge_results(unsigned long long* res, uint32_t siz
   const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint32_t n = s.nres;
   // below zero (the scalar-quantized inner product) the exploration radius is the tighter one
-  if (key_dist(sv[0]) < 0.f || (n && key_dist(res[0]) < 0.f)) return false;
+  if (key_dist(sv[0]) < 0.f || (n && key_dist(res[0]) < 0.f)) {
+    __syncthreads();                         // every warp has decided before the replay rewrites res and s.nres
+    return false;
+  }
   const uint32_t p = upper_bound_dist(sv, m, radius);
   const bool ro = mode == (uint32_t)GraphMode::ReadOnly;
   const uint32_t fill = n < size ? size - n : 0u;

@@ -118,3 +118,43 @@ def test_result_sets_with_ties(tmp_path, k, mode):
     assert np.array_equal(n, on)
     for j in range(len(q)):
         assert np.array_equal(ids[j, :n[j]], oi[j, :n[j]]) and np.array_equal(ds[j, :n[j]], od[j, :n[j]])
+
+
+# Distances below zero (int8 codes under the inner product: whole numbers of either sign,
+# exact in a float), where the updates of the result set are replayed one by one.  With size 1
+# and a radius a read-only search may hold one negative result and a round of neighbours none
+# of which is negative.
+@pytest.mark.parametrize("mode", ["read_only", "updatable"])
+@pytest.mark.parametrize("k", [1, 2, 30])
+def test_negative_distances(tmp_path, k, mode):
+    from ngt_gb300 import Index
+    path = str(tmp_path / "ix")
+    n, dim = 2000, 15                                     # 16 elements a row with the inner product's own
+    _index(path, n, dim, 24, 11)
+    prf = open(os.path.join(path, "prf")).read()
+    for old, new in (("ObjectType\tFloat-4", "ObjectType\tQSUInteger-8B"), ("DistanceType\tL2",
+                     "DistanceType\tInnerProduct\nMaxMagnitude\t1\nQuantizationOffset\t0\nQuantizationScale\t127.5")):
+        prf = prf.replace(old, new)
+    open(os.path.join(path, "prf"), "w").write(prf)
+    rng = np.random.default_rng(12)
+    rec = np.empty((n, 2 + dim), np.uint8)
+    rec[:, 0] = ord("+")
+    rec[:, 1:] = rng.integers(0, 256, (n, dim + 1))       # 127 * 127 * 16 - sum of products: of either sign
+    with open(os.path.join(path, "obj"), "wb") as f:
+        f.write(np.uint64(n + 1).tobytes() + b"-" + rec.tobytes())
+    q = (rng.integers(75, 128, (160, 1)) - rng.integers(0, 50, (160, dim))).astype(np.float32)
+    o = oracle.Oracle(oracle.IndexFiles(path))
+    signs = set()
+    with Index(path, read_only=mode == "read_only") as ix:
+        for eps in (-0.2, 0.0, 0.3, 4.0):
+            for radius in (-1.0, 0.0, 20000.0):
+                oi, od, on, dc = o.search(q, k=k, epsilon=eps, radius=radius, mode=mode, threads=8)
+                for nq in (9, 160):                       # 512 and 128 threads a query
+                    ids, ds, c, st = ix.batch_search(q[:nq], k=k, epsilon=eps, radius=radius, with_stats=True)
+                    assert np.array_equal(c, on[:nq]), (eps, radius, nq)
+                    assert np.array_equal(st["distance_computations"], dc[:nq]), (eps, radius, nq)
+                    for j in range(nq):
+                        assert np.array_equal(ids[j, :c[j]], oi[j, :c[j]]), (eps, radius, nq, j)
+                        assert np.array_equal(ds[j, :c[j]], od[j, :c[j]]), (eps, radius, nq, j)
+                        signs.update(np.sign(ds[j, :c[j]]).tolist())
+    assert -1.0 in signs and 1.0 in signs
