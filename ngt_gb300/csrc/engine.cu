@@ -742,47 +742,49 @@ void GraphEngine::search_device_slot(const uint4* d_rows, size_t nq, const Searc
   // the pageable host parameter copies above are complete once they return
 }
 
-size_t GraphEngine::exact_launch_config(uint32_t max_size, ExactConfig& cfg, uint32_t threads) const {
+size_t GraphEngine::exact_launch_config(uint32_t max_size, ExactConfig& cfg, uint32_t& threads) const {
   cfg = ExactConfig{};
   cfg.kcap = max_size + 1;
   // a short shared list: what it cannot hold waits in the overflow tier, and a step merges
   // less (1M x 128, 10,000 queries: 1024 keys 42.5 ms, 512 35.0 ms, 256 34.4 ms)
   cfg.ccap = std::min<uint32_t>(1024, std::max<uint32_t>(256, next_pow2(cfg.kcap)));
-  // the visited set: a bitmap in shared memory of at most 32 KB (200,000 objects, 25 KB:
-  // 1,500 queries in 1.03 ms against 1.10 ms with a hash that moves to global memory;
-  // 50,000 objects, 6 KB: 10,000 queries in 1.14 against 1.22 ms), else a small hash, from
-  // which every query of a large index moves to its global bitmap soon anyway
-  cfg.hcap = 2048;
   cfg.mode = (uint32_t)mode_;
   cfg.group = std::min<uint32_t>(32, next_pow2((uint32_t)dev_.row_chunks));
   cfg.bitmap_words = (host_.nrows + 31) / 32;
   cfg.ocap = kOverflowCapacity;
   int max_smem = 0;
   NGT_CUDA(cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, device_));
+  auto bytes = [&] { return exact_smem_bytes(dev_.row_chunks, cfg, threads); };
+  auto fits = [&] { return bytes() <= (size_t)max_smem; };
+  // the visited set of 128 threads: a bitmap in shared memory of at most 32 KB (200,000
+  // objects, 25 KB: 1,500 queries in 1.03 ms against 1.10 ms with a hash that moves to
+  // global memory; 50,000 objects, 6 KB: 10,000 queries in 1.14 against 1.22 ms), else a
+  // small hash, from which every query of a large index moves to its global bitmap soon
+  // anyway.  512 threads have an SM to themselves: a bitmap where it fits (up to about 1.6M
+  // objects), else a larger hash.
+  const auto visited = [&](uint32_t hash, bool bitmap) {
+    cfg.smem_bitmap = bitmap ? 1u : 0u;
+    cfg.hcap = bitmap ? cfg.bitmap_words : hash;
+    return fits();
+  };
+  // a result set that leaves less room takes the hash, then smaller ones and a shorter list
+  const auto shrink = [&](uint32_t hash, bool bitmap) {
+    if (bitmap && visited(hash, true)) return true;
+    if (visited(hash, false)) return true;
+    while (cfg.hcap > 2048 && !fits()) cfg.hcap >>= 1;
+    while (cfg.ccap > 256 && !fits()) cfg.ccap >>= 1;
+    while (cfg.hcap > 1024 && !fits()) cfg.hcap >>= 1;
+    return fits();
+  };
   if (threads == 512) {
-    // the query has an SM to itself: a visited bitmap in shared memory where it fits (up
-    // to about 1.6M objects), else a larger hash
-    cfg.hcap = cfg.bitmap_words;
-    cfg.smem_bitmap = 1;
-    const size_t smem = exact_smem_bytes(dev_.row_chunks, cfg, threads);
-    if (smem <= (size_t)max_smem) return smem;
-    cfg.smem_bitmap = 0;
-    cfg.hcap = 16384;
-  } else if (cfg.bitmap_words <= 8192) {
-    cfg.smem_bitmap = 1;
-    cfg.hcap = cfg.bitmap_words;
+    const uint32_t ccap = cfg.ccap;
+    if (shrink(16384, true)) return bytes();
+    threads = kExactThreads;                 // whose rounds are half as large
+    cfg.ccap = ccap;
   }
-  size_t smem = exact_smem_bytes(dev_.row_chunks, cfg, threads);
-  while (smem > (size_t)max_smem && !cfg.smem_bitmap && cfg.hcap > 2048) {
-    cfg.hcap >>= 1;
-    smem = exact_smem_bytes(dev_.row_chunks, cfg, threads);
-  }
-  while (smem > (size_t)max_smem && cfg.ccap > 256) {
-    cfg.ccap >>= 1;
-    smem = exact_smem_bytes(dev_.row_chunks, cfg, threads);
-  }
-  if (smem > (size_t)max_smem) throw std::runtime_error("result size too large for the on-chip search state");
-  return smem;
+  if (!shrink(2048, cfg.bitmap_words <= 8192))
+    throw std::runtime_error("result size too large for the on-chip search state");
+  return bytes();
 }
 
 void GraphEngine::launch_exact(const uint4* d_rows, size_t nq, const QueryParams* d_params, const uint32_t* d_seeds,
@@ -793,7 +795,7 @@ void GraphEngine::launch_exact(const uint4* d_rows, size_t nq, const QueryParams
   int per_sm = 0, sms = 0;
   NGT_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device_));
   // a launch of no more CTAs than SMs leaves each query an SM: 512 threads per query
-  const uint32_t threads = (bitmaps ? std::min(nq, grid_cap) : nq) <= (size_t)sms ? 512u : (uint32_t)kExactThreads;
+  uint32_t threads = (bitmaps ? std::min(nq, grid_cap) : nq) <= (size_t)sms ? 512u : (uint32_t)kExactThreads;
   const size_t smem = exact_launch_config(max_size, cfg, threads);
   ExactKernelFn fn = exact_kernel(host_.prop.otype, host_.prop.metric, threads);
   NGT_CUDA(cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -1363,7 +1365,8 @@ void GraphEngine::search_device_noalloc(void* scratch, size_t scratch_bytes, con
   uint32_t max_size = 0;
   build_params(args, nargs, nq, kmax, params, seeds, max_size);
   ExactConfig cfg;
-  const size_t smem = exact_launch_config(max_size, cfg, kExactThreads);
+  uint32_t threads = kExactThreads;
+  const size_t smem = exact_launch_config(max_size, cfg, threads);
   // scratch layout: params | seeds | bitmaps[grid] | overflow[grid], each 256-byte aligned
   auto up = [](size_t v) { return (v + 255) & ~(size_t)255; };
   const size_t params_bytes = up(nq * sizeof(QueryParams));

@@ -268,9 +268,9 @@ class GraphEngine {
                              const SearchArgs* args, size_t nargs, ObjDist* d_out, uint32_t* d_counts,
                              QueryStats* d_stats, size_t kmax, cudaStream_t stream);
   // The exact kernel's configuration for result sizes up to max_size and `threads` per
-  // query: fills cfg and returns its dynamic shared memory (shared by every exact launch
-  // path).
-  size_t exact_launch_config(uint32_t max_size, ExactConfig& cfg, uint32_t threads) const;
+  // query (512 become 128 where their state would not fit): fills cfg and returns its
+  // dynamic shared memory (shared by every exact launch path).
+  size_t exact_launch_config(uint32_t max_size, ExactConfig& cfg, uint32_t& threads) const;
   void set_tuning(const FastTuning& t) { tuning_ = t; }
   const FastTuning& tuning() const { return tuning_; }
   bool fast_supported(Kernel k) const;

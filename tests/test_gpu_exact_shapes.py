@@ -158,3 +158,39 @@ def test_negative_distances(tmp_path, k, mode):
                         assert np.array_equal(ds[j, :c[j]], od[j, :c[j]]), (eps, radius, nq, j)
                         signs.update(np.sign(ds[j, :c[j]]).tolist())
     assert -1.0 in signs and 1.0 in signs
+
+
+# Result sets that leave no room for a visited bitmap in shared memory: the hash takes its
+# place, then smaller ones, then (one query an SM) 128 threads instead of 512.  26,981 is what
+# 232,448 bytes held beside a row of four chunks, 256 keys of the list twice, a round's keys
+# and a hash of 2,048 words.
+@pytest.mark.parametrize("n", [30_000, 200_000, 262_143])
+def test_largest_result_sizes(tmp_path, n):
+    import ctypes
+
+    import torch
+    from ngt_gb300 import Index
+    from ngt_gb300.base import QUERY_STATS_DTYPE
+    from test_zz_no_alloc import _noalloc
+    path = str(tmp_path / "ix")
+    q = _index(path, n, 4, 12, n)[:153]
+    files = oracle.IndexFiles(path)
+    for k in (23_900, 26_981):
+        oi, od, on, dc = oracle.Oracle(files).search(q[:12], k=k, epsilon=0.0, threads=8)
+        with Index(path, read_only=True) as ix:
+            for nq in (1, 153):
+                ids, ds, c, st = ix.batch_search(q[:nq], k=k, epsilon=0.0, with_stats=True)
+                for j in range(min(nq, 12)):
+                    assert c[j] == on[j] and st["distance_computations"][j] == dc[j]
+                    assert np.array_equal(ids[j, :c[j]], oi[j, :c[j]]) and np.array_equal(ds[j, :c[j]], od[j, :c[j]])
+            rows = torch.from_numpy(ix.convert_queries(q[:12])).cuda()
+            params, nparams = ix.make_params(k, 0.0)
+            r = torch.zeros((12, k, 2), dtype=torch.int32, device="cuda")
+            c = torch.zeros(12, dtype=torch.int32, device="cuda")
+            st = torch.zeros((12, QUERY_STATS_DTYPE.itemsize // 4), dtype=torch.int32, device="cuda")
+            ix._check(_noalloc(ix._lib)(ix._index, rows.data_ptr(), 12, ctypes.cast(params, ctypes.c_void_p), nparams,
+                                        r.data_ptr(), k, c.data_ptr(), st.data_ptr(), None, ix._err))
+            torch.cuda.synchronize()
+            c, r = c.cpu().numpy(), r.cpu().numpy()
+            for j in range(12):
+                assert c[j] == on[j] and np.array_equal(r[j, :c[j], 0].view(np.uint32), oi[j, :c[j]])
