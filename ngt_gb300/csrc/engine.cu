@@ -826,17 +826,17 @@ void GraphEngine::launch_wide(const uint4* d_rows, size_t nq, const QueryParams*
   int sms = 0;
   NGT_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device_));
   // Threads per query: the tuning's, or by how many queries share the SMs.  512 while each
-  // has an SM to itself (152 queries, 1M x 128, 10 parents: 1.03 ms, with 256 threads
-  // 1.22 ms; 200k x 100 cosine 0.17 and 0.23 ms), and up to two per SM on large indexes,
-  // whose visited bitmaps then stay in shared memory (304 queries: 1.20 and 1.28 ms; 200k:
-  // 0.31 and 0.24 ms).  128 from six per SM on, where there is such a kernel and few parents
+  // has an SM to itself (100 queries, 1M x 128, 10 parents: 0.97 ms, with 256 threads
+  // 1.10 ms; 200k x 100 cosine, 152: 0.17 and 0.23 ms; 2M x 32, whose visited bitmap is in
+  // global memory: 0.27 both), 256 from there on (304 queries, 1M x 128: 1.15 ms, with 512
+  // threads, which then take two rounds, 1.29 ms; 300k x 96: 0.18 and 0.21 ms; 2M x 32:
+  // 0.28 and 0.39 ms).  128 from six per SM on, where there is such a kernel and few parents
   // a step (10,000 queries: 9.5 ms, with 256 threads 12.0 ms; 50k x 64: 0.80 and 1.25 ms;
   // with 32 parents 30.2 and 25.0 ms).
   uint32_t threads = tuning_.cta_threads;
   if (!threads) {
-    const size_t own_sm = host_.nrows >= (1u << 18) ? 2 * (size_t)sms : (size_t)sms;
     const bool few_parents = tuning_.parents <= 16;
-    threads = nq <= own_sm ? 512u : 256u;
+    threads = nq <= (size_t)sms ? 512u : 256u;
     if (nq >= 6 * (size_t)sms && few_parents && wide_kernel(host_.prop.otype, host_.prop.metric, rows, 128))
       threads = 128;
   }
