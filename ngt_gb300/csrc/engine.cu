@@ -823,23 +823,7 @@ void GraphEngine::launch_wide(const uint4* d_rows, size_t nq, const QueryParams*
                               cudaStream_t stream, FastScratch& scratch) {
   const SearchRows rows = wide_search_rows();
   const bool bf16 = rows == SearchRows::Bf16, sq8 = rows == SearchRows::Sq8;
-  int sms = 0;
-  NGT_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device_));
-  // Threads per query: the tuning's, or by how many queries share the SMs.  512 while each
-  // has an SM to itself (100 queries, 1M x 128, 10 parents: 0.97 ms, with 256 threads
-  // 1.10 ms; 200k x 100 cosine, 152: 0.17 and 0.23 ms; 2M x 32, whose visited bitmap is in
-  // global memory: 0.27 both), 256 from there on (304 queries, 1M x 128: 1.15 ms, with 512
-  // threads, which then take two rounds, 1.29 ms; 300k x 96: 0.18 and 0.21 ms; 2M x 32:
-  // 0.28 and 0.39 ms).  128 from six per SM on, where there is such a kernel and few parents
-  // a step (10,000 queries: 9.5 ms, with 256 threads 12.0 ms; 50k x 64: 0.80 and 1.25 ms;
-  // with 32 parents 30.2 and 25.0 ms).
-  uint32_t threads = tuning_.cta_threads;
-  if (!threads) {
-    const bool few_parents = tuning_.parents <= 16;
-    threads = nq <= (size_t)sms ? 512u : 256u;
-    if (nq >= 6 * (size_t)sms && few_parents && wide_kernel(host_.prop.otype, host_.prop.metric, rows, 128))
-      threads = 128;
-  }
+  uint32_t threads = tuning_.cta_threads ? tuning_.cta_threads : 256u;
   WideKernelFn fn = wide_kernel(host_.prop.otype, host_.prop.metric, rows, threads);
   if (!fn) throw std::runtime_error("the wide kernel does not support this index type or CTA size");
   if (bf16) ensure_bf16_rows();
@@ -857,6 +841,26 @@ void GraphEngine::launch_wide(const uint4* d_rows, size_t nq, const QueryParams*
   cfg.nbr_cap = tuning_.nbr_cap ? std::max<uint32_t>({next_pow2(tuning_.nbr_cap), next_pow2(rerank_max), L})
                                 : std::max<uint32_t>({512u, next_pow2(rerank_max), L,
                                                       std::min<uint32_t>(4096, next_pow2(cfg.parents * 100))});
+  // Threads per query where the tuning does not say: by how many queries share the SMs.  512
+  // while each has an SM to itself (100 queries, 1M x 128, 10 parents: 0.97 ms, with 256
+  // threads 1.10 ms; 200k x 100 cosine, 152: 0.17 and 0.23 ms; 2M x 32, whose visited bitmap
+  // is in global memory: 0.27 both), 256 from there on (304 queries, 1M x 128: 1.15 ms, with
+  // 512 threads, which then take two rounds, 1.29 ms; 300k x 96: 0.18 and 0.21 ms; 2M x 32:
+  // 0.28 and 0.39 ms).  128 from six per SM on, where there is such a kernel and a step has at
+  // most 1,024 neighbour slots, by default up to 10 parents (6,000 queries, 1M x 128, 10
+  // parents: 5.9 ms, with 256 threads 7.0 ms; 16 parents of 1,024 slots: 5.4 and 6.0 ms).
+  // More slots in each of six CTAs' shared memory leave L1 too little for the row loads: 10
+  // parents with 2,048 slots 9.4 ms, with 256 threads 6.9 ms; 11 parents 9.4 and 6.8 ms, 16
+  // 9.4 and 6.3 ms, 32 8.5 and 7.0 ms; 200k x 64, 12 parents 3.9 and 3.0 ms.
+  int sms = 0;
+  NGT_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device_));
+  if (!tuning_.cta_threads) {
+    threads = nq <= (size_t)sms ? 512u : 256u;
+    if (nq >= 6 * (size_t)sms && cfg.nbr_cap <= 1024 &&
+        wide_kernel(host_.prop.otype, host_.prop.metric, rows, 128))
+      threads = 128;
+    fn = wide_kernel(host_.prop.otype, host_.prop.metric, rows, threads);
+  }
   cfg.search_chunks = bf16 ? dev_.row_chunks / 2 : sq8 ? dev_.row_chunks / 4 : dev_.row_chunks;
   if (sq8) {
     cfg.sq8 = 1;

@@ -80,3 +80,21 @@ def test_integer_dot_products(tmp_path, dim):
         for j in (1, 3):                     # a query's form does not depend on the others'
             alone = _wide(ix, q[j:j + 1], 10, 0.3, search_rows=2)
             assert np.array_equal(alone[0][0], one[0][j]) and np.array_equal(alone[1][0], one[1][j])
+
+
+# The rule's other line: 128 threads only while a step has at most 1,024 neighbour slots (10
+# parents, or as many slots as the caller sets).
+@pytest.mark.parametrize("tuning", [dict(parents=10), dict(parents=11), dict(parents=16), dict(parents=17),
+                                    dict(parents=16, neighbour_capacity=1024),
+                                    dict(parents=4, neighbour_capacity=2048)])
+def test_threads_by_neighbour_slots(tmp_path, tuning):
+    from ngt_gb300 import Index
+    path = str(tmp_path / "ix")
+    q = np.concatenate([_index(path, 5000, 20, 40, 3)] * 3)[:920]
+    with Index(path, read_only=True) as ix:
+        for rows in (1, 2):
+            got = _wide(ix, q, 10, 0.2, search_rows=rows, **tuning)
+            for threads in (128, 256):
+                ref = _wide(ix, q, 10, 0.2, search_rows=rows, cta_threads=threads, **tuning)
+                for a, b in zip(ref, got):
+                    assert np.array_equal(a, b), (rows, threads)
