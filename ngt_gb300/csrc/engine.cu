@@ -91,6 +91,29 @@ bool is_normalized(Metric m) {
 
 }  // namespace
 
+cudaError_t allow_smem(const void* fn, int device, size_t bytes) {
+  // the functions' static sizes, asked for once each (2 us a call)
+  static std::mutex mu;
+  static std::map<const void*, int> sizes;
+  int own = 0, optin = 0;
+  {
+    std::lock_guard<std::mutex> lock(mu);
+    const auto it = sizes.find(fn);
+    if (it != sizes.end()) {
+      own = it->second;
+    } else {
+      cudaFuncAttributes a{};
+      const cudaError_t e = cudaFuncGetAttributes(&a, fn);
+      if (e != cudaSuccess) return e;
+      own = sizes[fn] = (int)a.sharedSizeBytes;
+    }
+  }
+  const cudaError_t e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
+  if (e != cudaSuccess) return e;
+  if (bytes > (size_t)(optin - own)) return cudaErrorInvalidValue;
+  return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - own);
+}
+
 // The engine's own memory pool for the buffers of one call.  The device's default pool
 // returns its memory to the driver at every synchronisation, so that each host-buffer call
 // mapped its few buffers anew (about 0.3 ms); this one keeps up to 64 MB until the engine
@@ -798,7 +821,7 @@ void GraphEngine::launch_exact(const uint4* d_rows, size_t nq, const QueryParams
   uint32_t threads = (bitmaps ? std::min(nq, grid_cap) : nq) <= (size_t)sms ? 512u : (uint32_t)kExactThreads;
   const size_t smem = exact_launch_config(max_size, cfg, threads);
   ExactKernelFn fn = exact_kernel(host_.prop.otype, host_.prop.metric, threads);
-  NGT_CUDA(cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  NGT_CUDA(allow_smem((const void*)fn, device_, smem));
   NGT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)fn, (int)threads, smem));
   size_t grid = std::min<size_t>(nq, (size_t)std::max(1, per_sm) * sms);
   if (bitmaps) {
@@ -884,12 +907,12 @@ void GraphEngine::launch_wide(const uint4* d_rows, size_t nq, const QueryParams*
   NGT_CUDA(cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, device_));
   auto ctas_per_sm = [&](size_t smem) {
     int n = 0;
-    NGT_CUDA(cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     NGT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, (const void*)fn, (int)threads, smem));
     return n;
   };
   size_t smem = wide_kernel_smem_bytes(dev_.row_chunks, cfg);
   if (smem > (size_t)max_smem) throw std::runtime_error("wide search state does not fit in shared memory");
+  NGT_CUDA(allow_smem((const void*)fn, device_, smem));    // and any size up to max_smem
   per_sm = ctas_per_sm(smem);
   // the visited bitmap lies in shared memory where that costs no CTA of an SM (200k x 100
   // cosine, 10,000 queries: 4.21 ms, in global memory 4.39 ms), with 512 threads wherever
@@ -907,7 +930,6 @@ void GraphEngine::launch_wide(const uint4* d_rows, size_t nq, const QueryParams*
   } else {
     cfg.smem_bitmap = 0;
   }
-  NGT_CUDA(cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   size_t grid = std::min<size_t>(nq, (size_t)std::max(1, per_sm) * sms);
   ensure_fast_scratch(scratch, grid, stream);
   NGT_CUDA(cudaMemsetAsync(scratch.work, 0, 4, stream));
@@ -957,7 +979,7 @@ void GraphEngine::launch_fast(const uint4* d_rows, size_t nq, const QueryParams*
   int max_smem = 0, per_sm = 0, sms = 0;
   NGT_CUDA(cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, device_));
   if (smem > (size_t)max_smem) throw std::runtime_error("batched search state does not fit in shared memory");
-  NGT_CUDA(cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  NGT_CUDA(allow_smem((const void*)fn, device_, smem));
   NGT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)fn, kFastThreads, smem));
   NGT_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device_));
   size_t grid = std::min<size_t>((nq + kFastWarps - 1) / kFastWarps, (size_t)std::max(1, per_sm) * sms);
@@ -1111,7 +1133,7 @@ void GraphEngine::search_refined(const void* queries, QueryType qt, size_t nq, s
   const uint32_t P = next_pow2(std::max<uint32_t>((uint32_t)cand.kmax, 2));
   const uint32_t rchunks = host_.rdim_pad / 4;
   const size_t smem = (size_t)rchunks * 16 + (size_t)P * 8;
-  NGT_CUDA(cudaFuncSetAttribute((const void*)rf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  NGT_CUDA(allow_smem((const void*)rf, device_, smem));
   rf<<<(unsigned)std::min<size_t>(nq, (size_t)sms * 8), 256, smem, s>>>(
       d_cand, d_cc, (uint32_t)cand.kmax, d_q, (uint32_t)qdim, static_cast<const uint4*>(d_robj_), rchunks,
       (uint32_t)host_.prop.dimension, host_.robj_rows, d_exact, (uint32_t)nq, P, d_out, (uint32_t)kmax, d_counts);
@@ -1301,8 +1323,7 @@ void GraphEngine::linear_search(const void* queries, QueryType qt, size_t nq, si
   const uint32_t group = std::min<uint32_t>(32, next_pow2(rc));
   int sms = 0;
   NGT_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device_));
-  NGT_CUDA(cudaFuncSetAttribute((const void*)linear_collect_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)(kpow * 8)));
+  NGT_CUDA(allow_smem((const void*)linear_collect_kernel, device_, kpow * 8));
   for (size_t q0 = 0; q0 < nq; q0 += qb) {
     const size_t nb = std::min(qb, nq - q0);
     std::memcpy(h, rows.data() + q0 * rb, nb * rb);
@@ -1386,7 +1407,7 @@ void GraphEngine::search_device_noalloc(void* scratch, size_t scratch_bytes, con
     throw std::runtime_error(m.str());
   }
   ExactKernelFn fn = exact_kernel(host_.prop.otype, host_.prop.metric);
-  NGT_CUDA(cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  NGT_CUDA(allow_smem((const void*)fn, device_, smem));
   int per_sm = 0, sms = 0;
   NGT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)fn, kExactThreads, smem));
   NGT_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device_));
@@ -1496,7 +1517,7 @@ void GraphEngine::qg_search_device(const uint4* d_rows, size_t nq, const QGArgs*
   const size_t smem = qg_kernel_smem_bytes(dev_.row_chunks, qg_.dim, qg_.m, cfg);
   if (smem > (size_t)max_smem) throw std::runtime_error("quantized graph search state does not fit in shared memory");
   QGKernelFn fn = qg_kernel(qg_.m);
-  NGT_CUDA(cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  NGT_CUDA(allow_smem((const void*)fn, device_, smem));
   int per_sm = 0, sms = 0;
   NGT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)fn, kExactThreads, smem));
   NGT_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device_));
@@ -1582,7 +1603,7 @@ void GraphEngine::qg_search_device_relaxed(const uint4* d_rows, size_t nq, const
   int max_smem = 0, per_sm = 0, sms = 0;
   NGT_CUDA(cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, device_));
   if (smem > (size_t)max_smem) throw std::runtime_error("relaxed quantized graph search state does not fit in shared memory");
-  NGT_CUDA(cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  NGT_CUDA(allow_smem((const void*)fn, device_, smem));
   NGT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)fn, (int)kQGWideThreads, smem));
   NGT_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device_));
   const size_t grid = std::min<size_t>(nq, (size_t)std::max(1, per_sm) * sms);
@@ -1852,7 +1873,7 @@ void GraphEngine::qbg_search_device(const uint4* d_rows, size_t nq, const QBGArg
     if (!fn) throw std::runtime_error("too many subspaces in the QBG index");
     const size_t smem = qbg_scan_kernel_smem_bytes(dev_.row_chunks, qb_.dim, qb_.m, max_size);
     if (smem > (size_t)max_smem) throw std::runtime_error("QBG search state does not fit in shared memory");
-    NGT_CUDA(cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    NGT_CUDA(allow_smem((const void*)fn, device_, smem));
     int per_sm = 0;
     NGT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)fn, kExactThreads, smem));
     size_t grid = std::min<size_t>(nq, (size_t)std::max(1, per_sm) * sms);
@@ -1893,7 +1914,7 @@ void GraphEngine::qbg_search_device(const uint4* d_rows, size_t nq, const QBGArg
     }
     if (smem > (size_t)max_smem) throw std::runtime_error("QBG search state does not fit in shared memory");
     QBGKernelFn fn = qbg_kernel(qb_.m);
-    NGT_CUDA(cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    NGT_CUDA(allow_smem((const void*)fn, device_, smem));
     int per_sm = 0;
     NGT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)fn, kExactThreads, smem));
     size_t grid = std::min<size_t>(nq, (size_t)std::max(1, per_sm) * sms);
@@ -1926,7 +1947,7 @@ void GraphEngine::qbg_search_device(const uint4* d_rows, size_t nq, const QBGArg
     const uint32_t P = next_pow2(std::max<uint32_t>(max_size, 2));
     const size_t smem = (size_t)olist_chunks_ * 16 + (size_t)P * 8;
     QBGRefineKernelFn rf = qbg_refine_kernel_for(olist_uint8_);
-    NGT_CUDA(cudaFuncSetAttribute((const void*)rf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    NGT_CUDA(allow_smem((const void*)rf, device_, smem));
     const unsigned grid = (unsigned)std::min<size_t>(nq, (size_t)sms * 8);
     rf<<<grid, 256, smem, stream>>>(d_sout, d_scount, (uint32_t)stride, reinterpret_cast<const float*>(d_rows),
                                     (uint32_t)(dev_.row_chunks * 4), static_cast<const uint4*>(d_olist_),

@@ -8,6 +8,13 @@ namespace ngtg {
 
 struct ExactConfig;
 
+// Lets fn be launched with `bytes` of dynamic shared memory.  The attribute belongs to the
+// function, which every index and thread of the process shares, each with a size of its own:
+// a smaller one set between another thread's setting and its launch would make that launch
+// fail.  So it is always set to the same value, all that the device allows beside the
+// function's static shared memory.
+cudaError_t allow_smem(const void* fn, int device, size_t bytes);
+
 typedef void (*ExactKernelFn)(DevGraph, const uint4*, uint32_t, const QueryParams*, const uint32_t*, ObjDist*,
                               uint32_t*, QueryStats*, uint32_t*, unsigned long long*, ExactConfig);
 typedef void (*LinearKernelFn)(DevGraph, const uint4*, uint32_t, uint32_t, const uint8_t*, float*, uint32_t);

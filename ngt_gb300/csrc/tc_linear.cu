@@ -1560,11 +1560,9 @@ void GraphEngine::linear_search_tc_device(const uint4* d_rows, size_t nq, size_t
   while (group < rc && group < 32) group <<= 1;
   const size_t fin_smem = (size_t)rc * 16 + (size_t)P * 8;
   const uint32_t held = C <= 2048 ? 2048u : cap;           // keys a compaction holds in shared memory
-  TC_CUDA(cudaFuncSetAttribute((const void*)fin, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fin_smem));
-  TC_CUDA(cudaFuncSetAttribute((const void*)tc::tc_first_select_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)(first * 4)));
-  TC_CUDA(cudaFuncSetAttribute((const void*)tc::tc_compact_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)(held * 8)));
+  TC_CUDA(allow_smem((const void*)fin, device_, fin_smem));
+  TC_CUDA(allow_smem((const void*)tc::tc_first_select_kernel, device_, first * 4));
+  TC_CUDA(allow_smem((const void*)tc::tc_compact_kernel, device_, held * 8));
   prepare_score_kernels();
   const uint32_t growth = part_growth(nq, C, cap);
   // the launch sequence (timing: phase events between its parts; R: growth of the parts)
