@@ -1286,9 +1286,11 @@ void GraphEngine::linear_search(const void* queries, QueryType qt, size_t nq, si
   cudaStream_t s = stream_;
   const uint32_t rc = dev_.row_chunks;
   const size_t nrows = host_.nrows, rb = host_.row_bytes();
-  // queries per block: at most 16 MB of distances (or one query's)
-  const size_t qb = std::max<size_t>(1, std::min<size_t>({nq, ((size_t)1 << 22) / nrows, (size_t)65535}));
   const uint32_t kpow = next_pow2((uint32_t)size);
+  // queries per block: at most 16 MB of distances, and 64 MB with all else that a query
+  // takes (on small indexes its 8 KB histogram is the most); one query at least
+  const size_t per = rb + nrows * 4 + kSelBins * 4 + sizeof(LinearSelect) + (size_t)kpow * 8 + kmax * sizeof(ObjDist) + 4;
+  const size_t qb = std::max<size_t>(1, std::min<size_t>({nq, ((size_t)1 << 22) / nrows, kLinearScratchBytes / per}));
   auto al = [](size_t x) { return (x + 255) & ~(size_t)255; };
   // device block: rows | distances | histograms, states | keys | results, counts; the
   // pinned block holds the rows going in and the results and counts coming out

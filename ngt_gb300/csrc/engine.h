@@ -449,8 +449,9 @@ class GraphEngine {
   float sq8_offset_ = 0.f, sq8_scale_ = 1.f;
   FastTuning tuning_;
   DevGraph dev_;
-  // buffers of the exhaustive search, grown on demand and kept (mu_ held): at most about
-  // 115 MB, or one query's distances where those are more
+  // buffers of the exhaustive search, grown on demand and kept (mu_ held): at most 64 MB of
+  // each kind, or one query's where those are more
+  static constexpr size_t kLinearScratchBytes = (size_t)64 << 20;
   struct LinearScratch {
     void* dev = nullptr;
     size_t dev_bytes = 0;

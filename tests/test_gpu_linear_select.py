@@ -55,3 +55,23 @@ def test_selection_leaves_out_what_is_not_finite(tmp_path):
             d = np.where(np.isfinite(x).all(1), x[:, 0], np.inf)
             order = [i for i in np.argsort(d, kind="stable") if np.isfinite(d[i])][:k]
             assert [r.id for r in got] == [i + 1 for i in order]
+
+
+def test_many_queries_over_a_small_index(tmp_path):
+    """The autotuner's ground truth is the exhaustive search of all its sample queries: 65,000
+    over 100 objects run in several blocks, whose buffers stay within the engine's limits (64 MB
+    here and 64 MB of its memory pool) however many queries there are."""
+    import torch
+    from ngt_gb300 import Index
+    from test_gpu_exact_shapes import _index as random_index
+    path = str(tmp_path / "ix")
+    random_index(path, 100, 128, 60, 4, bytes_=True)
+    q = np.random.default_rng(5).integers(0, 60, (65_000, 128)).astype(np.float32)
+    with Index(path, read_only=True) as ix:
+        # the search kernels' own buffers: as large as they get
+        ix.autotune(q[:6000], k=99, epsilon=0.5, recall_floor=1.0)
+        torch.cuda.synchronize()
+        before = torch.cuda.mem_get_info()[0]
+        ix.autotune(q, k=99, epsilon=0.6, recall_floor=1.0)
+        torch.cuda.synchronize()
+        assert before - torch.cuda.mem_get_info()[0] <= 160 << 20
