@@ -94,7 +94,6 @@ constexpr uint32_t epi_warps(uint32_t bn) { return bn == SMALL_BN ? 8 : 16; }
 constexpr uint32_t tc_threads(uint32_t bn) { return 64 + 32 * epi_warps(bn); }   // warp 0 TMA, 1 MMA, 2.. epilogue
 constexpr uint32_t kInvalidKey = 0xff800000u;   // score key of -inf; valid keys are smaller
 constexpr uint64_t kWaitNs = 2000000000ull;     // bound of every wait (2 s)
-constexpr uint32_t kErrorOverflow = 8u;         // bit of the error word: a candidate list overflowed
 constexpr int kDeferQueries = 8;                // filter epilogue: see tc_score_kernel
 
 // Instruction descriptor of tcgen05.mma kind::f16: D fp32 (bits 4-5 = 1), A and
@@ -124,7 +123,7 @@ struct ScoreArgs {
   uint32_t* cand_count;
   uint32_t cap;
   uint32_t* status;                     // bit 1: candidate list overflow
-  uint32_t* error;                      // bit 1: producer wait, 2: MMA wait, 4: epilogue wait ran out (8: overflow)
+  uint32_t* error;                      // bit 1: producer wait, 2: MMA wait, 4: epilogue wait ran out
   const float* qscale;                  // fp8 scores: per-query dequantisation scale (bf16: unused)
 };
 
@@ -853,7 +852,7 @@ constexpr int kCompactThreads = 256;
 __global__ void __launch_bounds__(kCompactThreads)
 tc_compact_kernel(unsigned long long* __restrict__ cand, uint32_t* __restrict__ cand_count, uint32_t cap, uint32_t C,
                   uint32_t held, float* __restrict__ thr, uint32_t* __restrict__ status,
-                  uint32_t* __restrict__ error) {
+                  uint32_t* __restrict__ overflow) {
   extern __shared__ __align__(16) unsigned char smem[];
   unsigned long long* keys = reinterpret_cast<unsigned long long*>(smem);   // held
   __shared__ uint32_t hist[2048];
@@ -864,7 +863,7 @@ tc_compact_kernel(unsigned long long* __restrict__ cand, uint32_t* __restrict__ 
   if (n > cap) {
     if (threadIdx.x == 0) {
       status[q] |= 1u;
-      atomicOr(error, kErrorOverflow);
+      *overflow = 1u;
     }
     n = cap;
   }
@@ -948,7 +947,7 @@ __global__ void __launch_bounds__(kFinalThreads)
 tc_final_kernel(DevGraph g, const uint4* __restrict__ queries, uint32_t q0, const unsigned long long* __restrict__ cand,
                 const uint32_t* __restrict__ cand_count, uint32_t cap, uint32_t C, uint32_t P, uint32_t size,
                 uint32_t group, ObjDist* __restrict__ out, uint32_t kmax, uint32_t* __restrict__ out_count,
-                uint32_t* __restrict__ status, uint32_t* __restrict__ error) {
+                uint32_t* __restrict__ status, uint32_t* __restrict__ overflow) {
   extern __shared__ __align__(16) unsigned char smem[];
   uint4* qv = reinterpret_cast<uint4*>(smem);                                        // row_chunks
   unsigned long long* sel = reinterpret_cast<unsigned long long*>(qv + g.row_chunks);   // P
@@ -1081,7 +1080,7 @@ tc_final_kernel(DevGraph g, const uint4* __restrict__ queries, uint32_t q0, cons
     out_count[q] = kk;
     if (status && cand_count[qi] > cap) {
       status[q] |= 1u;
-      atomicOr(error, kErrorOverflow);
+      *overflow = 1u;
     }
   }
 }
@@ -1139,8 +1138,10 @@ __global__ void tc_rows8_kernel(const float* __restrict__ x, uint32_t nrows, uin
 // Per-query scaled E4M3 query rows [nq_pad][kpad8] and their scales (one warp per
 // query; rows past nq and columns past dpad are zero).
 __global__ void tc_queries8_kernel(const float* __restrict__ rows, uint32_t dpad, uint32_t nq, uint32_t nq_pad,
-                                   uint32_t kpad8, uint8_t* __restrict__ out, float* __restrict__ qscale) {
+                                   uint32_t kpad8, uint8_t* __restrict__ out, float* __restrict__ qscale,
+                                   uint32_t* __restrict__ overflow) {
   const uint32_t lane = threadIdx.x & 31;
+  if (overflow && blockIdx.x == 0 && threadIdx.x == 0) *overflow = 0u;
   for (uint32_t q = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5); q < nq_pad;
        q += gridDim.x * (blockDim.x / 32)) {
     const float* xr = rows + (size_t)q * dpad;
@@ -1159,7 +1160,8 @@ __global__ void tc_queries8_kernel(const float* __restrict__ rows, uint32_t dpad
 
 // bf16 query rows [nq_pad][kpad]; rows past nq and columns past dpad are zero.
 __global__ void tc_queries_kernel(const float* __restrict__ rows, uint32_t dpad, uint32_t nq, uint32_t nq_pad,
-                                  uint32_t kpad, __nv_bfloat16* __restrict__ out) {
+                                  uint32_t kpad, __nv_bfloat16* __restrict__ out, uint32_t* __restrict__ overflow) {
+  if (overflow && blockIdx.x == 0 && threadIdx.x == 0) *overflow = 0u;
   const size_t n = (size_t)nq_pad * kpad;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
     const uint32_t q = (uint32_t)(i / kpad), c = (uint32_t)(i % kpad);
@@ -1261,7 +1263,7 @@ struct TcState {
   // scratch, grown on demand
   void* scratch = nullptr;
   size_t scratch_bytes = 0;
-  uint32_t* error = nullptr;
+  uint32_t* error = nullptr;       // [0] pipeline waits that ran out, [1] a candidate list of this search overflowed
   // phase timing of the last query batch: dense part + selection, filtered
   // part (the score kernel over the remaining rows), final re-rank
   cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
@@ -1311,9 +1313,9 @@ void GraphEngine::ensure_tc_rows() {
   TC_CUDA(cudaMalloc(&s->rows, nrows * s->kpad * 2));
   TC_CUDA(cudaMalloc(&s->scale, nrows * 4));
   TC_CUDA(cudaMalloc(&s->bias, nrows * 4));
-  TC_CUDA(cudaMalloc(&s->error, 4));
+  TC_CUDA(cudaMalloc(&s->error, 8));
   for (cudaEvent_t& e : s->ev) TC_CUDA(cudaEventCreate(&e));
-  TC_CUDA(cudaMemsetAsync(s->error, 0, 4, stream_));
+  TC_CUDA(cudaMemsetAsync(s->error, 0, 8, stream_));
   const unsigned blocks = (unsigned)((nrows + 7) / 8);
   tc::tc_rows_kernel<<<blocks, 256, 0, stream_>>>(static_cast<const float*>(d_objects_), (uint32_t)nrows, dpad,
                                                   s->kpad, tc::row_mode(host_.prop.metric), s->rows, s->scale,
@@ -1444,16 +1446,16 @@ uint32_t part_growth(size_t nq, size_t C, uint32_t cap) {
 }
 
 // Waits for the stream; throws when a pipeline wait ran out; true when a candidate list
-// overflowed.
+// of the last search overflowed (the word is cleared by each search's first kernel).
 bool check_error(const TcState& st, cudaStream_t s) {
-  uint32_t err = 0;
-  TC_CUDA(cudaMemcpyAsync(&err, st.error, 4, cudaMemcpyDeviceToHost, s));
+  uint32_t err[2] = {0, 0};
+  TC_CUDA(cudaMemcpyAsync(err, st.error, 8, cudaMemcpyDeviceToHost, s));
   TC_CUDA(cudaStreamSynchronize(s));
-  if (err) TC_CUDA(cudaMemsetAsync(st.error, 0, 4, s));
-  if (err & ~tc::kErrorOverflow) {
-    throw std::runtime_error("tensor-core score kernel: a pipeline wait ran out (code " + std::to_string(err) + ")");
+  if (err[0]) {
+    TC_CUDA(cudaMemsetAsync(st.error, 0, 4, s));
+    throw std::runtime_error("tensor-core score kernel: a pipeline wait ran out (code " + std::to_string(err[0]) + ")");
   }
-  return err != 0;
+  return err[1] != 0;
 }
 
 }  // namespace
@@ -1473,7 +1475,7 @@ void GraphEngine::tc_scores_device(const uint4* d_rows, size_t nq, float* d_scor
   const size_t nq_pad = (nq + bn - 1) / bn * bn;
   TC_CUDA(cudaMallocAsync(&qb, nq_pad * st.kpad * 2, stream));
   tc::tc_queries_kernel<<<1024, 256, 0, stream>>>(reinterpret_cast<const float*>(d_rows), host_.dpad, (uint32_t)nq,
-                                                  (uint32_t)nq_pad, st.kpad, qb);
+                                                  (uint32_t)nq_pad, st.kpad, qb, nullptr);
   TC_CUDA(cudaGetLastError());
   CUtensorMap mapB = tc::make_map(qb, nq_pad, st.kpad, bn);
   tc::ScoreArgs a{};
@@ -1574,13 +1576,14 @@ void GraphEngine::linear_search_tc_device(const uint4* d_rows, size_t nq, size_t
     const uint32_t nbpad = (nb + bn - 1) / bn * bn;
     if (timing) TC_CUDA(cudaEventRecord(st.ev[0], stream));
     const float* qrows = reinterpret_cast<const float*>(d_rows) + q0 * host_.dpad;
+    uint32_t* fresh = q0 == 0 ? st.error + 1 : nullptr;      // no list of this search has overflowed yet
     CUtensorMap mapB, mapBh;
     if (fp8) {
-      tc::tc_queries8_kernel<<<1024, 256, 0, stream>>>(qrows, host_.dpad, nb, nbpad, st.kpad8, qbuf8, qscale);
+      tc::tc_queries8_kernel<<<1024, 256, 0, stream>>>(qrows, host_.dpad, nb, nbpad, st.kpad8, qbuf8, qscale, fresh);
       mapB = tc::make_map8(qbuf8, nbpad, st.kpad8, bn);
       if (pair) mapBh = tc::make_map8(qbuf8, nbpad, st.kpad8, tc::BN / 2);
     } else {
-      tc::tc_queries_kernel<<<1024, 256, 0, stream>>>(qrows, host_.dpad, nb, nbpad, st.kpad, qbuf);
+      tc::tc_queries_kernel<<<1024, 256, 0, stream>>>(qrows, host_.dpad, nb, nbpad, st.kpad, qbuf, fresh);
       mapB = tc::make_map(qbuf, nbpad, st.kpad, bn);
       if (pair) mapBh = tc::make_map(qbuf, nbpad, st.kpad, tc::BN / 2);
     }
@@ -1641,8 +1644,7 @@ void GraphEngine::linear_search_tc_device(const uint4* d_rows, size_t nq, size_t
       launches_++;
       if (end < nrows) {
         tc::tc_compact_kernel<<<nb, tc::kCompactThreads, held * 8, stream>>>(cand, ccount, cap, (uint32_t)C, held, thr,
-                                                                             d_status + q0,
-                                                            st.error);
+                                                                             d_status + q0, st.error + 1);
         TC_CUDA(cudaGetLastError());
         launches_++;
       }
@@ -1650,7 +1652,7 @@ void GraphEngine::linear_search_tc_device(const uint4* d_rows, size_t nq, size_t
     }
     if (timing) TC_CUDA(cudaEventRecord(st.ev[2], stream));
     fin<<<nb, tc::kFinalThreads, fin_smem, stream>>>(dev_, d_rows, (uint32_t)q0, cand, ccount, cap, (uint32_t)C, P,
-                                       (uint32_t)size, group, d_out, (uint32_t)kmax, d_counts, d_status, st.error);
+                                       (uint32_t)size, group, d_out, (uint32_t)kmax, d_counts, d_status, st.error + 1);
     TC_CUDA(cudaGetLastError());
     if (timing) TC_CUDA(cudaEventRecord(st.ev[3], stream));
     launches_++;

@@ -69,3 +69,42 @@ def test_a_part_beyond_the_list_still_reports_overflow(tmp_path):
     with _index(tmp_path, x) as ix:
         ids, ds, cnt, st = ix.linear_search_tc(np.zeros((3, 2), np.float32), k=10, candidates=64)
         assert (st & 1 != 0).all()
+
+
+def test_an_overflow_in_a_replayed_capture_is_not_the_next_search_s(tmp_path):
+    """A search inside a caller's capture cannot read its overflow word; a later search that
+    overflows no list runs once, as it does on a fresh index."""
+    import torch
+    n = 120_000
+    x = np.zeros((n, 2), np.float32)
+    x[:, 0] = np.arange(n, 0, -1) // 2                           # comes nearer to 0, farther from n
+    with _index(tmp_path, x) as ix:
+        def buffers(v):
+            rows = torch.from_numpy(ix.convert_queries(v)).cuda()
+            return (rows, torch.zeros((3, 10, 2), dtype=torch.int32, device="cuda"),
+                    torch.zeros(3, dtype=torch.int32, device="cuda"), torch.zeros(3, dtype=torch.int32, device="cuda"))
+
+        def search(b, stream=None):
+            ix._check(ix._lib.ngtgpu_linear_search_tc_ex(ix._index, b[0].data_ptr(), 3, 10, 64, 0, 0, b[1].data_ptr(),
+                                                         10, b[2].data_ptr(), b[3].data_ptr(), stream, ix._err))
+
+        near, far = buffers(np.zeros((3, 2), np.float32)), buffers(np.full((3, 2), n, np.float32))
+        search(far)
+        torch.cuda.synchronize()
+        assert (far[3] == 0).all()
+        first = ix.kernel_launches()
+        search(far)
+        once = ix.kernel_launches() - first
+        want = far[1].clone()
+        side = torch.cuda.Stream()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=side, capture_error_mode="thread_local"):
+            search(near, side.cuda_stream)
+        graph.replay()
+        torch.cuda.synchronize()
+        assert (near[3] & 1 != 0).all()
+        before = ix.kernel_launches()
+        search(far)
+        torch.cuda.synchronize()
+        assert ix.kernel_launches() - before == once
+        assert (far[3] == 0).all() and torch.equal(far[1], want)
