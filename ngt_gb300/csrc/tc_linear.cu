@@ -125,6 +125,7 @@ struct ScoreArgs {
   uint32_t* status;                     // bit 1: candidate list overflow
   uint32_t* error;                      // bit 1: producer wait, 2: MMA wait, 4: epilogue wait ran out
   const float* qscale;                  // fp8 scores: per-query dequantisation scale (bf16: unused)
+  const uint32_t* skip;                 // not null and not 0: the search will be done again, nothing is scored
 };
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -346,6 +347,7 @@ tc_score_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
   constexpr uint32_t NST = kPair ? STAGES2 : kBN == SMALL_BN ? STAGES_SMALL : STAGES;
   constexpr uint32_t SBYTES = kPair ? STAGE2_BYTES : kBN == SMALL_BN ? STAGE_SMALL_BYTES : STAGE_BYTES;
   constexpr uint32_t EPI_WARPS = epi_warps(kBN), EPI_PARTS = EPI_WARPS / 4, TMEM_COLS = 2 * kBN;
+  if (a.skip && *a.skip) return;               // written by earlier launches only: alike in the grid
   extern __shared__ __align__(1024) unsigned char dsmem[];
   __shared__ __align__(8) uint64_t bar_full[MAX_STAGES], bar_empty[MAX_STAGES], bar_tfull[2], bar_tempty[2], bar_drain;
   __shared__ uint32_t tmem_base_sh;
@@ -789,7 +791,9 @@ constexpr int kSelectThreads = 512;
 __global__ void __launch_bounds__(kSelectThreads)
 tc_first_select_kernel(const float* __restrict__ dense, uint32_t ld, uint32_t nrows, uint32_t C,
                        float* __restrict__ thr, unsigned long long* __restrict__ cand,
-                       uint32_t* __restrict__ cand_count, uint32_t cap, uint32_t row_offset) {
+                       uint32_t* __restrict__ cand_count, uint32_t cap, uint32_t row_offset,
+                       const uint32_t* skip) {
+  if (skip && *skip) return;
   extern __shared__ __align__(16) unsigned char smem[];
   uint32_t* keys = reinterpret_cast<uint32_t*>(smem);                       // nrows score keys
   __shared__ uint32_t hist[2048];
@@ -947,7 +951,7 @@ __global__ void __launch_bounds__(kFinalThreads)
 tc_final_kernel(DevGraph g, const uint4* __restrict__ queries, uint32_t q0, const unsigned long long* __restrict__ cand,
                 const uint32_t* __restrict__ cand_count, uint32_t cap, uint32_t C, uint32_t P, uint32_t size,
                 uint32_t group, ObjDist* __restrict__ out, uint32_t kmax, uint32_t* __restrict__ out_count,
-                uint32_t* __restrict__ status, uint32_t* __restrict__ overflow) {
+                uint32_t* __restrict__ status, uint32_t* overflow, uint32_t again) {
   extern __shared__ __align__(16) unsigned char smem[];
   uint4* qv = reinterpret_cast<uint4*>(smem);                                        // row_chunks
   unsigned long long* sel = reinterpret_cast<unsigned long long*>(qv + g.row_chunks);   // P
@@ -959,8 +963,11 @@ tc_final_kernel(DevGraph g, const uint4* __restrict__ queries, uint32_t q0, cons
   uint32_t n = cand_count[qi];
   if (n > cap) n = cap;
   const unsigned long long* src = cand + (size_t)qi * cap;
-  if (threadIdx.x == 0) sh_m = 0;
+  // a search that will be done again (a list overflowed, maybe in this very launch) ends here
+  if (threadIdx.x == 0) sh_m = again && *(const volatile uint32_t*)overflow ? ~0u : 0u;
   __syncthreads();
+  if (sh_m) return;
+  __syncthreads();                             // sh_m is read before it counts
   unsigned long long kth = ~0ull;
   if (n > C) {
     unsigned long long mn = ~0ull, mx = 0ull;
@@ -1170,7 +1177,7 @@ __global__ void tc_queries_kernel(const float* __restrict__ rows, uint32_t dpad,
 }
 
 typedef void (*FinalFn)(DevGraph, const uint4*, uint32_t, const unsigned long long*, const uint32_t*, uint32_t,
-                        uint32_t, uint32_t, uint32_t, uint32_t, ObjDist*, uint32_t, uint32_t*, uint32_t*, uint32_t*);
+                        uint32_t, uint32_t, uint32_t, uint32_t, ObjDist*, uint32_t, uint32_t*, uint32_t*, uint32_t*, uint32_t);
 
 template <bool kTies>
 FinalFn final_kernel_t(Metric m) {
@@ -1264,6 +1271,10 @@ struct TcState {
   void* scratch = nullptr;
   size_t scratch_bytes = 0;
   uint32_t* error = nullptr;       // [0] pipeline waits that ran out, [1] a candidate list of this search overflowed
+  // After a list overflowed in fast-growing parts the rows may lie in an order that makes it
+  // overflow every time, so the next `doubling_calls` searches take doubling parts at once:
+  // 1, then 2, 4 .. 64 while the tries between them overflow too, none after one that does not.
+  uint32_t backoff = 0, doubling_calls = 0;
   // phase timing of the last query batch: dense part + selection, filtered
   // part (the score kernel over the remaining rows), final re-rank
   cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
@@ -1431,6 +1442,8 @@ void launch_scores(const TcState& st, const CUtensorMap& mapB, const CUtensorMap
 // launches in 8 parts, 280 us in 3).  A quarter of the list's capacity is not exceeded on rows
 // in no particular order; a list that overflows all the same (rows sorted by nearness) has
 // the whole search done again with R = 1, as searches inside a caller's capture always are.
+// The launches that follow the overflow return at once, and the searches after it do not try
+// again for a while (TcState::backoff).
 uint32_t part_growth(size_t nq, size_t C, uint32_t cap) {
   uint32_t best = 1;
   double least = 0.0;
@@ -1566,7 +1579,24 @@ void GraphEngine::linear_search_tc_device(const uint4* d_rows, size_t nq, size_t
   TC_CUDA(allow_smem((const void*)tc::tc_first_select_kernel, device_, first * 4));
   TC_CUDA(allow_smem((const void*)tc::tc_compact_kernel, device_, held * 8));
   prepare_score_kernels();
-  const uint32_t growth = part_growth(nq, C, cap);
+  // fast-growing parts, but for the calls after one of their lists overflowed
+  uint32_t growth = part_growth(nq, C, cap);
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  TC_CUDA(cudaStreamIsCapturing(stream, &capture));
+  if (capture != cudaStreamCaptureStatusNone) {
+    growth = 1;
+  } else if (growth > 1 && tc_->doubling_calls > 0) {
+    tc_->doubling_calls--;
+    growth = 1;
+  }
+  // whether the search has to be done again with doubling parts
+  auto overflowed = [&] {
+    const bool over = check_error(st, stream);
+    if (growth == 1) return false;
+    tc_->backoff = over ? std::min<uint32_t>(64, std::max<uint32_t>(1, 2 * tc_->backoff)) : 0u;
+    tc_->doubling_calls = tc_->backoff;
+    return over;
+  };
   // the launch sequence (timing: phase events between its parts; R: growth of the parts)
   auto enqueue = [&](bool timing, uint32_t R) {
   TC_CUDA(cudaMemsetAsync(d_status, 0, nq * 4, stream));
@@ -1597,6 +1627,7 @@ void GraphEngine::linear_search_tc_device(const uint4* d_rows, size_t nq, size_t
     a.row_bias = st.bias;
     a.present = d_present_;
     a.error = st.error;
+    a.skip = R > 1 ? st.error + 1 : nullptr;
     // dense first part
     a.row_begin = rb;
     a.row_end = r0;
@@ -1604,7 +1635,7 @@ void GraphEngine::linear_search_tc_device(const uint4* d_rows, size_t nq, size_t
     a.dense_ld = (uint32_t)first;
     launch_scores(st, mapB, half, a, true, stream, sms, fp8);
     tc::tc_first_select_kernel<<<nb, tc::kSelectThreads, first * 4, stream>>>(dense, (uint32_t)first, r0 - rb, (uint32_t)C, thr,
-                                                               cand, ccount, cap, rb);
+                                                               cand, ccount, cap, rb, a.skip);
     TC_CUDA(cudaGetLastError());
     launches_ += 3;
     if (timing) TC_CUDA(cudaEventRecord(st.ev[1], stream));
@@ -1652,22 +1683,18 @@ void GraphEngine::linear_search_tc_device(const uint4* d_rows, size_t nq, size_t
     }
     if (timing) TC_CUDA(cudaEventRecord(st.ev[2], stream));
     fin<<<nb, tc::kFinalThreads, fin_smem, stream>>>(dev_, d_rows, (uint32_t)q0, cand, ccount, cap, (uint32_t)C, P,
-                                       (uint32_t)size, group, d_out, (uint32_t)kmax, d_counts, d_status, st.error + 1);
+                                       (uint32_t)size, group, d_out, (uint32_t)kmax, d_counts, d_status, st.error + 1,
+                                       R > 1 ? 1u : 0u);
     TC_CUDA(cudaGetLastError());
     if (timing) TC_CUDA(cudaEventRecord(st.ev[3], stream));
     launches_++;
   }
   };
-  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-  TC_CUDA(cudaStreamIsCapturing(stream, &capture));
   if (!tc_graphs_ || capture != cudaStreamCaptureStatusNone) {
     // launched directly (also into a capture the caller runs on this stream)
-    if (capture != cudaStreamCaptureStatusNone) {
-      enqueue(false, 1);
-      return;
-    }
-    enqueue(true, growth);
-    if (check_error(st, stream) && growth > 1) {
+    enqueue(capture == cudaStreamCaptureStatusNone, growth);
+    if (capture != cudaStreamCaptureStatusNone) return;
+    if (overflowed()) {
       enqueue(true, 1);
       check_error(st, stream);
     }
@@ -1680,7 +1707,7 @@ void GraphEngine::linear_search_tc_device(const uint4* d_rows, size_t nq, size_t
                                         (uint64_t)(uintptr_t)d_out, kmax, (uint64_t)(uintptr_t)d_counts,
                                         (uint64_t)(uintptr_t)d_status,
                                         (uint64_t)fp8 | (uint64_t)fp64_ties << 1 | (uint64_t)pair << 2, rb, nrows,
-                                        first, (uint64_t)(uintptr_t)tc_->scratch, tc_->scratch_bytes, 0, 0};
+                                        first, (uint64_t)(uintptr_t)tc_->scratch, tc_->scratch_bytes, growth, 0};
   TcState::Graph* g = nullptr;
   for (auto& x : tc_->graphs)
     if (x.key == key) g = &x;
@@ -1713,7 +1740,7 @@ void GraphEngine::linear_search_tc_device(const uint4* d_rows, size_t nq, size_t
   TC_CUDA(cudaGraphLaunch(g->exec, stream));
   TC_CUDA(cudaEventRecord(st.ev[3], stream));
   launches_ += g->launches;
-  if (check_error(st, stream) && growth > 1) {
+  if (overflowed()) {
     enqueue(false, 1);
     TC_CUDA(cudaEventRecord(st.ev[3], stream));
     check_error(st, stream);

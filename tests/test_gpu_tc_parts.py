@@ -108,3 +108,38 @@ def test_an_overflow_in_a_replayed_capture_is_not_the_next_search_s(tmp_path):
         torch.cuda.synchronize()
         assert ix.kernel_launches() - before == once
         assert (far[3] == 0).all() and torch.equal(far[1], want)
+
+
+def test_sorted_rows_are_not_searched_twice_every_time(tmp_path):
+    """Where fast-growing parts overflow, the next searches take doubling parts at once: 1 of
+    them, then 2, 4 ..; a search whose lists hold ends that."""
+    n = 150_000
+    rng = np.random.default_rng(3)
+    x = rng.integers(90, 100, (n, 4)).astype(np.float32)
+    row, near = 8192 - 1, 80
+    while row < n:
+        x[row:row + 5000] = rng.integers(near - 10, near, (min(5000, n - row), 4))
+        row, near = 2 * (row + 1) - 1, near - 15
+    toward = rng.integers(0, 3, (40, 4)).astype(np.float32)      # nearer and nearer rows
+    away = np.full((40, 4), 95, np.float32)                      # the first rows are the nearest
+    for graphs in (False, True):
+        with _index(tmp_path / str(graphs), x) as ix:
+            pi, pd = _plain(ix, toward, 10)
+            ix.set_tc_graphs(graphs)
+
+            def launches(q):
+                before = ix.kernel_launches()
+                ids, ds, cnt, st = ix.linear_search_tc(q, k=10, candidates=64)
+                assert (st == 0).all() and (cnt == 10).all()
+                if q is toward:
+                    assert np.array_equal(ids, pi) and np.array_equal(ds, pd)
+                return ix.kernel_launches() - before
+
+            launches(away)                                       # converts the rows too
+            fast = launches(away)
+            twice, once = launches(toward), launches(toward)
+            assert fast < once and twice == fast + once
+            assert [launches(toward) for _ in range(3)] == [twice, once, once]
+            assert [launches(toward) for _ in range(5)] == [twice] + [once] * 4
+            assert launches(away) == fast                        # a try that holds: all is as at first
+            assert [launches(toward) for _ in range(2)] == [twice, once]
