@@ -2,10 +2,9 @@
 //
 // For one index, result size and epsilon it times a fixed list of candidate
 // configurations -- the warp-per-query kernel with its row pipelines and register
-// budgets, the CTA-per-query kernel with its CTA sizes, staged rows and parents per
-// step -- on a sample of the caller's queries (device resident, CUDA events, median
-// of three launches), and keeps the fastest whose tie-aware recall@k against the
-// exact answer (the index's exhaustive search) is at least a floor: the caller's, or
+// budgets, the CTA-per-query kernel with its CTA sizes and parents per step -- on a
+// sample of the caller's queries (device resident, CUDA events, median of three
+// launches), and keeps the fastest whose tie-aware recall@k against the exact answer (the index's exhaustive search) is at least a floor: the caller's, or
 // (floor < 0) the exact-order kernel's own recall at the same epsilon, i.e. the
 // reference's.  With epsilon < 0 each configuration runs at the smallest epsilon of
 // a sweep that reaches the floor, and the epsilon becomes part of the choice.  The

@@ -376,4 +376,19 @@ struct TreeSpace {
 };
 __device__ __forceinline__ uint32_t key_id(unsigned long long k) { return (uint32_t)k; }
 
+// Ranks of the m <= T unique keys in[0..m), written sorted to out, by the whole CTA:
+// as many threads per key as the CTA has to spare (at most 8) split the comparisons.
+template <int T>
+__device__ __forceinline__ void rank_sort_split(const unsigned long long* in, unsigned long long* out, uint32_t m) {
+  uint32_t split = 1;
+  while (split < 8 && m * split * 2 <= (uint32_t)T) split *= 2;
+  const uint32_t i = threadIdx.x / split, sub = threadIdx.x & (split - 1);
+  const unsigned long long k = i < m ? in[i] : 0ull;
+  uint32_t r = 0;
+  if (i < m)
+    for (uint32_t j = sub; j < m; j += split) r += in[j] < k ? 1u : 0u;
+  for (uint32_t off = 1; off < split; off <<= 1) r += __shfl_xor_sync(0xffffffffu, r, off);
+  if (i < m && sub == 0) out[r] = k;
+}
+
 }  // namespace ngtg

@@ -901,7 +901,7 @@ void GraphEngine::launch_wide(const uint4* d_rows, size_t nq, const QueryParams*
   cfg.bitmap_words = ((host_.nrows + 31) / 32 + 3) / 4 * 4;
   cfg.max_iters = 1u << 22;
   cfg.spill_cap = kSpillCapacity;
-  // default: visited bitmaps kept in L2, staged rows streamed through it
+  // default: visited bitmaps kept in L2, search rows streamed through it
   cfg.l2_policy = tuning_.l2_policy ? tuning_.l2_policy - 1 : 2u;
   int max_smem = 0, per_sm = 0;
   NGT_CUDA(cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, device_));

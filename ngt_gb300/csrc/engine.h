@@ -47,8 +47,8 @@ enum class QueryType { Float32 = 0, Float64 = 1, Uint8 = 2, Float16 = 3 };
 // Exact: reference-order search, one query per CTA (results equal the reference's).
 // Fast: batched warp-per-query search on bf16 rows (float objects) or the native
 //       rows (other types), with an exact re-rank.  FastFp32: the same on fp32 rows.
-// Wide: the batched search with one query per CTA (rows of an iteration staged in
-//       shared memory at once), for low per-query latency.
+// Wide: the batched search with one query per CTA (all rows of an iteration in flight
+//       at once), for low per-query latency and for large batches.
 enum class Kernel { Exact = 0, Fast = 1, FastFp32 = 2, Wide = 3 };
 
 // Knobs of the batched kernel (0 = automatic).
@@ -59,8 +59,8 @@ struct FastTuning {
   uint32_t rows_in_flight = 0; // rows per lane group in flight in the distance loop (2, 4, 6 or 8)
   uint32_t ctas_per_sm = 0;    // register budget of the instantiation (4..8)
   uint32_t nbr_cap = 0;        // neighbour slots per iteration (power of two >= 256)
-  uint32_t cta_threads = 0;    // wide kernel: threads per CTA (128 or 256)
-  uint32_t stage_kb = 0;       // wide kernel: shared memory for staged rows (KB)
+  uint32_t cta_threads = 0;    // wide kernel: threads per CTA (64, 128 or 256; 0: by the number of queries)
+  uint32_t stage_kb = 0;       // no effect (the caller's value is kept, and old tuning caches have one)
   uint32_t l2_policy = 0;      // wide kernel: 0 automatic, else WideConfig::l2_policy + 1
   uint32_t search_rows = 0;    // wide kernel, float objects: 0 automatic (8-bit when lossless, else bf16),
                                // 1 bf16, 2 8-bit codes

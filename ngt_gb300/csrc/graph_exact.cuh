@@ -9,9 +9,11 @@
 //
 // Why the results are the reference's, not just close to them:
 //   * The neighbours of the expanded node are filtered against the visited set
-//     in edge order and their distances computed in parallel; the result-set
-//     updates (the only order-dependent step) are then replayed sequentially by
-//     one warp in edge order, with the reference's push / push_pop semantics.
+//     in edge order and their distances computed in parallel.  The result-set
+//     updates are the only order-dependent step: what the reference's sequence of
+//     push / push_pop leaves is merged at once (merge_results); where the order
+//     decides (epsilon < 0, negative distances, a tie at the last result) one warp
+//     replays them one by one in edge order.
 //   * The candidate queue only needs the set of entries <= explorationRadius:
 //     the radius never grows, the loop stops at the first popped entry above it,
 //     so pushing a chunk's survivors after the chunk (against the radius reached
@@ -22,13 +24,14 @@
 //   * The queue has two tiers: the best `ccap` entries sorted in shared memory
 //     and an unsorted overflow tier in global memory whose entries are all
 //     larger than every shared-memory entry.  When the shared list drains, the
-//     overflow's live entries (<= explorationRadius) are filtered, the ccap
-//     smallest picked by an exact radix select over the 64-bit keys, sorted, and
-//     moved back.  Pops therefore follow the reference's order exactly.
+//     overflow's live entries (<= explorationRadius) are filtered and the smallest
+//     of them, up to the edge of a radix bin that fills at least half the list,
+//     sorted and moved back (exact_refill).  Pops therefore follow the reference's
+//     order exactly.
 // The only limit that can make a query inexact is the overflow tier's capacity
 // (reported in QueryStats::status).  The visited set never loses entries: it
-// starts as a hash table in shared memory and moves to a per-CTA bitmap in
-// global memory when the table is half full.
+// is a bitmap in shared memory where that fits, else a hash table there that moves
+// to a per-CTA bitmap in global memory when it is half full.
 #pragma once
 #include <cfloat>
 #include <type_traits>
@@ -207,21 +210,6 @@ __device__ __forceinline__ void prefetch_row(const uint4* row, uint32_t rc) {
 #pragma unroll
   for (uint32_t c = 0; c < 64; c += 8)
     if (c < rc) asm volatile("prefetch.global.L2 [%0];" ::"l"(row + c));
-}
-
-// Ranks of the m <= T unique keys in[0..m), written sorted to out, by the whole CTA:
-// as many threads per key as the CTA has to spare (at most 8) split the comparisons.
-template <int T>
-__device__ __forceinline__ void rank_sort_split(const unsigned long long* in, unsigned long long* out, uint32_t m) {
-  uint32_t split = 1;
-  while (split < 8 && m * split * 2 <= (uint32_t)T) split *= 2;
-  const uint32_t i = threadIdx.x / split, sub = threadIdx.x & (split - 1);
-  const unsigned long long k = i < m ? in[i] : 0ull;
-  uint32_t r = 0;
-  if (i < m)
-    for (uint32_t j = sub; j < m; j += split) r += in[j] < k ? 1u : 0u;
-  for (uint32_t off = 1; off < split; off <<= 1) r += __shfl_xor_sync(0xffffffffu, r, off);
-  if (i < m && sub == 0) out[r] = k;
 }
 
 // A round's updates of the result set res (n = s.nres keys, ascending) as one merge: the

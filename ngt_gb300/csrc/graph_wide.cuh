@@ -4,7 +4,7 @@
 // re-rank of the best candidates), with every phase of an iteration spread
 // over the CTA so that one query moves many rows at once:
 //   * the P parents' edge slots are read, filtered against the query's
-//     visited bitmap and compacted by all threads of the CTA (128 or 256);
+//     visited bitmap and compacted by all threads of the CTA (64 to 512);
 //   * the new neighbours' search rows (bf16 or 8-bit copies of float objects, or
 //     the objects themselves) are loaded straight into registers, several rows per
 //     lane group in flight, and scored; a row within the limit goes to the new
@@ -13,7 +13,7 @@
 //     when there are few, else after a sort) plus its rank in the list; keys land
 //     in a second list buffer.
 // A step takes four CTA barriers: parents chosen, new ids gathered, rows scored,
-// list merged (with a shared-memory row stage, two more per 64 rows).
+// list merged.
 // One warp (warp 0) owns the control decisions (parent selection, the refill
 // from the spill tier), exactly as the warp-per-query kernel makes them.
 // Per-query latency is set by a few memory round trips per iteration instead of
@@ -29,7 +29,6 @@
 namespace ngtg {
 
 constexpr int kWideMaxThreads = 512;
-constexpr int kWideMaxWarps = kWideMaxThreads / 32;
 
 struct WideConfig {
   uint32_t list_cap;       // L: power of two
@@ -216,21 +215,6 @@ __device__ __forceinline__ uint32_t group_sums(uint32_t (&v)[KR], int SG, int la
     for (; off > 0; off >>= 1) v[0] = add(v[0], __shfl_xor_sync(0xffffffffu, v[0], off));
   }
   return first;
-}
-
-// The m <= T unique keys in[0..m) sorted to out by their ranks, several threads per key
-// where the CTA has them to spare.
-template <int T>
-__device__ __forceinline__ void rank_sort_keys(const unsigned long long* in, unsigned long long* out, uint32_t m) {
-  uint32_t split = 1;
-  while (split < 8 && m * split * 2 <= (uint32_t)T) split *= 2;
-  const uint32_t i = threadIdx.x / split, sub = threadIdx.x & (split - 1);
-  const unsigned long long k = i < m ? in[i] : 0ull;
-  uint32_t r = 0;
-  if (i < m)
-    for (uint32_t j = sub; j < m; j += split) r += in[j] < k ? 1u : 0u;
-  for (uint32_t off = 1; off < split; off <<= 1) r += __shfl_xor_sync(0xffffffffu, r, off);
-  if (i < m && sub == 0) out[r] = k;
 }
 
 // T: threads per CTA (64, 128, 256 or 512), one query per CTA.
@@ -793,7 +777,7 @@ graph_search_wide_kernel(DevGraph g, const uint4* __restrict__ srows, const uint
       const unsigned long long* nk = nkey;
       if (!by_count) {
         if (kept <= (uint32_t)T) {
-          rank_sort_keys<T>(nkey, nsorted, kept);
+          rank_sort_split<T>(nkey, nsorted, kept);
           nk = nsorted;
           __syncthreads();
         } else {

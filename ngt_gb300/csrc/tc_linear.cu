@@ -18,7 +18,8 @@
 //      (cp.async.bulk.tensor, 128-byte swizzle) through a 4-stage mbarrier
 //      pipeline, accumulators double-buffered in TMEM (2 x 256 columns) and
 //      read back with tcgen05.ld by sixteen epilogue warps (four per TMEM lane
-//      quadrant).  The first `first_rows` rows are written out densely; on the
+//      quadrant); up to 64 queries take N = 64, 8 stages, 2 x 64 columns and
+//      eight epilogue warps.  The first `first_rows` rows are written out densely; on the
 //      remaining rows, taken in growing parts (part_growth), the epilogue keeps
 //      only scores that beat the query's threshold, and tc_compact_kernel cuts
 //      each list back to the C best and raises the threshold between two parts.
@@ -38,7 +39,8 @@
 //
 // The result equals the plain linear search whenever the true `size` nearest
 // rows are among the C best approximate scores; the candidate oversampling C
-// is the caller's choice.  A query whose candidate list overflowed reports
+// is the caller's choice.  Where a candidate list overflows in fast-growing parts the
+// search is done again with doubling ones; a query whose list overflows then reports
 // status bit 1.
 #include <cuda.h>
 #include <cudaTypedefs.h>
