@@ -230,7 +230,7 @@ __device__ __forceinline__ uint32_t group_sums(uint32_t (&v)[KR], int SG, int la
 // buffers: 1.80 -> 1.0 ms (packed lanes, three CTAs per SM instead of two).  Not kept:
 // prefetching a step's rows into L2 when they are gathered (5 % slower), 1,024 threads (8 %
 // slower than 512), seven and eight CTAs an SM (10 and 24 % slower: their visited bitmaps of
-// 125 KB no longer fit L2).
+// 125 KB no longer fit L2; eight on 200k x 64, bitmaps of 25 KB, 10 %).
 template <ObjType ST, ObjType OT, Metric M, int T>
 __global__ void __launch_bounds__(T, T == 64 ? 10 : T == 128 ? 6 : T == 256 ? 3 : 1)
 graph_search_wide_kernel(DevGraph g, const uint4* __restrict__ srows, const uint4* __restrict__ queries,
