@@ -1629,7 +1629,8 @@ void GraphEngine::linear_search_tc_device(const uint4* d_rows, size_t nq, size_t
     a.row_bias = st.bias;
     a.present = d_present_;
     a.error = st.error;
-    a.skip = R > 1 ? st.error + 1 : nullptr;
+    // no list has overflowed before the first compaction, so the launches up to it do not ask
+    a.skip = R > 1 && q0 > 0 ? st.error + 1 : nullptr;
     // dense first part
     a.row_begin = rb;
     a.row_end = r0;
@@ -1680,6 +1681,7 @@ void GraphEngine::linear_search_tc_device(const uint4* d_rows, size_t nq, size_t
                                                                              d_status + q0, st.error + 1);
         TC_CUDA(cudaGetLastError());
         launches_++;
+        if (R > 1) a.skip = st.error + 1;
       }
       row = end;
     }
